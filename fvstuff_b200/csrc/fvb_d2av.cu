@@ -18,10 +18,18 @@
 // Every expression keeps the reference's association order and this file
 // is compiled without FMA contraction (-fmad=false), so a stage reproduces
 // the reference kernels' arithmetic operation for operation.
+//
+// What bounds it: instruction issue and the FP64 pipe, not memory (1024^2,
+// UP5: 14 us of a stage at the copy bandwidth).  The operators' divisions and
+// roots were most of it: 60 divisions a cell, 4970 instructions and 1530 FP64
+// ones, 235 us a stage.  Rounding the same quotients from shared reciprocals
+// (fvb_ieee.cuh: one reciprocal of a density for the three quotients by it,
+// none for the constant denominators and h) takes a stage to 105 us.
 #include <algorithm>
 
 #include "fvb_aux.h"
 #include "fvb_device.cuh"
+#include "fvb_ieee.cuh"
 
 namespace fvb {
 namespace {
@@ -102,6 +110,90 @@ __device__ __forceinline__ void d2_recon(const double *s, double &vL, double &vR
     }
 }
 
+// ---- the same operations with the quotients and roots of fvb_ieee.cuh ------
+// Every function below returns the bits of its operator form above while its
+// range tests hold (their result: true); the caller evaluates the operator
+// form otherwise.
+
+struct D2State {
+    double p, c, u, v, y;  // y: reciprocal of the density
+};
+
+__device__ __forceinline__ bool d2_prim_near(double gam, const double U[4], D2State &w)
+{
+    const double y = recip(U[0]);
+    w.y = y;
+    w.u = quot(U[1], U[0], y);
+    w.v = quot(U[2], U[0], y);
+    w.p = (gam - 1.0) * (U[3] - 0.5 * (U[1] * w.u + U[2] * w.v));
+    const double gp = gam * w.p, cs2 = quot(gp, U[0], y);
+    const double x = cs2 > 1e-14 ? cs2 : 1e-14;
+    w.c = root(x);
+    return den_ok(U[0]) && num_ok(U[1], U[2], gp) && num_ok(x);
+}
+
+__device__ __forceinline__ bool d2_hllc_near(double gam, const double UL[4], const double UR[4], double F[4])
+{
+    D2State l, r;
+    bool ok = d2_prim_near(gam, UL, l);
+    ok = d2_prim_near(gam, UR, r) && ok;
+    const double SL = smin<double>(l.u - l.c, r.u - r.c);
+    const double SR = smax<double>(l.u + l.c, r.u + r.c);
+    if (SL >= 0.0) {
+        F[0] = UL[1]; F[1] = UL[1] * l.u + l.p; F[2] = UL[1] * l.v; F[3] = (UL[3] + l.p) * l.u;
+        return ok;
+    }
+    if (SR <= 0.0) {
+        F[0] = UR[1]; F[1] = UR[1] * r.u + r.p; F[2] = UR[1] * r.v; F[3] = (UR[3] + r.p) * r.u;
+        return ok;
+    }
+    const double dL = UL[0] * (SL - l.u), dR = UR[0] * (SR - r.u);
+    const double sn = r.p - l.p + dL * l.u - dR * r.u, sd = dL - dR;
+    const double Ss = quot(sn, sd, recip(sd));
+    const bool left = Ss >= 0.0;
+    const double K0 = left ? UL[0] : UR[0], K1 = left ? UL[1] : UR[1];
+    const double K2 = left ? UL[2] : UR[2], K3 = left ? UL[3] : UR[3];
+    const double pK = left ? l.p : r.p, uK = left ? l.u : r.u, vK = left ? l.v : r.v, SK = left ? SL : SR;
+    const double yK = left ? l.y : r.y;
+    const double dK = left ? dL : dR;  // K0 (SK - uK), the same product
+    const double sq = SK - Ss;
+    const double f = quot(dK, sq, recip(sq));
+    const double s3 = f * (quot(K3, K0, yK) + (Ss - uK) * (Ss + quot(pK, dK, recip(dK))));
+    F[0] = K1 + SK * (f - K0);
+    F[1] = (K1 * uK + pK) + SK * (f * Ss - K1);
+    F[2] = K1 * vK + SK * (f * vK - K2);
+    F[3] = (K3 + pK) * uK + SK * (s3 - K3);
+    return ok && den_ok(sd) && den_ok(sq) && den_ok(dK) && num_ok(sn, K3, pK);
+}
+
+// (a product with 2 or 4 is exact, so fused with the sum beside it it rounds
+// as the separate operations do)
+template <int ORDER>
+__device__ __forceinline__ void d2_recon_near(const double *s, double &vL, double &vR)
+{
+    if constexpr (ORDER == 3) {
+        vL = quot(fma(2.0, s[2], -s[0] + 5.0 * s[1]), 6.0, 1.0 / 6.0);
+        vR = quot(fma(2.0, s[1], 5.0 * s[2]) - s[3], 6.0, 1.0 / 6.0);
+    } else if constexpr (ORDER == 5) {
+        vL = quot(fma(2.0, s[0], -(13.0 * s[1])) + 47.0 * s[2] + 27.0 * s[3] - 3.0 * s[4], 60.0, 1.0 / 60.0);
+        vR = quot(fma(2.0, s[5], -3.0 * s[1] + 27.0 * s[2] + 47.0 * s[3] - 13.0 * s[4]), 60.0, 1.0 / 60.0);
+    } else if constexpr (ORDER == 9) {
+        vL = quot(3.0 * s[0] - 25.0 * s[1] + 101.0 * s[2] - 319.0 * s[3] + 2765.0 * s[4] + 2139.0 * s[5] -
+                      533.0 * s[6] + 97.0 * s[7] - 11.0 * s[8],
+                  2520.0, 1.0 / 2520.0);
+        vR = quot(-11.0 * s[1] + 97.0 * s[2] - 533.0 * s[3] + 2139.0 * s[4] + 2765.0 * s[5] - 319.0 * s[6] +
+                      101.0 * s[7] - 25.0 * s[8] + 3.0 * s[9],
+                  2520.0, 1.0 / 2520.0);
+    } else {
+        vL = quot(fma(4.0, s[6], -3.0 * s[0] + 25.0 * s[1] - 101.0 * s[2] + 319.0 * s[3] + 214.0 * s[4] -
+                                     38.0 * s[5]),
+                  420.0, 1.0 / 420.0);
+        vR = quot(fma(4.0, s[1], -(38.0 * s[2])) + 214.0 * s[3] + 319.0 * s[4] - 101.0 * s[5] + 25.0 * s[6] -
+                      3.0 * s[7],
+                  420.0, 1.0 / 420.0);
+    }
+}
+
 template <int ORDER>
 struct D2Shape {
     static constexpr int HW = (ORDER + 1) / 2;         // reconstruction half width
@@ -115,6 +207,131 @@ struct D2Shape {
     // and UP9's 5
     static constexpr int MINB = HB == 3 ? 4 : 3;
 };
+
+// the flux of one face in its normal frame, b its right / top cell, st the
+// stride to the left / bottom one; NEAR: the shared-reciprocal form
+template <int ORDER, bool NEAR>
+__device__ __forceinline__ bool d2_face(const double *Q, int b, int st, bool xf, double gam, double Fn[4])
+{
+    using S = D2Shape<ORDER>;
+    constexpr int HW = S::HW;
+    double L[4], R[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        double s[2 * HW];
+#pragma unroll
+        for (int d = 0; d < 2 * HW; ++d) s[d] = Q[q * S::PL + b + (d - HW) * st];
+        if constexpr (NEAR) d2_recon_near<ORDER>(s, L[q], R[q]);
+        else d2_recon<ORDER>(s, L[q], R[q]);
+    }
+    const double UL[4] = {L[0], xf ? L[1] : L[2], xf ? L[2] : L[1], L[3]};
+    const double UR[4] = {R[0], xf ? R[1] : R[2], xf ? R[2] : R[1], R[3]};
+    if constexpr (NEAR) return d2_hllc_near(gam, UL, UR, Fn);
+    d2_hllc(gam, UL, UR, Fn);
+    return true;
+}
+
+template <int ORDER>
+__device__ __noinline__ void d2_face_any(const double *Q, int b, int st, bool xf, double gam, double Fn[4])
+{
+    d2_face<ORDER, false>(Q, b, st, xf, gam, Fn);
+}
+
+// per-cell quantities of the box in the operator form
+__device__ __noinline__ void d2_box_any(double gam, const double U[4], double o[5])
+{
+    const double rf = U[0] > 1e-14 ? U[0] : 1e-14;
+    double p, cc, u, v;
+    d2_prim(gam, U[0], U[1], U[2], U[3], p, cc, u, v);
+    o[0] = U[1] / rf;
+    o[1] = U[2] / rf;
+    o[2] = fabs(u) + cc;
+    o[3] = fabs(v) + cc;
+    o[4] = cc;
+}
+
+__device__ __noinline__ double d2_lam_any(double gam, const double U[4])
+{
+    double p, cc, u, v;
+    d2_prim(gam, U[0], U[1], U[2], U[3], p, cc, u, v);
+    return fabs(u) + fabs(v) + cc;
+}
+
+// what the cell update needs that is the same for every cell
+struct D2Cell {
+    double h, yh, h60, y60, c2h, cgh, sch, dt;  // y*: reciprocals of h and 60 h
+    int stage;
+    bool global;  // Cg is not 0
+};
+
+// residual (flux divergence, Ducros weight, viscosity) and RK combination of
+// the cell at b of the box; ua: U0 of the cell.  NEAR: quotients by h and by
+// the sensor's denominator in the shared-reciprocal form
+//                                          fv_up7_ducros_2d.cu.bak:344-445
+template <int ORDER, bool NEAR>
+__device__ __forceinline__ void d2_cell(const double *Q, const double *FX, const double *FY, int b, int r, int c,
+                                        const D2Cell &k, const double ua[4], double v[4])
+{
+    using S = D2Shape<ORDER>;
+    constexpr int BW = S::BW, PL = S::PL;
+    const double *SU = Q + 4 * PL, *SV = SU + PL, *LX = SV + PL, *LY = LX + PL, *CS = LY + PL;
+    const double wc[6] = {-1., 9., -45., 45., -9., 1.};
+    const int wo[6] = {-3, -2, -1, 1, 2, 3};
+    double du_dx = 0., dv_dy = 0.;
+#pragma unroll
+    for (int m = 0; m < 6; ++m) {
+        du_dx += wc[m] * SU[b + wo[m]];
+        dv_dy += wc[m] * SV[b + wo[m] * BW];
+    }
+    if constexpr (NEAR) {
+        du_dx = quot(du_dx, k.h60, k.y60);
+        dv_dy = quot(dv_dy, k.h60, k.y60);
+    } else {
+        du_dx /= k.h60;
+        dv_dy /= k.h60;
+    }
+    double div_u = du_dx + dv_dy;
+    if (div_u > 0.) div_u = 0.;
+    const double c0 = CS[b];
+    const double sos2 = k.sch * c0 * c0;
+    const double dd = div_u * div_u, den = dd + sos2 + 1e-40;
+    double S_D;
+    if constexpr (NEAR) S_D = quot(dd, den, recip(den));
+    else S_D = dd / den;
+    // face-averaged directional wave speeds   :359-367
+    const double lamx_c = LX[b], lamy_c = LY[b];
+    const double lhxp = 0.5 * (lamx_c + LX[b + 1]);
+    const double lhxm = 0.5 * (lamx_c + LX[b - 1]);
+    const double lhyp = 0.5 * (lamy_c + LY[b + BW]);
+    const double lhym = 0.5 * (lamy_c + LY[b - BW]);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const double *Qq = Q + q * PL;
+        const double Uc = Qq[b];
+        const double dxp = Qq[b + 1] - Uc, dxm = Uc - Qq[b - 1];
+        const double dyp = Qq[b + BW] - Uc, dym = Uc - Qq[b - BW];
+        double D2 = k.c2h * (lhxp * S_D * dxp - lhxm * S_D * dxm + lhyp * S_D * dyp - lhym * S_D * dym);
+        // (with Cg = 0 the term is +0 or -0 for finite states: nothing to add)
+        if (!NEAR || k.global)
+            D2 = D2 + k.cgh * (lhxp * (1. - S_D) * dxp - lhxm * (1. - S_D) * dxm + lhyp * (1. - S_D) * dyp -
+                               lhym * (1. - S_D) * dym);
+        const double *fx = FX + q * S::NFX + r * (DTX + 1) + c;
+        const double *fy = FY + q * S::NFY + r * DTX + c;
+        double L;
+        if constexpr (NEAR) L = -quot(fx[1] - fx[0], k.h, k.yh) - quot(fy[DTX] - fy[0], k.h, k.yh) + D2;
+        else L = -(fx[1] - fx[0]) / k.h - (fy[DTX] - fy[0]) / k.h + D2;  // :386
+        if (k.stage == 1) v[q] = ua[q] + k.dt * L;                                   // :433-435
+        else if (k.stage == 2) v[q] = 0.75 * ua[q] + 0.25 * (Uc + k.dt * L);         // :437-440
+        else v[q] = (1. / 3.) * ua[q] + (2. / 3.) * (Uc + k.dt * L);                 // :442-445
+    }
+}
+
+template <int ORDER>
+__device__ __noinline__ void d2_cell_any(const double *Q, const double *FX, const double *FY, int b, int r, int c,
+                                         const D2Cell &k, const double ua[4], double v[4])
+{
+    d2_cell<ORDER, false>(Q, FX, FY, b, r, c, k, ua, v);
+}
 
 // one SSP-RK3 stage                        fv_up7_ducros_2d.cu.bak:287-446
 template <int ORDER>
@@ -140,17 +357,27 @@ __global__ void __launch_bounds__(DNT, D2Shape<ORDER>::MINB)
     const double *u0 = (const double *)gd.st[0];
     double *out = (double *)(stage == 1 ? gd.k1 : stage == 2 ? gd.k2 : gd.st[0]);
     double lacc = 0.0;
+    // (in shared memory: 18 registers a thread would hold across the faces)
+    __shared__ D2Cell ck;
+    if (tid == 0)
+        ck = D2Cell{h, recip(h), 60. * h, recip(60. * h), av.c2 / h, av.cg / h, av.sc / (h * h), 0.0, stage,
+                    av.cg != 0.0};
+    const bool hok = den_ok(h) && den_ok(60. * h);
 
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const int tx0 = (t % gd.tiles_x) * DTX, ty0 = (t / gd.tiles_x) * DTY;
-        if (tid == 0) s_ctl = tile_control<P64>(gd.ctrl, stage, t == 0);
+        if (tid == 0) {
+            s_ctl = tile_control<P64>(gd.ctrl, stage, t == 0);
+            ck.dt = s_ctl.dt;
+        }
         __syncthreads();
-        const TileCtl ctl = s_ctl;
-        if (!ctl.run) {
+        if (!s_ctl.run) {
             __syncthreads();
             continue;
         }
-        // ---- halo box of the stage input and its per-cell quantities ------
+        // ---- halo box of the stage input and its per-cell quantities: the
+        //      sensor's velocities in the rows / columns it reaches, the wave
+        //      speeds on the cells and their direct neighbours --------------
         for (int k = tid; k < PL; k += DNT) {
             const int r = k / BW, c = k - r * BW, jp = ty0 + r, ip = tx0 + c;
             double U[4] = {1.0, 0.0, 0.0, 2.5};  // admissible filler beyond the padded grid
@@ -161,14 +388,22 @@ __global__ void __launch_bounds__(DNT, D2Shape<ORDER>::MINB)
             }
 #pragma unroll
             for (int q = 0; q < 4; ++q) Q[q * PL + k] = U[q];
-            const double rf = U[0] > 1e-14 ? U[0] : 1e-14;
-            SU[k] = U[1] / rf;
-            SV[k] = U[2] / rf;
-            double p, cc, u, v;
-            d2_prim(gam, U[0], U[1], U[2], U[3], p, cc, u, v);
-            LX[k] = fabs(u) + cc;
-            LY[k] = fabs(v) + cc;
-            CS[k] = cc;
+            const bool inr = (unsigned)(r - HB) < (unsigned)DTY, inc = (unsigned)(c - HB) < (unsigned)DTX;
+            if (!inr && !inc) continue;
+            D2State w;
+            // (the sensor's velocities divide by the density floored at 1e-14)
+            if (d2_prim_near(gam, U, w) && U[0] > 1e-14) {
+                SU[k] = w.u;
+                SV[k] = w.v;
+                LX[k] = fabs(w.u) + w.c;
+                LY[k] = fabs(w.v) + w.c;
+                CS[k] = w.c;
+            } else {
+                double o[5];
+                d2_box_any(gam, U, o);
+#pragma unroll
+                for (int m = 0; m < 5; ++m) SU[m * PL + k] = o[m];
+            }
         }
         __syncthreads();
         // ---- faces: x-face (r, c) between tile cells c-1 and c, y-face
@@ -179,19 +414,14 @@ __global__ void __launch_bounds__(DNT, D2Shape<ORDER>::MINB)
             if (xf) { r = f / (DTX + 1); c = f - r * (DTX + 1); st = 1; }
             else { const int f2 = f - S::NFX; r = f2 / DTX; c = f2 - r * DTX; st = BW; }
             const int b = (r + HB) * BW + (c + HB);
-            double L[4], R[4];
+            double Fn[4];
+            if (!d2_face<ORDER, true>(Q, b, st, xf, gam, Fn)) {
+                double Fa[4];
+                d2_face_any<ORDER>(Q, b, st, xf, gam, Fa);
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                double s[2 * HW];
-#pragma unroll
-                for (int d = 0; d < 2 * HW; ++d) s[d] = Q[q * PL + b + (d - HW) * st];
-                d2_recon<ORDER>(s, L[q], R[q]);
+                for (int q = 0; q < 4; ++q) Fn[q] = Fa[q];
             }
             const int qn = xf ? 1 : 2, qt = xf ? 2 : 1;
-            const double UL[4] = {L[0], xf ? L[1] : L[2], xf ? L[2] : L[1], L[3]};
-            const double UR[4] = {R[0], xf ? R[1] : R[2], xf ? R[2] : R[1], R[3]};
-            double Fn[4];
-            d2_hllc(gam, UL, UR, Fn);
             double *o = xf ? FX + r * (DTX + 1) + c : FY + r * DTX + c;
             const int os = xf ? S::NFX : S::NFY;
             o[0] = Fn[0];
@@ -205,54 +435,22 @@ __global__ void __launch_bounds__(DNT, D2Shape<ORDER>::MINB)
             const int r = k / DTX, c = k - r * DTX, i = tx0 + c, j = ty0 + r;
             if (i >= n || j >= n) continue;
             const int b = (r + HB) * BW + (c + HB);
-            // Ducros weight                fv_up7_ducros_2d.cu.bak:344-357
-            const double wc[6] = {-1., 9., -45., 45., -9., 1.};
-            const int wo[6] = {-3, -2, -1, 1, 2, 3};
-            double du_dx = 0., dv_dy = 0.;
-#pragma unroll
-            for (int m = 0; m < 6; ++m) {
-                du_dx += wc[m] * SU[b + wo[m]];
-                dv_dy += wc[m] * SV[b + wo[m] * BW];
-            }
-            du_dx /= 60. * h;
-            dv_dy /= 60. * h;
-            double div_u = du_dx + dv_dy;
-            if (div_u > 0.) div_u = 0.;
-            const double c0 = CS[b];
-            const double sos2 = (av.sc / (h * h)) * c0 * c0;
-            const double S_D = (div_u * div_u) / (div_u * div_u + sos2 + 1e-40);
-            // face-averaged directional wave speeds   :359-367
-            const double lamx_c = LX[b], lamy_c = LY[b];
-            const double lhxp = 0.5 * (lamx_c + LX[b + 1]);
-            const double lhxm = 0.5 * (lamx_c + LX[b - 1]);
-            const double lhyp = 0.5 * (lamy_c + LY[b + BW]);
-            const double lhym = 0.5 * (lamy_c + LY[b - BW]);
             const long long e = (long long)(j + HB) * gd.pitch + (i + HB) + gd.xoff;
-            double v[4];
+            double ua[4], v[4];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const double *Qq = Q + q * PL;
-                const double Uc = Qq[b];
-                const double dxp = Qq[b + 1] - Uc, dxm = Uc - Qq[b - 1];
-                const double dyp = Qq[b + BW] - Uc, dym = Uc - Qq[b - BW];
-                const double d2_duc = (av.c2 / h) * (lhxp * S_D * dxp - lhxm * S_D * dxm + lhyp * S_D * dyp -
-                                                     lhym * S_D * dym);
-                const double d2_glb = (av.cg / h) * (lhxp * (1. - S_D) * dxp - lhxm * (1. - S_D) * dxm +
-                                                     lhyp * (1. - S_D) * dyp - lhym * (1. - S_D) * dym);
-                const double D2 = d2_duc + d2_glb;
-                const double *fx = FX + q * S::NFX + r * (DTX + 1) + c;
-                const double *fy = FY + q * S::NFY + r * DTX + c;
-                const double L = -(fx[1] - fx[0]) / h - (fy[DTX] - fy[0]) / h + D2;  // :386
-                const double ua = u0[e + q * gd.plane];
-                if (stage == 1) v[q] = ua + ctl.dt * L;                                   // :433-435
-                else if (stage == 2) v[q] = 0.75 * ua + 0.25 * (Uc + ctl.dt * L);         // :437-440
-                else v[q] = (1. / 3.) * ua + (2. / 3.) * (Uc + ctl.dt * L);               // :442-445
+            for (int q = 0; q < 4; ++q) ua[q] = stage == 1 ? Q[q * PL + b] : u0[e + q * gd.plane];
+            d2_cell<ORDER, true>(Q, FX, FY, b, r, c, ck, ua, v);
+            if (!hok || max(max(hi_mag(v[0]), hi_mag(v[1])), max(hi_mag(v[2]), hi_mag(v[3]))) >= kHiMax) {
+                double va[4];
+                d2_cell_any<ORDER>(Q, FX, FY, b, r, c, ck, ua, va);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) v[q] = va[q];
             }
             put_cell<double>(gd, out, j, i, v);
             if (stage == 3) {
-                double p, cc, u, w;
-                d2_prim(gam, v[0], v[1], v[2], v[3], p, cc, u, w);
-                lacc = smax<double>(fabs(u) + fabs(w) + cc, lacc);  // lam_c, :362
+                D2State w;
+                lacc = smax<double>(d2_prim_near(gam, v, w) ? fabs(w.u) + fabs(w.v) + w.c : d2_lam_any(gam, v),
+                                    lacc);  // lam_c, :362
             }
         }
         if (stage == 3 && tid == 0 && t == 0) leader_finish<P64>(gd.ctrl);
