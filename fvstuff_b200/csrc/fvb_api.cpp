@@ -379,7 +379,9 @@ fvb_status fvb_create(const fvb_config *cfg, fvb_solver **out)
     // buffers | step control | TMA descriptors (64-byte aligned)
     const size_t ctrl_off = (s->G.bytes + 255) / 256 * 256;
     const size_t tmap_off = ctrl_off + 256;
-    size_t total = tmap_off + TM_COUNT * sizeof(CUtensorMap);
+    // | KEEP: one plane of cell entropies, which its sensor pass leaves for its stage kernel
+    const size_t ent_off = (tmap_off + TM_COUNT * sizeof(CUtensorMap) + 255) / 256 * 256;
+    size_t total = keep ? ent_off + (size_t)s->G.plane * sizeof(double) : tmap_off + TM_COUNT * sizeof(CUtensorMap);
     e = cudaMalloc(&s->block, total);
     if (e != cudaSuccess) {
         fvb_destroy(s);
@@ -388,6 +390,7 @@ fvb_status fvb_create(const fvb_config *cfg, fvb_solver **out)
     e = cudaMemsetAsync(s->block, 0, total, s->stream);
     if (e != cudaSuccess) { fvb_destroy(s); return cuda_fail(e, "cudaMemset"); }
     grid_pointers(s->gd, s->block, s->G, s->prec);
+    if (keep) s->gd.lo[0] = (char *)s->block + ent_off;
     s->ctrl = (Ctrl *)((char *)s->block + ctrl_off);
     s->gd.ctrl = s->ctrl;
     s->gd.tmap = nullptr;

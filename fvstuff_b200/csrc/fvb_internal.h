@@ -46,7 +46,7 @@ struct GridDev {
     int bcx, bcy;
     double h, gam;
     void *st[2];    // state: prim (F64/F32, st[0] only) or conserved hi (F32C, ping-pong)
-    void *lo[2];    // F32C: lo words of the conserved state
+    void *lo[2];    // F32C: lo words of the conserved state; KEEP: lo[0] holds the cells' entropies
     void *k1, *k2;  // stage outputs: U1/U2 primitives (F64/F32) or increments d1/d2 (F32C)
     Ctrl *ctrl;
     const CUtensorMap *tmap;  // TMA descriptors of st[0], st[1], k1, k2 for the

@@ -16,9 +16,19 @@
 // -- and form every face's terms from those, so no face repeats the
 // divisions and logarithms of its two cells.  The step control is the same
 // device-side Ctrl as the UP path.
+//
+// What bounds it: instruction issue and latency, not memory (1024^2: 16 us of
+// a stage at the copy bandwidth).  log and pow of every cell, once for each
+// of the two kernels and for every halo, IEEE divisions and exp per face were
+// 3340 instructions a cell; now a cell's entropy is formed once (the sensor
+// pass leaves it in a plane for the stage kernel), quotients share
+// reciprocals (fvb_ieee.cuh), a face evaluates the one dissipation its sensor
+// selects, and exp is evaluated only next to the sensor's threshold: 1760
+// instructions a cell, 202 -> 131 us a stage, bit-identical.
 #include "fvb_aux.h"
 #include "fvb_physics.cuh"
 #include "fvb_device.cuh"
+#include "fvb_ieee.cuh"
 
 namespace fvb {
 namespace {
@@ -50,6 +60,49 @@ __device__ __forceinline__ void k_evars(const double W[4], double s, double gam,
     V[2] = rho * v / p;
     V[3] = -rho / p;
 }
+
+// The same conversions with the quotients of fvb_ieee.cuh (one reciprocal of
+// rho, one of p); true while their range tests hold.  ygm1: recip(gam - 1).
+__device__ __forceinline__ bool k_prim_near(const double U[4], double gam, double W[4], double Uf[4])
+{
+    double rho = smax<double>(U[0], KG_MIN), mx = U[1], my = U[2], E = U[3];
+    const double y = recip(rho);
+    double u = quot(mx, rho, y), v = quot(my, rho, y);
+    W[0] = rho;
+    W[1] = u;
+    W[2] = v;
+    W[3] = smax<double>((gam - 1.) * (E - 0.5 * rho * (u * u + v * v)), KG_MIN);
+    Uf[0] = rho; Uf[1] = mx; Uf[2] = my; Uf[3] = E;
+    return den_ok(rho) && num_ok(mx, my) && num_ok(W[3]);
+}
+
+__device__ __forceinline__ bool k_evars_near(const double W[4], double s, double gam, double ygm1, double V[4])
+{
+    double rho = W[0], u = W[1], v = W[2], p = W[3];
+    const double y = recip(p);
+    const double ke = rho * (u * u + v * v), ru = rho * u, rv = rho * v;
+    // (the reciprocal of 2 p is half that of p, exactly)
+    V[0] = __dsub_rn(quot(gam - s, gam - 1., ygm1), quot(ke, 2. * p, 0.5 * y));
+    V[1] = quot(ru, p, y);
+    V[2] = quot(rv, p, y);
+    V[3] = -quot(rho, p, y);
+    return den_ok(p) && num_ok(ke, ru, rv) && num_ok(s);
+}
+
+// both in the operator form
+__device__ __noinline__ void k_prim_any(const double U[4], double gam, double W[4])
+{
+    double Uf[4], s;
+    k_cell(U, gam, W, Uf, s);
+}
+__device__ __noinline__ double k_snd_any(double rho, double p, double gam) { return k_snd(rho, p, gam); }
+__device__ __noinline__ void k_evars_any(const double W[4], double s, double gam, double V[4])
+{
+    k_evars(W, s, gam, V);
+}
+
+// s = ln(p / rho^gamma)
+__device__ __forceinline__ double k_entropy(const double W[4], double gam) { return log(W[3] / pow(W[0], gam)); }
 
 // ECKEP central flux (Cartesian) and MOVERS-RH coefficient  keep_fv:145-219
 // VL, VR: the two cells' entropy variables in the face frame (the Cartesian
@@ -117,24 +170,174 @@ __device__ __forceinline__ void load_cell(const double *buf, const GridDev &gd, 
     for (int q = 0; q < 4; ++q) U[q] = buf[e + q * gd.plane];
 }
 
-struct KCtl {
-    double dt;
-    int run;
-};
-
 constexpr int KTX = 32, KTY = 16, KNT = 256, KG = 2;
 constexpr int KSW = KTX + 2 * KG, KSH = KTY + 2 * KG, KPL = KSW * KSH;
 constexpr int EW = KTX + 1, EH = KTY + 1, EPL = EW * EH;  // a tile and its right / top neighbours
+
+// sqrt(gam p / rho) of positive rho, p; x: the root's argument for its test
+__device__ __forceinline__ double k_snd_near(double rho, double p, double gam, double &x)
+{
+    x = quot(gam * p, rho, recip(rho));
+    return root(x);
+}
+
+// what a launch's faces share
+struct KFace {
+    double gam, ygm1;    // gamma, recip(gamma - 1)
+    double edmax, kphi;  // sensor scale, 12 / (edmax + 1e-30)
+};
+
+// -ln(0.95): the shock sensor's 1 - exp(-12 sed) > 0.05 is 12 sed above it
+constexpr double KG_PHI = 0.051293294387550533427;
+
+// One face's flux F_EC + (1 - phi) F_JST + phi F_RH in Cartesian components,
+// the same operations as k_flux and the sum below it (k_face_any): phi is 0 or
+// 1, so only the dissipation that it selects is evaluated (the other enters
+// the reference's sum as a zero), and exp() only within 1e-10 of the sensor's
+// threshold.  XF: an x-face, between cells a and b.  False: a range test
+// failed, take k_face_any.
+template <bool XF>
+__device__ __forceinline__ bool k_face_near(const double *U, const double *W, const double *V, int a, int b,
+                                            const KFace &k, double F[4])
+{
+    constexpr int st = XF ? 1 : KSW;
+    constexpr int QN = XF ? 1 : 2, QT = XF ? 2 : 1;
+    const double gam = k.gam;
+    const double rL = U[a], pL = W[2 * KPL + a], rR = U[b], pR = W[2 * KPL + b];
+    // face frame: (un, ut) = (u, v) on x-faces, (v, -u) on y-faces
+    const double unL = W[(QN - 1) * KPL + a], unR = W[(QN - 1) * KPL + b];
+    const double utL = XF ? W[KPL + a] : -W[a], utR = XF ? W[KPL + b] : -W[b];
+    const double VL0 = V[a], VR0 = V[b], VL1 = V[QN * KPL + a], VR1 = V[QN * KPL + b];
+    const double VL2 = XF ? V[QT * KPL + a] : -V[QT * KPL + a], VR2 = XF ? V[QT * KPL + b] : -V[QT * KPL + b];
+    const double VL3 = V[3 * KPL + a], VR3 = V[3 * KPL + b];
+    const double EL = quot(pL, gam - 1., k.ygm1) + 0.5 * rL * (unL * unL + utL * utL);
+    const double ER = quot(pR, gam - 1., k.ygm1) + 0.5 * rR * (unR * unR + utR * utR);
+    // Which products are rounded before a sum and which enter it fused is
+    // fixed here by the _rn forms, so that the values do not depend on what
+    // else a compiler finds to share (num / den below turns a last bit into
+    // 1e-9 of the energy where dV3 is small).
+    const double mL = __dmul_rn(rL, unL), mR = __dmul_rn(rR, unR);
+    const double FL3 = __dmul_rn(EL + pL, unL), FR3 = __dmul_rn(ER + pR, unR);
+    const double dV0 = VR0 - VL0, dV1 = VR1 - VL1, dV2 = VR2 - VL2, dV3 = VR3 - VL3;
+    const double dpsi = __dsub_rn(mR, mL);
+    const double Fc0 = 0.5 * __dadd_rn(mL, mR);
+    const double unb = 0.5 * (unL + unR), utb = 0.5 * (utL + utR), pb = 0.5 * (pL + pR);
+    const double Fc1 = Fc0 * unb + pb;
+    const double Fc2 = __dmul_rn(Fc0, utb);
+    const double Feb = 0.5 * __dadd_rn(FL3, FR3);
+    const double num = dV0 * Fc0 + dV1 * Fc1 + dV2 * Fc2 + dV3 * Feb - dpsi;
+    const double den = dV3 * dV3 + 1e-16;
+    const double Fc3 = Feb - quot(num, den, recip(den)) * dV3;
+    const double rav = 0.5 * (rL + rR);
+    double sx;
+    const double aav = k_snd_near(rav, pb, gam, sx);
+    bool ok = num_ok(num) && den_ok(den) && den_ok(sx) && num_ok(EL, ER);
+    // shock sensor                                 keep_fv:249-258, :347-349
+    const double dU0 = rR - rL, dU1 = U[KPL + b] - U[KPL + a], dU2 = U[2 * KPL + b] - U[2 * KPL + a];
+    const double dU3 = U[3 * KPL + b] - U[3 * KPL + a];
+    double ed = 0.;
+    ed += dU0 * (VR0 - VL0);
+    ed += dU1 * (V[KPL + b] - V[KPL + a]);
+    ed += dU2 * (V[2 * KPL + b] - V[2 * KPL + a]);
+    ed += dU3 * (VR3 - VL3);
+    const double xs = fabs(ed) * k.kphi;
+    bool shock = xs > KG_PHI;
+    if (fabs(xs - KG_PHI) < 1e-10 * KG_PHI) {
+        const double sed = fabs(ed) / (k.edmax + 1e-30);
+        shock = (1. - exp(-12.0 * sed)) > 0.05;
+    }
+    const double fec[4] = {Fc0, XF ? Fc1 : -Fc2, XF ? Fc2 : Fc1, Fc3};
+    if (!shock) {
+        const double lamt = smax<double>(fabs(unL), fabs(unR)) + aav;
+        const double aJST = (1.0 / 32.0) * lamt;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const double *u = U + q * KPL;
+            const double jst = __dmul_rn(aJST, u[b + st] - 3. * u[b] + 3. * u[a] - u[a - st]);
+            F[q] = __dadd_rn(fec[q], jst);
+        }
+        return ok;
+    }
+    const double l1 = fabs(unb - aav), l2 = fabs(unb), l3 = fabs(unb + aav);
+    const double lmin = smin<double>(l1, smin<double>(l2, l3)), lmax = smax<double>(l1, smax<double>(l2, l3));
+    double aS = lmax;
+    const double dUq[4] = {dU0, dpsi, __dsub_rn(__dmul_rn(rR, utR), __dmul_rn(rL, utL)), ER - EL};
+    const double dFq[4] = {dpsi, __dsub_rn(__fma_rn(mR, unR, pR), __fma_rn(mL, unL, pL)),
+                           __dsub_rn(__dmul_rn(mR, utR), __dmul_rn(mL, utL)), __dsub_rn(FR3, FL3)};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const double dU = dUq[q], dF = dFq[q];
+        const bool small = fabs(dU) < 1e-12;
+        double sk = small ? lmin : fabs(quot(dF, dU, recip(small ? 1.0 : dU)));
+        if (sk >= lmax) sk = lmax;
+        else if (sk <= lmin) sk = lmin;
+        if (sk < aS) aS = sk;
+        ok = ok && num_ok(dF, dU);
+    }
+    if (aS < 0.1) aS = (aS * aS + 0.1 * 0.1) / (2. * 0.1);
+    const double dUc[4] = {dU0, dU1, dU2, dU3};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) F[q] = __dadd_rn(fec[q], __dmul_rn(-0.5 * aS, dUc[q]));
+    return ok;
+}
+
+// the same face in the operator form, as the reference writes it
+__device__ __noinline__ void k_face_any(const double *U, const double *Wuvp, const double *V, int a, int b, bool xf,
+                                        double gam, double edmax, double F[4])
+{
+    const int st = b - a;
+    const double nx = xf ? 1. : 0., ny = xf ? 0. : 1.;
+    double WL[4], WR[4], UL[4], UR[4], VL[4], VR[4], fec[4], aS;
+    for (int q = 0; q < 4; ++q) {
+        WL[q] = q ? Wuvp[(q - 1) * KPL + a] : U[a]; WR[q] = q ? Wuvp[(q - 1) * KPL + b] : U[b];
+        UL[q] = U[q * KPL + a]; UR[q] = U[q * KPL + b];
+        VL[q] = V[q * KPL + a]; VR[q] = V[q * KPL + b];
+    }
+    const double VLn[4] = {VL[0], xf ? VL[1] : VL[2], xf ? VL[2] : -VL[1], VL[3]};
+    const double VRn[4] = {VR[0], xf ? VR[1] : VR[2], xf ? VR[2] : -VR[1], VR[3]};
+    k_flux(WL, WR, VLn, VRn, nx, ny, gam, fec, &aS);
+    const double unL = WL[1] * nx + WL[2] * ny, unR = WR[1] * nx + WR[2] * ny;
+    const double aR = k_snd(0.5 * (WL[0] + WR[0]), 0.5 * (WL[3] + WR[3]), gam);
+    const double lamt = smax<double>(fabs(unL), fabs(unR)) + aR;
+    const double aJST = (1.0 / 32.0) * lamt;
+    // entropy distance of the face                  keep_fv:249-258
+    double ed = 0.;
+    for (int q = 0; q < 4; ++q) ed += (UR[q] - UL[q]) * (VR[q] - VL[q]);
+    const double sed = fabs(ed) / (edmax + 1e-30);
+    const double phi = (1. - exp(-12.0 * sed)) > 0.05 ? 1. : 0.;
+    for (int q = 0; q < 4; ++q) {
+        const double jst = aJST * (U[q * KPL + b + st] - 3. * UR[q] + 3. * UL[q] - U[q * KPL + a - st]);
+        const double rh = -0.5 * aS * (UR[q] - UL[q]);
+        F[q] = fec[q] + (1. - phi) * jst + phi * rh;
+    }
+}
+
+// store a per-cell scalar and its ghost images (no sign: it is even in the
+// velocities)
+__device__ __forceinline__ void put_scalar(const GridDev &gd, double *buf, int j, int i, double v)
+{
+    buf[gidx(gd, 0, j, i)] = v;
+    const int g = gd.g, n = gd.n;
+    if (i >= g && i < n - g && j >= g && j < n - g) return;
+    const int nx = n_images(i, n, g, gd.bcx), ny = n_images(j, n, g, gd.bcy);
+    bool f;
+    for (int ka = 0; ka < ny; ++ka)
+        for (int kb = (ka == 0 ? 1 : 0); kb < nx; ++kb)
+            buf[gidx(gd, 0, image_of(ka, j, n, g, gd.bcy, f), image_of(kb, i, n, g, gd.bcx, f))] = v;
+}
 
 // per-cell max of the entropy distance |(U_n - U_c) . (V_n - V_c)| across
 // its right and top faces, max-reduced into ctrl->aux; a tile's cells and
 // their right / top neighbours are converted once each (floored conserved
 // state and entropy variables in shared memory)   keep_fv_euler_2d.cu:249-277
-__global__ void __launch_bounds__(KNT) keep_ed_kernel(const GridDev gd, const double *buf, int ntiles)
+// Each cell's entropy, its log and pow the costliest operations of the
+// scheme, goes to the plane `ent`, from which the stage kernel reads it.
+__global__ void __launch_bounds__(KNT) keep_ed_kernel(const GridDev gd, const double *buf, double *ent, int ntiles)
 {
     __shared__ double sU[4][EPL], sV[4][EPL];
     __shared__ double sh[KNT / 32];
     const int tid = threadIdx.x, n = gd.n;
+    const double gam = gd.gam, ygm1 = recip(gam - 1.);
     double m = 0.0;
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const int tx0 = (t % gd.tiles_x) * KTX, ty0 = (t / gd.tiles_x) * KTY;
@@ -142,13 +345,17 @@ __global__ void __launch_bounds__(KNT) keep_ed_kernel(const GridDev gd, const do
             const int r = k / EW, c = k - r * EW, j = ty0 + r, i = tx0 + c;
             double U[4] = {1, 0, 0, 2.5};  // admissible filler beyond the ghost layer
             if (j <= n && i <= n) load_cell(buf, gd, j, i, U);
-            double W[4], Uf[4], sc, V[4];
-            k_cell(U, gd.gam, W, Uf, sc);
-            k_evars(W, sc, gd.gam, V);
+            double W[4], Uf[4], V[4];
+            bool ok = k_prim_near(U, gam, W, Uf);
+            if (!ok) k_prim_any(U, gam, W);
+            const double sc = k_entropy(W, gam);
+            ok = k_evars_near(W, sc, gam, ygm1, V) && ok;
+            if (!ok) k_evars_any(W, sc, gam, V);
             for (int q = 0; q < 4; ++q) {
                 sU[q][k] = Uf[q];
                 sV[q][k] = V[q];
             }
+            if (r < KTY && c < KTX && j < n && i < n) put_scalar(gd, ent, j, i, sc);
         }
         __syncthreads();
         for (int k = tid; k < KTX * KTY; k += KNT) {
@@ -179,85 +386,79 @@ __global__ void __launch_bounds__(KNT, 2) keep_stage_kernel(const GridDev gd, in
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double *U = reinterpret_cast<double *>(smem_raw);  // [4][KSH][KSW] conserved, rho floored
-    double *W = U + 4 * KPL;                           // [4] floored primitives
-    double *V = W + 4 * KPL;                           // [4] entropy variables (Cartesian)
+    double *W = U + 4 * KPL;                           // [3] u, v, floored p
+    double *V = W + 3 * KPL;                           // [4] entropy variables (Cartesian)
     double *FX = V + 4 * KPL;                          // [4][KTY][KTX+1]
     double *FY = FX + 4 * KTY * (KTX + 1);             // [4][KTY+1][KTX]
-    __shared__ KCtl s_ctl;
+    __shared__ TileCtl s_ctl;
     __shared__ double s_red[KNT / 32];
     const int tid = threadIdx.x, n = gd.n, np = n + 2 * KG;
     const double gam = gd.gam;
     const double *in = (const double *)(stage == 2 ? gd.k1 : stage == 3 ? gd.k2 : gd.st[0]);
     const double *u0 = (const double *)gd.st[0];
     double *out = (double *)(stage == 1 ? gd.k1 : stage == 2 ? gd.k2 : gd.st[0]);
+    const double *ent = (const double *)gd.lo[0];  // the stage input's entropies (keep_ed_kernel)
     const double edmax = __longlong_as_double((long long)gd.ctrl->aux);
     const double inv_h = 1. / gd.h;
+    const KFace kf{gam, recip(gam - 1.), edmax, 12. / (edmax + 1e-30)};
 
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const int tx0 = (t % gd.tiles_x) * KTX, ty0 = (t / gd.tiles_x) * KTY;
-        if (tid == 0) {
-            TileCtl c = tile_control<P64>(gd.ctrl, stage, t == 0);
-            s_ctl = KCtl{c.dt, c.run};
-        }
+        if (tid == 0) s_ctl = tile_control<P64>(gd.ctrl, stage, t == 0);
         __syncthreads();
-        const KCtl ctl = s_ctl;
+        const TileCtl ctl = s_ctl;
         if (!ctl.run) {
             __syncthreads();
             continue;
         }
+        // conserved state of the box; primitives and entropy variables of the
+        // cells next to a face (the outer ring is the JST stencil's alone)
         for (int k = tid; k < KPL; k += KNT) {
             const int r = k / KSW, c = k - r * KSW, jp = ty0 + r, ip = tx0 + c;
-            double Uc[4] = {1, 0, 0, 2.5};
+            const bool ring = (unsigned)(r - 1) < (unsigned)(KTY + 2) && (unsigned)(c - 1) < (unsigned)(KTX + 2);
+            double Uc[4] = {1, 0, 0, 2.5}, sc = 0.;
             if (jp < np && ip < np) {
                 long long e = (long long)jp * gd.pitch + ip + gd.xoff;
+#pragma unroll
                 for (int q = 0; q < 4; ++q) Uc[q] = in[e + q * gd.plane];
+                if (ring) sc = ent[e];
             }
-            double Wc[4], Fc[4], sc, Vc[4];
-            k_cell(Uc, gam, Wc, Fc, sc);
-            k_evars(Wc, sc, gam, Vc);
-            for (int q = 0; q < 4; ++q) {
-                U[q * KPL + k] = Fc[q];
-                W[q * KPL + k] = Wc[q];
-                V[q * KPL + k] = Vc[q];
-            }
+            U[k] = smax<double>(Uc[0], KG_MIN);
+            U[KPL + k] = Uc[1];
+            U[2 * KPL + k] = Uc[2];
+            U[3 * KPL + k] = Uc[3];
+            if (!ring) continue;
+            double Wc[4], Fc[4], Vc[4];
+            bool ok = k_prim_near(Uc, gam, Wc, Fc);
+            if (!ok) k_prim_any(Uc, gam, Wc);
+            ok = k_evars_near(Wc, sc, gam, kf.ygm1, Vc) && ok;
+            if (!ok) k_evars_any(Wc, sc, gam, Vc);
+            W[k] = Wc[1];
+            W[KPL + k] = Wc[2];
+            W[2 * KPL + k] = Wc[3];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) V[q * KPL + k] = Vc[q];
         }
         __syncthreads();
         // faces: x then y; the face lies between cells a (left/bottom) and
         // b = a + st, with the JST stencil reaching a - st and b + st
-        for (int f = tid; f < (KTX + 1) * KTY + KTX * (KTY + 1); f += KNT) {
-            const bool xf = f < (KTX + 1) * KTY;
-            int r, c, st;
-            if (xf) { r = f / (KTX + 1); c = f - r * (KTX + 1); st = 1; }
-            else { const int f2 = f - (KTX + 1) * KTY; r = f2 / KTX; c = f2 - r * KTX; st = KSW; }
-            const int b = (r + KG) * KSW + (c + KG), a = b - st;
-            const double nx = xf ? 1. : 0., ny = xf ? 0. : 1.;
-            double WL[4], WR[4], UL[4], UR[4], Up2[4], Um1[4], VL[4], VR[4], fec[4], aS;
-            for (int q = 0; q < 4; ++q) {
-                WL[q] = W[q * KPL + a]; WR[q] = W[q * KPL + b];
-                UL[q] = U[q * KPL + a]; UR[q] = U[q * KPL + b];
-                Up2[q] = U[q * KPL + b + st]; Um1[q] = U[q * KPL + a - st];
-                VL[q] = V[q * KPL + a]; VR[q] = V[q * KPL + b];
-            }
-            // face frame: (un, ut) = (u, v) on x-faces, (v, -u) on y-faces
-            const double VLn[4] = {VL[0], xf ? VL[1] : VL[2], xf ? VL[2] : -VL[1], VL[3]};
-            const double VRn[4] = {VR[0], xf ? VR[1] : VR[2], xf ? VR[2] : -VR[1], VR[3]};
-            k_flux(WL, WR, VLn, VRn, nx, ny, gam, fec, &aS);
-            const double unL = WL[1] * nx + WL[2] * ny, unR = WR[1] * nx + WR[2] * ny;
-            const double aR = k_snd(0.5 * (WL[0] + WR[0]), 0.5 * (WL[3] + WR[3]), gam);
-            const double lamt = smax<double>(fabs(unL), fabs(unR)) + aR;
-            const double aJST = (1.0 / 32.0) * lamt;
-            // entropy distance of the face                  keep_fv:249-258
-            double ed = 0.;
-            for (int q = 0; q < 4; ++q) ed += (UR[q] - UL[q]) * (VR[q] - VL[q]);
-            const double sed = fabs(ed) / (edmax + 1e-30);
-            const double phi = (1. - exp(-12.0 * sed)) > 0.05 ? 1. : 0.;
-            double *o = xf ? FX + r * (KTX + 1) + c : FY + r * KTX + c;
-            const int os = xf ? KTY * (KTX + 1) : (KTY + 1) * KTX;
-            for (int q = 0; q < 4; ++q) {
-                const double jst = aJST * (Up2[q] - 3. * UR[q] + 3. * UL[q] - Um1[q]);
-                const double rh = -0.5 * aS * (UR[q] - UL[q]);
-                o[q * os] = fec[q] + (1. - phi) * jst + phi * rh;
-            }
+        for (int f = tid; f < (KTX + 1) * KTY; f += KNT) {
+            const int r = f / (KTX + 1), c = f - r * (KTX + 1);
+            const int b = (r + KG) * KSW + (c + KG), a = b - 1;
+            double F[4];
+            if (!k_face_near<true>(U, W, V, a, b, kf, F)) k_face_any(U, W, V, a, b, true, gam, edmax, F);
+            double *o = FX + f;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) o[q * KTY * (KTX + 1)] = F[q];
+        }
+        for (int f = tid; f < KTX * (KTY + 1); f += KNT) {
+            const int r = f / KTX, c = f - r * KTX;
+            const int b = (r + KG) * KSW + (c + KG), a = b - KSW;
+            double F[4];
+            if (!k_face_near<false>(U, W, V, a, b, kf, F)) k_face_any(U, W, V, a, b, false, gam, edmax, F);
+            double *o = FY + f;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) o[q * (KTY + 1) * KTX] = F[q];
         }
         __syncthreads();
         double lmax = 0.0;
@@ -280,9 +481,13 @@ __global__ void __launch_bounds__(KNT, 2) keep_stage_kernel(const GridDev gd, in
             v[3] = smax<double>(v[3], KG_MIN);
             put_cell<double>(gd, out, j, i, v);
             if (stage == 3) {
-                double Wn[4], Fn[4], sn;
-                k_cell(v, gam, Wn, Fn, sn);
-                const double cs = k_snd(Wn[0], Wn[3], gam);
+                double Wn[4], Fn[4], x;
+                bool ok = k_prim_near(v, gam, Wn, Fn);
+                double cs = k_snd_near(Wn[0], Wn[3], gam, x);
+                if (!(ok && den_ok(x))) {
+                    k_prim_any(v, gam, Wn);
+                    cs = k_snd_any(Wn[0], Wn[3], gam);
+                }
                 lmax = smax<double>((fabs(Wn[1]) + cs) + (fabs(Wn[2]) + cs), lmax);
             }
         }
@@ -326,7 +531,7 @@ __global__ void keep_lam_kernel(const GridDev gd)
     }
 }
 
-size_t keep_smem() { return sizeof(double) * (12 * KPL + 4 * KTY * (KTX + 1) + 4 * (KTY + 1) * KTX); }
+size_t keep_smem() { return sizeof(double) * (11 * KPL + 4 * KTY * (KTX + 1) + 4 * (KTY + 1) * KTX); }
 
 }  // namespace
 
@@ -348,7 +553,7 @@ cudaError_t keep_launch_stage(const GridDev &gd, int stage, int tiles, cudaStrea
     e = cudaMemsetAsync(&gd.ctrl->aux, 0, sizeof(unsigned long long), s);
     if (e != cudaSuccess) return e;
     const int eb = tiles < 4 * sms ? tiles : 4 * sms;
-    keep_ed_kernel<<<eb, KNT, 0, s>>>(gd, (const double *)in, tiles);
+    keep_ed_kernel<<<eb, KNT, 0, s>>>(gd, (const double *)in, (double *)gd.lo[0], tiles);
     const int grid = tiles < ctas_per_sm * sms ? tiles : ctas_per_sm * sms;
     keep_stage_kernel<<<grid, KNT, keep_smem(), s>>>(gd, stage, tiles);
     return cudaGetLastError();
