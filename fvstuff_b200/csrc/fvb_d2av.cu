@@ -238,8 +238,9 @@ __device__ __noinline__ void d2_face_any(const double *Q, int b, int st, bool xf
 }
 
 // per-cell quantities of the box in the operator form
-__device__ __noinline__ void d2_box_any(double gam, const double U[4], double o[5])
+__device__ __noinline__ void d2_box_any(double gam, double U0, double U1, double U2, double U3, double o[5])
 {
+    const double U[4] = {U0, U1, U2, U3};
     const double rf = U[0] > 1e-14 ? U[0] : 1e-14;
     double p, cc, u, v;
     d2_prim(gam, U[0], U[1], U[2], U[3], p, cc, u, v);
@@ -250,8 +251,9 @@ __device__ __noinline__ void d2_box_any(double gam, const double U[4], double o[
     o[4] = cc;
 }
 
-__device__ __noinline__ double d2_lam_any(double gam, const double U[4])
+__device__ __noinline__ double d2_lam_any(double gam, double U0, double U1, double U2, double U3)
 {
+    const double U[4] = {U0, U1, U2, U3};
     double p, cc, u, v;
     d2_prim(gam, U[0], U[1], U[2], U[3], p, cc, u, v);
     return fabs(u) + fabs(v) + cc;
@@ -400,7 +402,7 @@ __global__ void __launch_bounds__(DNT, D2Shape<ORDER>::MINB)
                 CS[k] = w.c;
             } else {
                 double o[5];
-                d2_box_any(gam, U, o);
+                d2_box_any(gam, U[0], U[1], U[2], U[3], o);
 #pragma unroll
                 for (int m = 0; m < 5; ++m) SU[m * PL + k] = o[m];
             }
@@ -441,15 +443,17 @@ __global__ void __launch_bounds__(DNT, D2Shape<ORDER>::MINB)
             for (int q = 0; q < 4; ++q) ua[q] = stage == 1 ? Q[q * PL + b] : u0[e + q * gd.plane];
             d2_cell<ORDER, true>(Q, FX, FY, b, r, c, ck, ua, v);
             if (!hok || max(max(hi_mag(v[0]), hi_mag(v[1])), max(hi_mag(v[2]), hi_mag(v[3]))) >= kHiMax) {
-                double va[4];
-                d2_cell_any<ORDER>(Q, FX, FY, b, r, c, ck, ua, va);
+                double ub[4], va[4];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) ub[q] = ua[q];
+                d2_cell_any<ORDER>(Q, FX, FY, b, r, c, ck, ub, va);
 #pragma unroll
                 for (int q = 0; q < 4; ++q) v[q] = va[q];
             }
             put_cell<double>(gd, out, j, i, v);
             if (stage == 3) {
                 D2State w;
-                lacc = smax<double>(d2_prim_near(gam, v, w) ? fabs(w.u) + fabs(w.v) + w.c : d2_lam_any(gam, v),
+                lacc = smax<double>(d2_prim_near(gam, v, w) ? fabs(w.u) + fabs(w.v) + w.c : d2_lam_any(gam, v[0], v[1], v[2], v[3]),
                                     lacc);  // lam_c, :362
             }
         }

@@ -90,15 +90,32 @@ __device__ __forceinline__ bool k_evars_near(const double W[4], double s, double
 }
 
 // both in the operator form
-__device__ __noinline__ void k_prim_any(const double U[4], double gam, double W[4])
+__device__ __noinline__ void k_prim_any_(const double U[4], double gam, double W[4])
 {
     double Uf[4], s;
     k_cell(U, gam, W, Uf, s);
 }
 __device__ __noinline__ double k_snd_any(double rho, double p, double gam) { return k_snd(rho, p, gam); }
-__device__ __noinline__ void k_evars_any(const double W[4], double s, double gam, double V[4])
+__device__ __noinline__ void k_evars_any_(const double W[4], double s, double gam, double V[4])
 {
     k_evars(W, s, gam, V);
+}
+// (called with copies, so that the arrays of the usual path stay in registers)
+__device__ __forceinline__ void k_prim_any(const double U[4], double gam, double W[4])
+{
+    const double A[4] = {U[0], U[1], U[2], U[3]};
+    double B[4];
+    k_prim_any_(A, gam, B);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) W[q] = B[q];
+}
+__device__ __forceinline__ void k_evars_any(const double W[4], double s, double gam, double V[4])
+{
+    const double A[4] = {W[0], W[1], W[2], W[3]};
+    double B[4];
+    k_evars_any_(A, s, gam, B);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) V[q] = B[q];
 }
 
 // s = ln(p / rho^gamma)
@@ -446,7 +463,12 @@ __global__ void __launch_bounds__(KNT, 2) keep_stage_kernel(const GridDev gd, in
             const int r = f / (KTX + 1), c = f - r * (KTX + 1);
             const int b = (r + KG) * KSW + (c + KG), a = b - 1;
             double F[4];
-            if (!k_face_near<true>(U, W, V, a, b, kf, F)) k_face_any(U, W, V, a, b, true, gam, edmax, F);
+            if (!k_face_near<true>(U, W, V, a, b, kf, F)) {
+                double A[4];
+                k_face_any(U, W, V, a, b, true, gam, edmax, A);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) F[q] = A[q];
+            }
             double *o = FX + f;
 #pragma unroll
             for (int q = 0; q < 4; ++q) o[q * KTY * (KTX + 1)] = F[q];
@@ -455,7 +477,12 @@ __global__ void __launch_bounds__(KNT, 2) keep_stage_kernel(const GridDev gd, in
             const int r = f / KTX, c = f - r * KTX;
             const int b = (r + KG) * KSW + (c + KG), a = b - KSW;
             double F[4];
-            if (!k_face_near<false>(U, W, V, a, b, kf, F)) k_face_any(U, W, V, a, b, false, gam, edmax, F);
+            if (!k_face_near<false>(U, W, V, a, b, kf, F)) {
+                double A[4];
+                k_face_any(U, W, V, a, b, false, gam, edmax, A);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) F[q] = A[q];
+            }
             double *o = FY + f;
 #pragma unroll
             for (int q = 0; q < 4; ++q) o[q * (KTY + 1) * KTX] = F[q];
