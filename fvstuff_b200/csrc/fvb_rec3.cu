@@ -22,10 +22,21 @@
 // that scatter adds them (by source cell index), and this file is compiled
 // without FMA contraction (-fmad=false), so each stage reproduces the
 // reference's arithmetic operation for operation.
+//
+// What bounds it: instruction issue, and on shocks the bisections' dependent
+// chains; not memory (1024^2: 14 us of a stage at the copy bandwidth).
+// Quotients and roots come from shared reciprocals (fvb_ieee.cuh: 2500 -> 1090
+// instructions a cell).  A face or block that clears its floors, nearly all,
+// needs no scaling and takes none of its code; the faces that do not are
+// listed and then handled one a thread: in place, each warp along the shock
+// went through 25 dependent steps for one or two of its lanes, face after
+// face, and the tiles of the ring held the launch up (84 us of it).  Sod
+// 1024^2: 225 -> 116 us a stage, bit-identical.
 #include <algorithm>
 
 #include "fvb_aux.h"
 #include "fvb_device.cuh"
+#include "fvb_ieee.cuh"
 
 namespace fvb {
 namespace {
@@ -34,6 +45,7 @@ constexpr double R3_GAM = 1.4, R3_PFLOOR = 1e-9, R3_RHOFLOOR = 1e-12;
 constexpr int RTX = 32, RTY = 32, RNT = 256, RG = 2;
 constexpr int RSW = RTX + 2 * RG, RSH = RTY + 2 * RG, RPL = RSW * RSH;
 constexpr int RNC = RTX * RTY;
+constexpr int RNF = RTY * (RTX + 1) + (RTY + 1) * RTX;  // faces of a tile
 
 // c = sqrt(gamma p / rho)                       fv_rec3_2d.cu:68-69
 __device__ __forceinline__ double r3_snd(double rho, double p) { return sqrt(R3_GAM * p / rho); }
@@ -116,6 +128,115 @@ __device__ __forceinline__ void r3_scale_w(const double Ub[4], double U[4], doub
     W[0] = r; W[1] = u; W[2] = v; W[3] = smax<double>(p, R3_PFLOOR);
 }
 
+// ---- the same operations with the quotients and roots of fvb_ieee.cuh ------
+// Each returns the bits of its operator form above while its range tests hold
+// (`ok` stays true); the caller evaluates the operator form otherwise.
+constexpr double R3_GM1 = R3_GAM - 1.0, R3_YGM1 = 1.0 / R3_GM1;
+
+// velocity and pressure of a conserved state; r: the floored density
+__device__ __forceinline__ double r3_p_near(const double U[4], double &r, double &u, double &v, bool &ok)
+{
+    r = smax<double>(U[0], R3_RHOFLOOR);
+    const double y = recip(r);
+    u = quot(U[1], r, y);
+    v = quot(U[2], r, y);
+    ok = ok && den_ok(r) && num_ok(U[1], U[2], U[3]);
+    return R3_GM1 * (U[3] - 0.5 * r * (u * u + v * v));
+}
+
+__device__ __noinline__ void r3_scale_any(const double Ub[4], double U[4], double W[4])
+{
+    r3_scale_w(Ub, U, W);
+}
+
+// r3_scale_w of a face state that clears its floors (nearly all): converted
+// at once; false: it needs the scaling
+__device__ __forceinline__ bool r3_clear_near(const double U[4], double W[4])
+{
+    bool ok = U[0] >= R3_RHOFLOOR;
+    W[3] = r3_p_near(U, W[0], W[1], W[2], ok);
+    return ok && W[3] >= R3_PFLOOR;
+}
+
+// r3_scale_w with the bisection's pressures in the shared-reciprocal form
+__device__ __forceinline__ void r3_scale_near(const double Ub[4], double U[4], double W[4])
+{
+    bool ok = true;
+    double S[4] = {U[0], U[1], U[2], U[3]};
+    if (S[0] < R3_RHOFLOOR) {
+        const double d = Ub[0] - S[0];
+        const double th = (d > 0.) ? (Ub[0] - R3_RHOFLOOR) / d : 0.;
+#pragma unroll
+        for (int q = 0; q < 4; q++) S[q] = Ub[q] + th * (S[q] - Ub[q]);
+    }
+    double p = r3_p_near(S, W[0], W[1], W[2], ok);
+    if (p < R3_PFLOOR) {
+        double lo = 0., hi = 1.;
+#pragma unroll 1
+        for (int it = 0; it < 25; it++) {
+            const double mid = 0.5 * (lo + hi);
+            double V[4], r, u, v;
+#pragma unroll
+            for (int q = 0; q < 4; q++) V[q] = Ub[q] + mid * (S[q] - Ub[q]);
+            const double pv = r3_p_near(V, r, u, v, ok);
+            const bool in = V[0] >= R3_RHOFLOOR && pv >= R3_PFLOOR;
+            lo = in ? mid : lo;
+            hi = in ? hi : mid;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) S[q] = Ub[q] + lo * (S[q] - Ub[q]);
+        p = r3_p_near(S, W[0], W[1], W[2], ok);
+    }
+    W[3] = smax<double>(p, R3_PFLOOR);
+    if (!ok) {
+        // (by copies, so that the arrays of the usual path stay in registers)
+        double B[4], X[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) { B[q] = Ub[q]; S[q] = U[q]; }
+        double T[4] = {S[0], S[1], S[2], S[3]};
+        r3_scale_any(B, T, X);
+#pragma unroll
+        for (int q = 0; q < 4; q++) W[q] = X[q];
+    }
+}
+
+// HLLC of floored face states (rho, un, ut, p)
+__device__ __forceinline__ bool r3_hllc_near(const double L[4], const double R[4], double F[4])
+{
+    const double rL = L[0], uL = L[1], tL = L[2], pL = L[3];
+    const double rR = R[0], uR = R[1], tR = R[2], pR = R[3];
+    const double yL = recip(rL), yR = recip(rR);
+    const double xL = quot(R3_GAM * pL, rL, yL), xR = quot(R3_GAM * pR, rR, yR);
+    const double cL = root(xL), cR = root(xR);
+    bool ok = den_ok(rL) && den_ok(rR) && den_ok(xL) && den_ok(xR) && num_ok(pL, pR);
+    const double SL = smin<double>(uL - cL, uR - cR), SR = smax<double>(uL + cL, uR + cR);
+    const bool supL = SL >= 0., sup = supL || SR <= 0.;
+    const double dL = rL * (SL - uL), dR = rR * (SR - uR);
+    const double sn = pR - pL + dL * uL - dR * uR, sd = dL - dR;
+    const double Ss = quot(sn, sd, recip(sd));
+    // the side whose state the flux needs: the upwind one, or the contact's
+    const bool left = sup ? supL : Ss >= 0.;
+    const double rK = left ? rL : rR, uK = left ? uL : uR, tK = left ? tL : tR, pK = left ? pL : pR;
+    const double SK = left ? SL : SR, yK = left ? yL : yR, dK = left ? dL : dR;  // dK = rK (SK - uK)
+    const double EK = quot(pK, R3_GM1, R3_YGM1) + 0.5 * rK * (uK * uK + tK * tK);
+    const double mK = rK * uK;
+    const double F0 = mK, F1 = mK * uK + pK, F2 = mK * tK, F3 = (EK + pK) * uK;
+    if (sup) {
+        F[0] = F0; F[1] = F1; F[2] = F2; F[3] = F3;
+        return ok;
+    }
+    const double sq = SK - Ss;
+    const double f = quot(dK, sq, recip(sq));
+    const double Us3 = f * (quot(EK, rK, yK) + (Ss - uK) * (Ss + quot(pK, dK, recip(dK))));
+    F[0] = F0 + SK * (f - rK);
+    F[1] = F1 + SK * (f * Ss - mK);
+    F[2] = F2 + SK * (f * tK - rK * tK);
+    F[3] = F3 + SK * (Us3 - EK);
+    return ok && den_ok(sd) && den_ok(sq) && den_ok(dK) && num_ok(sn, EK);
+}
+
+__device__ __noinline__ void r3_hllc_any(const double L[4], const double R[4], double F[4]) { r3_hllc(L, R, F); }
+
 // 2x2-block limiter on U[c][q] (cells c = 0..3: (i0,j0), (i0+1,j0),
 // (i0,j0+1), (i0+1,j0+1)); true if the block changed; *brutal counts a
 // block whose mean itself needed the floor fix  fv_rec3_2d.cu:252-337
@@ -173,9 +294,154 @@ __device__ bool r3_limit_block(double U[4][4], int *brutal)
     return th < 1. || bad;
 }
 
+__device__ __noinline__ double r3_lam_any(double U0, double U1, double U2, double U3)
+{
+    const double U[4] = {U0, U1, U2, U3};
+    double W[4];
+    r3_w(U, W);
+    return fabs(W[1]) + fabs(W[2]) + r3_snd(W[0], W[3]);
+}
+
+__device__ __noinline__ bool r3_limit_any(double U[4][4], int *brutal) { return r3_limit_block(U, brutal); }
+
+// corner c of a 2x2 block by bilinear extrapolation: opposite cell 3 - c,
+// neighbours in the reference's order
+__device__ __forceinline__ void r3_corner(const double U[4][4], int c, double C[4])
+{
+    const int a = c ^ 1, b = c ^ 2;  // (1, 2), (0, 3), (3, 0), (2, 1)
+#pragma unroll
+    for (int q = 0; q < 4; q++) C[q] = (9. * U[c][q] - 3. * U[a][q] - 3. * U[b][q] + U[3 - c][q]) * 0.25;
+}
+
+// r3_limit_block of a block whose mean and corners clear the floors (nearly
+// all): left as it is; false: it needs the limiter
+__device__ __forceinline__ bool r3_clear_block(const double U[4][4])
+{
+    double Ub[4] = {0., 0., 0., 0.};
+#pragma unroll
+    for (int c = 0; c < 4; c++)
+#pragma unroll
+        for (int q = 0; q < 4; q++) Ub[q] += 0.25 * U[c][q];
+    bool ok = true;
+    double r, u, v;
+    double rmin = Ub[0], pmin = r3_p_near(Ub, r, u, v, ok);
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+        double C[4];
+        r3_corner(U, c, C);
+        const double p = r3_p_near(C, r, u, v, ok);
+        rmin = smin<double>(C[0], rmin);
+        pmin = smin<double>(p, pmin);
+    }
+    return ok && rmin >= R3_RHOFLOOR && pmin >= R3_PFLOOR;
+}
+
+// the limiter of a block with an admissible mean, the four corners' pressures
+// of a bisection step side by side in the shared-reciprocal form; false (U
+// untouched): take r3_limit_any
+__device__ __forceinline__ bool r3_limit_near(double U[4][4])
+{
+    double Ub[4] = {0., 0., 0., 0.}, C[4][4];
+#pragma unroll
+    for (int c = 0; c < 4; c++)
+#pragma unroll
+        for (int q = 0; q < 4; q++) Ub[q] += 0.25 * U[c][q];
+    bool ok = true;
+    double r, u, v;
+    const double pb = r3_p_near(Ub, r, u, v, ok);
+    if (!ok || !(Ub[0] >= R3_RHOFLOOR) || !(pb >= R3_PFLOOR)) return false;
+    double th = 1.;
+#pragma unroll
+    for (int c = 0; c < 4; c++) {
+        r3_corner(U, c, C[c]);
+        if (C[c][0] < R3_RHOFLOOR) {
+            const double d = Ub[0] - C[c][0];
+            if (d > 0.) th = smin<double>((Ub[0] - R3_RHOFLOOR) / d, th);
+        }
+    }
+    if (th < 1.)
+#pragma unroll
+        for (int c = 0; c < 4; c++)
+#pragma unroll
+            for (int q = 0; q < 4; q++) C[c][q] = Ub[q] + th * (C[c][q] - Ub[q]);
+    bool bad = false;
+#pragma unroll
+    for (int c = 0; c < 4; c++) bad = bad || C[c][0] < R3_RHOFLOOR || r3_p_near(C[c], r, u, v, ok) < R3_PFLOOR;
+    double lo = 0., hi = 1.;
+    if (bad) {
+#pragma unroll 1
+        for (int it = 0; it < 30; it++) {
+            const double mid = 0.5 * (lo + hi);
+            bool out = false;
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                double V[4];
+#pragma unroll
+                for (int q = 0; q < 4; q++) V[q] = Ub[q] + mid * (C[c][q] - Ub[q]);
+                const double p = r3_p_near(V, r, u, v, ok);
+                out = out || V[0] < R3_RHOFLOOR || p < R3_PFLOOR;
+            }
+            hi = out ? mid : hi;
+            lo = out ? lo : mid;
+        }
+    }
+    if (!ok) return false;
+#pragma unroll
+    for (int c = 0; c < 4; c++)
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            if (th < 1.) U[c][q] = Ub[q] + th * (U[c][q] - Ub[q]);
+            if (bad) U[c][q] = Ub[q] + lo * (U[c][q] - Ub[q]);
+        }
+    return true;
+}
+
 __device__ __forceinline__ long long r3_at(const GridDev &gd, int j, int i)
 {
     return (long long)(j + RG) * gd.pitch + (i + RG) + gd.xoff;
+}
+
+// the flux of face f of a tile's x- or y-faces into its plane set; SCALE: with
+// the scaling of its states, else only if both clear the floors (false: not
+// stored)
+template <bool XF, bool SCALE>
+__device__ __forceinline__ bool r3_face(const double *Q, int f, double *FP)
+{
+    constexpr int W = XF ? RTX + 1 : RTX, st = XF ? 1 : RSW, os = XF ? RTY * (RTX + 1) : (RTY + 1) * RTX;
+    constexpr int QN = XF ? 1 : 2, QT = XF ? 2 : 1;
+    const int r = f / W, c = f - r * W;
+    const int b = (r + RG) * RSW + (c + RG), a = b - st;
+    double UL[4], UR[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const double *v = Q + q * RPL;
+        const double um = v[a - st], uc = v[a], up = v[b], u2 = v[b + st];
+        UL[q] = fma(2., up, -um + 5. * uc) * (1. / 6.);  // (2 up is exact: the reference's own rounding)
+        UR[q] = (fma(2., uc, 5. * up) - u2) * (1. / 6.);
+    }
+    double WL[4], WR[4], Fn[4];
+    if constexpr (SCALE) {
+        const double UbL[4] = {Q[a], Q[RPL + a], Q[2 * RPL + a], Q[3 * RPL + a]};
+        const double UbR[4] = {Q[b], Q[RPL + b], Q[2 * RPL + b], Q[3 * RPL + b]};
+        r3_scale_near(UbL, UL, WL);
+        r3_scale_near(UbR, UR, WR);
+    } else {
+        const bool l = r3_clear_near(UL, WL), r2 = r3_clear_near(UR, WR);
+        if (!(l && r2)) return false;
+    }
+    const double L[4] = {WL[0], WL[QN], WL[QT], WL[3]}, Rr[4] = {WR[0], WR[QN], WR[QT], WR[3]};
+    if (!r3_hllc_near(L, Rr, Fn)) {
+        if (!SCALE) return false;
+        double A[4], B[4], G[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) { A[q] = L[q]; B[q] = Rr[q]; }
+        r3_hllc_any(A, B, G);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) Fn[q] = G[q];
+    }
+    double *o = FP + f;
+    o[0] = Fn[0]; o[QN * os] = Fn[1]; o[QT * os] = Fn[2]; o[3 * os] = Fn[3];
+    return true;
 }
 
 // one SSP-RK3 stage                             fv_rec3_2d.cu:166-353
@@ -187,6 +453,8 @@ __global__ void __launch_bounds__(RNT, 2) rec3_stage_kernel(const GridDev gd, in
     double *FY = FX + 4 * RTY * (RTX + 1);             // [4][RTY+1][RTX]
     __shared__ TileCtl s_ctl;
     __shared__ double s_red[RNT / 32];
+    __shared__ int s_nlist;
+    __shared__ unsigned short s_list[RNF];  // faces that need the scaling
     const int tid = threadIdx.x, n = gd.n, np = n + 2 * RG;
     const double *in = (const double *)(stage == 2 ? gd.k1 : stage == 3 ? gd.k2 : gd.st[0]);
     const double *u0 = (const double *)gd.st[0];
@@ -199,7 +467,10 @@ __global__ void __launch_bounds__(RNT, 2) rec3_stage_kernel(const GridDev gd, in
 
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const int tx0 = (t % gd.tiles_x) * RTX, ty0 = (t / gd.tiles_x) * RTY;
-        if (tid == 0) s_ctl = tile_control<P64>(gd.ctrl, stage, t == 0);
+        if (tid == 0) {
+            s_ctl = tile_control<P64>(gd.ctrl, stage, t == 0);
+            s_nlist = 0;
+        }
         __syncthreads();
         const TileCtl ctl = s_ctl;
         if (!ctl.run) {
@@ -214,34 +485,25 @@ __global__ void __launch_bounds__(RNT, 2) rec3_stage_kernel(const GridDev gd, in
             for (int q = 0; q < 4; ++q) Q[q * RPL + k] = inb ? in[e + q * gd.plane] : (q == 0 ? 1. : q == 3 ? 2.5 : 0.);
         }
         __syncthreads();
-        // ---- faces: x-face (r, c) lies between cells c-1 and c ------------
-        for (int f = tid; f < (RTX + 1) * RTY + RTX * (RTY + 1); f += RNT) {
-            const bool xf = f < (RTX + 1) * RTY;
-            int r, c, st;
-            if (xf) { r = f / (RTX + 1); c = f - r * (RTX + 1); st = 1; }
-            else { const int f2 = f - (RTX + 1) * RTY; r = f2 / RTX; c = f2 - r * RTX; st = RSW; }
-            const int b = (r + RG) * RSW + (c + RG), a = b - st;
-            double UL[4], UR[4], UbL[4], UbR[4];
-            for (int q = 0; q < 4; ++q) {
-                const double *v = Q + q * RPL;
-                const double um = v[a - st], uc = v[a], up = v[b], u2 = v[b + st];
-                UL[q] = (-um + 5. * uc + 2. * up) * (1. / 6.);
-                UR[q] = (2. * uc + 5. * up - u2) * (1. / 6.);
-                UbL[q] = uc;
-                UbR[q] = up;
-            }
-            double WL[4], WR[4], L[4], Rr[4], Fn[4];
-            r3_scale_w(UbL, UL, WL);
-            r3_scale_w(UbR, UR, WR);
-            const int QN = xf ? 1 : 2, QT = xf ? 2 : 1;
-            L[0] = WL[0]; L[1] = WL[QN]; L[2] = WL[QT]; L[3] = WL[3];
-            Rr[0] = WR[0]; Rr[1] = WR[QN]; Rr[2] = WR[QT]; Rr[3] = WR[3];
-            r3_hllc(L, Rr, Fn);
-            double *o = xf ? FX + r * (RTX + 1) + c : FY + r * RTX + c;
-            const int os = xf ? RTY * (RTX + 1) : (RTY + 1) * RTX;
-            o[0] = Fn[0]; o[QN * os] = Fn[1]; o[QT * os] = Fn[2]; o[3 * os] = Fn[3];
-        }
+        // ---- faces: x-face (r, c) lies between cells c-1 and c; a face with
+        //      a state below the floors goes on the list ------------------------
+        for (int f = tid; f < RTY * (RTX + 1); f += RNT)
+            if (!r3_face<true, false>(Q, f, FX)) s_list[atomicAdd(&s_nlist, 1)] = (unsigned short)f;
+        for (int f = tid; f < (RTY + 1) * RTX; f += RNT)
+            if (!r3_face<false, false>(Q, f, FY))
+                s_list[atomicAdd(&s_nlist, 1)] = (unsigned short)(f + RTY * (RTX + 1));
         __syncthreads();
+        // ---- the listed faces, one a thread, so that their bisections (25
+        //      dependent steps a side) run side by side ---------------------------
+        const int nl = s_nlist;
+        if (nl > 0) {
+            for (int m = tid; m < nl; m += RNT) {
+                const int f = s_list[m];
+                if (f < RTY * (RTX + 1)) r3_face<true, true>(Q, f, FX);
+                else r3_face<false, true>(Q, f - RTY * (RTX + 1), FY);
+            }
+            __syncthreads();
+        }
         // ---- per 2x2 block, one thread: residual of its four cells in the
         //      serial scatter's order, RK combination, the block limiter,
         //      stores with the periodic ghost images, stage-3 wave speed -----
@@ -250,9 +512,11 @@ __global__ void __launch_bounds__(RNT, 2) rec3_stage_kernel(const GridDev gd, in
             const int c0 = 2 * ib, r0 = 2 * jb;
             if (tx0 + c0 >= n || ty0 + r0 >= n) continue;  // n even: the block is whole
             double U[4][4];
+#pragma unroll
             for (int cc = 0; cc < 4; cc++) {
                 const int r = r0 + (cc >> 1), c = c0 + (cc & 1), i = tx0 + c, j = ty0 + r;
                 const long long e = r3_at(gd, j, i);
+#pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     const double *fx = FX + q * RTY * (RTX + 1) + r * (RTX + 1) + c;
                     const double *fy = FY + q * (RTY + 1) * RTX + r * RTX + c;
@@ -268,14 +532,31 @@ __global__ void __launch_bounds__(RNT, 2) rec3_stage_kernel(const GridDev gd, in
                     U[cc][q] = ca * qa + cb * (qb + ctl.dt * L);
                 }
             }
-            r3_limit_block(U, &brutal);
+            if (!r3_clear_block(U) && !r3_limit_near(U)) {
+                double T[4][4];
+                int nb = 0;
+#pragma unroll
+                for (int c = 0; c < 4; c++)
+#pragma unroll
+                    for (int q = 0; q < 4; q++) T[c][q] = U[c][q];
+                r3_limit_any(T, &nb);
+                brutal += nb;
+#pragma unroll
+                for (int c = 0; c < 4; c++)
+#pragma unroll
+                    for (int q = 0; q < 4; q++) U[c][q] = T[c][q];
+            }
+#pragma unroll
             for (int cc = 0; cc < 4; cc++) {
                 const int i = tx0 + c0 + (cc & 1), j = ty0 + r0 + (cc >> 1);
                 put_cell<double>(gd, out, j, i, U[cc]);
                 if (stage == 3) {
-                    double W[4];
-                    r3_w(U[cc], W);
-                    lacc = smax<double>(fabs(W[1]) + fabs(W[2]) + r3_snd(W[0], W[3]), lacc);
+                    double r, u, v;
+                    bool ok = true;
+                    const double p = smax<double>(r3_p_near(U[cc], r, u, v, ok), R3_PFLOOR);
+                    const double x = quot(R3_GAM * p, r, recip(r));
+                    const double lam = fabs(u) + fabs(v) + root(x);
+                    lacc = smax<double>(ok && den_ok(x) ? lam : r3_lam_any(U[cc][0], U[cc][1], U[cc][2], U[cc][3]), lacc);
                 }
             }
         }
