@@ -30,6 +30,9 @@ FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", 
 # reference's arithmetic operation for operation, so no multiply-add
 # contraction there
 FILE_FLAGS = {"fvb_rec3.cu": ["-fmad=false"], "fvb_d2av.cu": ["-fmad=false"],
+              # the FP64 stage kernel writes its fused multiply-adds out
+              "fvb_stage64_up7.cu": ["-fmad=false"], "fvb_stage64_rs.cu": ["-fmad=false"],
+              "fvb_stage64_orders.cu": ["-fmad=false"],
               # the FP32-compensated kernel: single-precision denormals flushed
               # to zero, so its reciprocals and square roots are the bare
               # hardware approximations without the denormal-range fix-ups

@@ -79,9 +79,9 @@ void grid_pointers(GridDev &gd, void *base, const Geometry &G, int prec)
 
 BufView view_of(const GridDev &gd) { return BufView{gd.n, gd.g, gd.pitch, gd.xoff, gd.plane}; }
 
-void tile_dims(int shape, int n, int &tiles_x, int &tiles)
+void tile_dims(int prec, int shape, int n, int &tiles_x, int &tiles)
 {
-    const TileShape &t = kTileShapes[shape];
+    const TileShape &t = tile_shape(prec, shape);
     tiles_x = (n + t.tx - 1) / t.tx;
     tiles = tiles_x * ((n + t.ty - 1) / t.ty);
 }
@@ -396,8 +396,7 @@ fvb_status fvb_create(const fvb_config *cfg, fvb_solver **out)
     s->gd.tmap = nullptr;
     s->gd.bcx = cfg->bc_x;
     s->gd.bcy = cfg->bc_y;
-    s->gd.h = cfg->length / cfg->n;
-    s->gd.gam = cfg->gamma;
+    set_scales(s->gd, cfg->length / cfg->n, cfg->gamma);
     e = cudaMallocHost(&s->ctrl_host, sizeof(Ctrl));
     if (e != cudaSuccess) { fvb_destroy(s); return cuda_fail(e, "cudaMallocHost"); }
 
@@ -414,7 +413,7 @@ fvb_status fvb_create(const fvb_config *cfg, fvb_solver **out)
         return FVB_OK;
     }
     s->shape = cfg->tile >= 0 ? cfg->tile : autotune_shape(s->prec, s->order, cfg->n);
-    tile_dims(s->shape, s->n, s->gd.tiles_x, s->tiles);
+    tile_dims(s->prec, s->shape, s->n, s->gd.tiles_x, s->tiles);
     {
         CUtensorMap maps[TM_COUNT];
         if (encode_tile_maps(s->gd, s->prec, s->order, s->shape, maps)) {
@@ -875,18 +874,16 @@ fvb_status fvb_up_rhs(const void *Qp, void *rhs, void *lam, int n, int np, int o
     gd.pitch = np;
     gd.xoff = 0;
     gd.plane = (long long)np * np;
-    gd.h = h;
-    gd.gam = gamma;
+    set_scales(gd, h, gamma);
     gd.st[0] = (void *)Qp;
     gd.ctrl = nullptr;
-    const int shape = 0;
+    const int shape = 0, prec = dtype == FVB_F64 ? P64 : P32;
     int tiles;
-    tile_dims(shape, n, gd.tiles_x, tiles);
+    tile_dims(prec, shape, n, gd.tiles_x, tiles);
     a.ntiles_static = tiles;
     a.stage = 0;
     a.rhs = rhs;
     a.lam = lam;
-    int prec = dtype == FVB_F64 ? P64 : P32;
     cudaError_t e = launch_stage(prec, order, shape, a, tiles, (cudaStream_t)stream);
     return e == cudaSuccess ? FVB_OK : cuda_fail(e, "fvb_up_rhs");
 }

@@ -114,12 +114,11 @@ static cudaError_t capture(fvb_batch *b, int parity)
 // (stream-ordered, so the next launch sees it).
 static fvb_status upload_table(fvb_batch *b)
 {
-    const TileShape &ts = kTileShapes[b->shape];
     size_t total = 0;
     for (auto &I : b->inst)
         if (I.live && I.in_table) {
             int tx, nt;
-            tile_dims(b->shape, I.G.n, tx, nt);
+            tile_dims(b->prec, b->shape, I.G.n, tx, nt);
             total += nt;
         }
     if (total > b->tiles_cap) {
@@ -143,12 +142,11 @@ static fvb_status upload_table(fvb_batch *b)
         Instance &I = b->inst[slot];
         if (!(I.live && I.in_table)) continue;
         int tx, nt;
-        tile_dims(b->shape, I.G.n, tx, nt);
+        tile_dims(b->prec, b->shape, I.G.n, tx, nt);
         I.gd.tiles_x = tx;
         b->desc_host[slot] = I.gd;
         for (int t = 0; t < nt; ++t) b->tiles_host[k++] = TileRef{slot, t};
     }
-    (void)ts;
     *b->ntiles_host = (int)k;
     e = cudaMemcpyAsync(b->desc_dev, b->desc_host, sizeof(GridDev) * b->inst.size(), cudaMemcpyHostToDevice,
                         b->stream);
@@ -292,14 +290,13 @@ fvb_status fvb_batch_add(fvb_batch *b, const fvb_instance_desc *d, int *id)
     grid_pointers(I.gd, I.block, G, b->cfg.precision);
     I.gd.bcx = d->bc_x;
     I.gd.bcy = d->bc_y;
-    I.gd.h = d->length / d->n;
-    I.gd.gam = d->gamma;
+    set_scales(I.gd, d->length / d->n, d->gamma);
     I.gd.ctrl = b->ctrl_dev + slot;
     I.gd.tmap = nullptr;
     {
         // descriptors for the batch's tile shape; every batched grid uses TMA
         int tx, nt;
-        tile_dims(b->shape, d->n, tx, nt);
+        tile_dims(b->prec, b->shape, d->n, tx, nt);
         I.gd.tiles_x = tx;
         CUtensorMap maps[TM_COUNT];
         if (!encode_tile_maps(I.gd, b->prec, 7, b->shape, maps)) {

@@ -34,7 +34,7 @@ size_t prec_elem(int prec);
 Geometry make_geometry(int n, int g, int prec);
 void grid_pointers(GridDev &gd, void *base, const Geometry &G, int prec);
 BufView view_of(const GridDev &gd);
-void tile_dims(int shape, int n, int &tiles_x, int &tiles);
+void tile_dims(int prec, int shape, int n, int &tiles_x, int &tiles);
 void case_defaults(fvb_case *c, int kind, double x0, double y0, double L);
 
 // tile variant for a grid size (fvb_tune.cpp)

@@ -45,17 +45,27 @@ struct GridDev {
     long long plane;
     int bcx, bcy;
     double h, gam;
+    double inv_h, igm1;  // 1 / h, 1 / (gam - 1)
     void *st[2];    // state: prim (F64/F32, st[0] only) or conserved hi (F32C, ping-pong)
     void *lo[2];    // F32C: lo words of the conserved state; KEEP: lo[0] holds the cells' entropies
     void *k1, *k2;  // stage outputs: U1/U2 primitives (F64/F32) or increments d1/d2 (F32C)
     Ctrl *ctrl;
-    const CUtensorMap *tmap;  // TMA descriptors of st[0], st[1], k1, k2 for the
-                              // kernel's halo box (device memory); null: plain loads
+    const CUtensorMap *tmap;  // TMA descriptors of st[0], st[1], k1, k2 for the kernel's halo
+                              // box and of st[0] for a tile (device memory); null: plain loads
     int tiles_x;    // tiles along x for the kernel's tile width
     int pad;
 };
 
-enum { TM_ST0 = 0, TM_ST1 = 1, TM_K1 = 2, TM_K2 = 3, TM_COUNT = 4 };
+inline void set_scales(GridDev &gd, double h, double gam)
+{
+    gd.h = h;
+    gd.gam = gam;
+    gd.inv_h = 1.0 / h;
+    gd.igm1 = 1.0 / (gam - 1.0);
+}
+
+// TM_U0: the FP64 kernel's U0 tile (no halo) of st[0]
+enum { TM_ST0 = 0, TM_ST1 = 1, TM_K1 = 2, TM_K2 = 3, TM_U0 = 4, TM_COUNT = 5 };
 
 // Tile-table entry of the batched launch: grid index and tile index.
 struct TileRef {
@@ -95,9 +105,18 @@ struct TileShape {
 constexpr int kNumTileShapes = 7;
 constexpr TileShape kTileShapes[kNumTileShapes] = {
     {32, 15, 256}, {32, 7, 128}, {64, 7, 256}, {16, 15, 256}, {32, 9, 256}, {32, 16, 256}, {32, 14, 256}};
+// the FP64 kernel's shapes of the same variant numbers (fvb_stage64.cuh): pairs
+// of faces and of cells a thread, NT = TX (TY + 1) / 2, or the split form, one
+// face a thread, NT = 2 TX (TY + 1)
+constexpr TileShape kTileShapes64[kNumTileShapes] = {
+    {32, 15, 256}, {32, 7, 128}, {64, 7, 256}, {16, 7, 256}, {16, 7, 64}, {32, 7, 512}, {16, 3, 128}};
+constexpr const TileShape &tile_shape(int prec, int shape)
+{
+    return prec == P64 ? kTileShapes64[shape] : kTileShapes[shape];
+}
 // the variant whose FP32-compensated kernel evaluates faces and cells as
-// pairs of rows TY/2 apart (fvb_stage32c.cu, stage32p_kernel); the FP64 and
-// FP32 kernels treat it as one more tile shape
+// pairs of rows TY/2 apart (fvb_stage32c.cu, stage32p_kernel); the FP32 kernel
+// treats it as one more tile shape
 constexpr int kRowPairShape = 6;
 
 // TMA descriptors (fvb_stage.cu): encode the four maps of a grid for a
@@ -105,6 +124,17 @@ constexpr int kRowPairShape = 6;
 bool encode_tile_maps(const GridDev &gd, int prec, int order, int shape, CUtensorMap out[TM_COUNT]);
 // stream-ordered copy of encoded maps into device memory (dst 64-byte aligned)
 cudaError_t put_tile_maps(const CUtensorMap maps[TM_COUNT], CUtensorMap *dst, cudaStream_t s);
+
+// a stage kernel as launched: for one grid, for a tile table (null where the
+// batched form is not built), its dynamic shared memory and threads
+struct StageKernel {
+    void *fn, *fn_batched;
+    size_t smem;
+    int nt;
+};
+// the FP64 stage kernel of an order, a tile variant and a solver on the
+// reconstructed states (fvb_stage64.cuh); fn null: not built
+StageKernel stage64_kernel_of(int order, int shape, int rs);
 
 // the FP32-compensated stage kernel of a tile shape and its shared memory
 // (fvb_stage32c.cu)
@@ -115,7 +145,6 @@ size_t stage32c_smem(int shape);
 // the FP64 UP7 kernel -- 0 HLLC, 1 HLL, 2 Roe
 cudaError_t launch_stage(int prec, int order, int shape, const StageArgs &a, int grid_ctas,
                          cudaStream_t s, int rs = 0);
-size_t stage_smem_bytes(int prec, int order, int shape, int rs = 0);
 int stage_max_ctas_per_sm(int prec, int order, int shape, int rs = 0);
 
 // What a persistent launch of kernel `fn` with `threads` threads and `smem`

@@ -71,8 +71,7 @@ extern "C" fvb_status fvb_step_noalloc(double *Qp, int n, int np, double h, doub
     gd.plane = (long long)np * np;
     gd.bcx = bc_x;
     gd.bcy = bc_y;
-    gd.h = h;
-    gd.gam = gamma;
+    set_scales(gd, h, gamma);
     gd.st[0] = Qp;
     gd.st[1] = nullptr;
     gd.lo[0] = gd.lo[1] = nullptr;
@@ -82,7 +81,7 @@ extern "C" fvb_status fvb_step_noalloc(double *Qp, int n, int np, double h, doub
     gd.tmap = nullptr;
     const int shape = 0;
     int tiles;
-    tile_dims(shape, n, gd.tiles_x, tiles);
+    tile_dims(P64, shape, n, gd.tiles_x, tiles);
     int per_sm = stage_max_ctas_per_sm(P64, 7, shape), sms = 0, dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);

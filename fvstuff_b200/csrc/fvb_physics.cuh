@@ -195,15 +195,6 @@ __device__ __forceinline__ void hlle(const R L[4], const R Rr[4], R F[4], const 
     F[3] = (SR * FL3 - SL * FR3 + SRL * (ER - EL)) / dS;
 }
 
-// ===========================================================================
-// Division-free forms for the throughput paths (FP64 plain and FP32c).  The
-// same formulas as above, with each quotient written as a product with one
-// reciprocal, the reciprocals shared where the reference divides by the same
-// quantity twice, 1/(gamma-1) precomputed, and the cell-centred sound speed
-// and energy of the HLLE states taken from per-cell values computed once.
-// Results differ from the reference's association order by a few ulp.
-// ===========================================================================
-
 // Reciprocal and square root per arithmetic type.  Every argument on these
 // paths is a positive normal number (densities and pressures are floored at
 // 1e-14, wave-speed spans at 1e-10, sound speeds squared at 1e-14).
@@ -251,264 +242,5 @@ __device__ __forceinline__ double fsqrt(double x)
 #endif
 __device__ __forceinline__ float frcp(float x) { return __fdividef(1.0f, x); }
 __device__ __forceinline__ float fsqrt(float x) { return x * rsqrtf(x); }
-
-// FP64 sound speed c = sqrt(max(gp / r, 1e-14)) from gp = gamma p and the
-// density, as gp / sqrt(gp r) = gp * rsqrt(gp r): the reciprocal root (seed
-// and the third-order step of fsqrt) replaces a reciprocal of r and a
-// square root; within 2 ulp of the correctly rounded sqrt(gp / r).  The
-// floor test gp > 1e-14 r is cs2 > 1e-14 without the division (r > 0).
-// sqrt(gp / r) without the floor (gp, r >= 1e-14)
-__device__ __forceinline__ double snd_rsq_raw(double gp, double r)
-{
-#if FVB_EXACT_RCP_SQRT
-    return sqrt(gp / r);
-#else
-    const double x = gp * r;
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-(x * y), y, 1.0);
-    y = fma(y, e * fma(e, 0.375, 0.5), y);
-    return gp * y;
-#endif
-}
-// (both sides evaluated and one selected: no branch)
-__device__ __forceinline__ double snd_rsq(double gp, double r)
-{
-    const double c = snd_rsq_raw(gp, r);
-    return gp > 1e-14 * r ? c : 1e-7;
-}
-
-template <class R> struct GasF {
-    R gam, igm1, gm1;  // gamma, 1/(gamma-1), gamma-1
-};
-
-// UP-ORDER face values with the weights pre-divided by their denominator
-template <class R, int ORDER>
-__device__ __forceinline__ void upface_fast(const R *s, R &vL, R &vR)
-{
-    if constexpr (ORDER == 3) {
-        const R k = R(1.0 / 6.0);
-        vL = (-s[0] + R(5) * s[1] + R(2) * s[2]) * k;
-        vR = (R(2) * s[1] + R(5) * s[2] - s[3]) * k;
-    } else if constexpr (ORDER == 5) {
-        const R k = R(1.0 / 60.0);
-        vL = (R(2) * s[0] - R(13) * s[1] + R(47) * s[2] + R(27) * s[3] - R(3) * s[4]) * k;
-        vR = (-R(3) * s[1] + R(27) * s[2] + R(47) * s[3] - R(13) * s[4] + R(2) * s[5]) * k;
-    } else if constexpr (ORDER == 9) {
-#define FVB_W9(a) R((a) / 2520.0)
-        vL = FVB_W9(3.) * s[0] + FVB_W9(-25.) * s[1] + FVB_W9(101.) * s[2] + FVB_W9(-319.) * s[3]
-             + FVB_W9(2765.) * s[4] + FVB_W9(2139.) * s[5] + FVB_W9(-533.) * s[6] + FVB_W9(97.) * s[7]
-             + FVB_W9(-11.) * s[8];
-        vR = FVB_W9(-11.) * s[1] + FVB_W9(97.) * s[2] + FVB_W9(-533.) * s[3] + FVB_W9(2139.) * s[4]
-             + FVB_W9(2765.) * s[5] + FVB_W9(-319.) * s[6] + FVB_W9(101.) * s[7] + FVB_W9(-25.) * s[8]
-             + FVB_W9(3.) * s[9];
-#undef FVB_W9
-    } else {
-        // weights pre-divided: one multiply and six fused multiply-adds a side
-#define FVB_W7(a) R((a) / 420.0)
-        vL = FVB_W7(-3.) * s[0] + FVB_W7(25.) * s[1] + FVB_W7(-101.) * s[2] + FVB_W7(319.) * s[3]
-             + FVB_W7(214.) * s[4] + FVB_W7(-38.) * s[5] + FVB_W7(4.) * s[6];
-        vR = FVB_W7(4.) * s[1] + FVB_W7(-38.) * s[2] + FVB_W7(214.) * s[3] + FVB_W7(319.) * s[4]
-             + FVB_W7(-101.) * s[5] + FVB_W7(25.) * s[6] + FVB_W7(-3.) * s[7];
-#undef FVB_W7
-    }
-}
-
-// sound speed and total energy of a cell state (rho, a, b, p)
-template <class R>
-__device__ __forceinline__ void cell_ce(R r, R a, R b, R p, const GasF<R> &gs, R &c, R &E)
-{
-    if constexpr (sizeof(R) == 8) {
-        c = snd_rsq(gs.gam * p, r);
-    } else {
-        R cs2 = gs.gam * p * frcp(r);
-        c = fsqrt(cs2 > FVB_LIT(R, 1e-14) ? cs2 : FVB_LIT(R, 1e-14));
-    }
-    E = p * gs.igm1 + R(0.5) * r * (a * a + b * b);
-}
-
-// Blended face flux, normal frame: (1-s) HLLC(L, R) + s HLLE(WL, WR) with
-// s the pressure-jump sensor of the two cells.  L, Rv: floored UP
-// reconstructions; WL, WR: cell states with their sound speeds cW* and
-// energies EW*.                               fv_up7_ducros_2d.cu:237-328, :433
-//
-// RS selects the solver on the reconstructed states: 0 HLLC (fv_up7), 1 HLL,
-// 2 Roe with the Harten-Hyman entropy fix (carb_fv_2d.cu:116-211, the
-// riemann_n alternatives of carb_fv), always blended with the HLLE of the
-// cell states by the Ducros sensor.
-template <class R>
-__device__ __forceinline__ void hll_fast(const R L[4], const R Rv[4], const GasF<R> &gs, R Fh[4])
-{
-    const R zero = R(0);
-    const R rL = L[0], uL = L[1], tL = L[2], pL = L[3];
-    const R rR = Rv[0], uR = Rv[1], tR = Rv[2], pR = Rv[3];
-    // sound speed without a floor, as carb_fv_2d.cu:60-61 (rho, p >= 1e-14)
-    const R cL = snd_rsq_raw(gs.gam * pL, rL), cR = snd_rsq_raw(gs.gam * pR, rR);
-    const R EL = pL * gs.igm1 + R(0.5) * rL * (uL * uL + tL * tL);
-    const R ER = pR * gs.igm1 + R(0.5) * rR * (uR * uR + tR * tR);
-    // Einfeldt's form of the two-wave average: FL, FR or the subsonic
-    // average without selects
-    const R SL = smin<R>(smin<R>(uL - cL, uR - cR), zero), SR = smax<R>(smax<R>(uL + cL, uR + cR), zero);
-    const R inv = frcp(SR - SL), SRL = SR * SL;
-    const R mL = rL * uL, mR = rR * uR;
-    Fh[0] = (SR * mL - SL * mR + SRL * (rR - rL)) * inv;
-    Fh[1] = (SR * (mL * uL + pL) - SL * (mR * uR + pR) + SRL * (mR - mL)) * inv;
-    Fh[2] = (SR * (mL * tL) - SL * (mR * tR) + SRL * (rR * tR - rL * tL)) * inv;
-    Fh[3] = (SR * ((EL + pL) * uL) - SL * ((ER + pR) * uR) + SRL * (ER - EL)) * inv;
-}
-
-template <class R>
-__device__ __forceinline__ void roe_fast(const R L[4], const R Rv[4], const GasF<R> &gs, R Fh[4])
-{
-    const R zero = R(0);
-    const R rL = L[0], uL = L[1], tL = L[2], pL = L[3];
-    const R rR = Rv[0], uR = Rv[1], tR = Rv[2], pR = Rv[3];
-    const R ip = frcp(rL * rR);
-    const R irL = rR * ip, irR = rL * ip;
-    const R cL = fsqrt(gs.gam * pL * irL), cR = fsqrt(gs.gam * pR * irR);
-    const R sqL = fsqrt(rL), sqR = fsqrt(rR);
-    const R iden = frcp(sqL + sqR);
-    const R a = (sqL * uL + sqR * uR) * iden, b = (sqL * tL + sqR * tR) * iden;  // Roe normal / tangential velocity
-    const R EL = pL * gs.igm1 + R(0.5) * rL * (uL * uL + tL * tL);
-    const R ER = pR * gs.igm1 + R(0.5) * rR * (uR * uR + tR * tR);
-    const R H = (sqL * ((EL + pL) * irL) + sqR * ((ER + pR) * irR)) * iden;
-    const R c2 = gs.gm1 * (H - R(0.5) * (a * a + b * b));
-    const R c = fsqrt(c2 > FVB_LIT(R, 1e-14) ? c2 : FVB_LIT(R, 1e-14));
-    const R ic2 = frcp(c2);
-    const R drho = rR - rL, dun = uR - uL, dut = tR - tL, dp = pR - pL;
-    const R rr = sqL * sqR;
-    const R b1 = (dp - rr * c * dun) * (R(0.5) * ic2);
-    const R b2 = drho - dp * ic2;
-    const R b3 = rr * dut;
-    const R b4 = (dp + rr * c * dun) * (R(0.5) * ic2);
-    // Harten-Hyman: |lambda| below eps/2 replaced by (lambda^2 + eps^2/4)/eps
-    const R lam1 = a - c, lam4 = a + c;
-    const R eps1 = smax<R>(R(2) * ((uR - cR) - (uL - cL)), zero);
-    const R eps4 = smax<R>(R(2) * ((uR + cR) - (uL + cL)), zero);
-    R al1 = dabs<R>(lam1), al4 = dabs<R>(lam4);
-    const R al2 = dabs<R>(a);
-    al1 = al1 < eps1 * R(0.5) ? (lam1 * lam1 + eps1 * eps1 * R(0.25)) * frcp(eps1) : al1;
-    al4 = al4 < eps4 * R(0.5) ? (lam4 * lam4 + eps4 * eps4 * R(0.25)) * frcp(eps4) : al4;
-    const R w1 = al1 * b1, w2 = al2 * b2, w3 = al2 * b3, w4 = al4 * b4;
-    const R d0 = w1 + w2 + w4;
-    const R d1 = w1 * lam1 + w2 * a + w4 * lam4;
-    const R d2 = (w1 + w2 + w4) * b + w3;
-    const R d3 = w1 * (H - a * c) + w2 * R(0.5) * (a * a + b * b) + w3 * b + w4 * (H + a * c);
-    const R mL = rL * uL, mR = rR * uR;
-    Fh[0] = R(0.5) * (mL + mR - d0);
-    Fh[1] = R(0.5) * (mL * uL + pL + mR * uR + pR - d1);
-    Fh[2] = R(0.5) * (mL * tL + mR * tR - d2);
-    Fh[3] = R(0.5) * ((EL + pL) * uL + (ER + pR) * uR - d3);
-}
-
-// Solver on the reconstructed states (normal frame): HLLC, or with RS 1 / 2
-// carb_fv's HLL / Roe.  Branch-free, so its chain can interleave with the
-// HLLE chain where both are evaluated together.
-template <class R, int RS = 0>
-__device__ __forceinline__ void recon_flux_fast(const R L[4], const R Rv[4], const GasF<R> &gs, R Fh[4])
-{
-    const R zero = R(0);
-    if constexpr (RS == 1 || RS == 2) {
-        if constexpr (RS == 1) hll_fast<R>(L, Rv, gs, Fh);
-        else roe_fast<R>(L, Rv, gs, Fh);
-    } else {
-        const R rL = L[0], uL = L[1], tL = L[2], pL = L[3];
-        const R rR = Rv[0], uR = Rv[1], tR = Rv[2], pR = Rv[3];
-        R cL, cR;
-        if constexpr (sizeof(R) == 8) {
-            // no reciprocal of the densities: c = gamma p rsqrt(gamma p rho)
-            cL = snd_rsq(gs.gam * pL, rL);
-            cR = snd_rsq(gs.gam * pR, rR);
-        } else {
-            const R cs2L = gs.gam * pL * frcp(rL), cs2R = gs.gam * pR * frcp(rR);
-            cL = fsqrt(cs2L > FVB_LIT(R, 1e-14) ? cs2L : FVB_LIT(R, 1e-14));
-            cR = fsqrt(cs2R > FVB_LIT(R, 1e-14) ? cs2R : FVB_LIT(R, 1e-14));
-        }
-        const R SL = smin<R>(uL - cL, uR - cR), SR = smax<R>(uL + cL, uR + cR);
-        const R dL = rL * (SL - uL), dR = rR * (SR - uR);
-        const R Ss = (pR - pL + dL * uL - dR * uR) * frcp(dL - dR);
-        // side K: by the contact when subsonic, by the fan when supersonic
-        const bool supL = (SL >= zero);
-        const bool sup = supL || (SR <= zero);
-        const bool left = sup ? supL : (Ss >= zero);
-        const R rK = left ? rL : rR, uK = left ? uL : uR, tK = left ? tL : tR;
-        const R pK = left ? pL : pR, SK = left ? SL : SR;
-        const R dK = left ? dL : dR;
-        // only side K's energy enters the flux: one evaluation, after the
-        // selection (the same expression as for either side)
-        const R EK = pK * gs.igm1 + R(0.5) * rK * (uK * uK + tK * tK);
-        // star terms weighted by SK, or by 0 when supersonic (q forced
-        // finite), so one set of expressions gives both fluxes.  With
-        // dK = rK (SK - uK) and q = 1 / (SK - Ss):  fact = dK q, and
-        //   fact (EK / rK + (Ss - uK)(Ss + pK / dK))
-        //     = q (EK (SK - uK) + (Ss - uK)(dK Ss + pK))   (no 1/rK, no 1/dK);
-        // the tangential momentum flux is the mass flux times tK
-        const R SKw = sup ? zero : SK;
-        const R q = sup ? zero : frcp(SK - Ss);
-        const R fact = dK * q;
-        const R m = rK * uK;
-        Fh[0] = m + SKw * (fact - rK);
-        Fh[1] = m * uK + pK + SKw * (fact * Ss - m);
-        Fh[2] = Fh[0] * tK;
-        Fh[3] = (EK + pK) * uK + SKw * (q * (EK * (SK - uK) + (Ss - uK) * (dK * Ss + pK)) - EK);
-    }
-}
-
-// HLLE of the two cell states (sound speeds cWL, cWR, energies EWL, EWR) and
-// the pressure-jump sensor s of the face, normal frame.
-template <class R>
-__device__ __forceinline__ void hlle_sensor_fast(const R WL[4], const R WR[4], R cWL, R cWR, R EWL, R EWR, R Fl[4],
-                                                 R &sd)
-{
-    const R zero = R(0);
-    const R rL = WL[0], uL = WL[1], tL = WL[2], pL = WL[3];
-    const R rR = WR[0], uR = WR[1], tR = WR[2], pR = WR[3];
-    // Einfeldt's form: with SL- = min(SL, 0), SR+ = max(SR, 0) the HLL
-    // average equals FL, FR or the subsonic average in the three wave
-    // configurations, with no selects
-    const R SL = smin<R>(smin<R>(uL - cWL, uR - cWR), zero), SR = smax<R>(smax<R>(uL + cWL, uR + cWR), zero);
-    const R mL = rL * uL, mR = rR * uR;
-    const R FL1 = mL * uL + pL, FR1 = mR * uR + pR;
-    const R FL2 = mL * tL, FR2 = mR * tR;
-    const R FL3 = (EWL + pL) * uL, FR3 = (EWR + pR) * uR;
-    const R dS = smax<R>(SR - SL, FVB_LIT(R, 1e-10));
-    const R dp = WR[3] - WL[3], ps = WR[3] + WL[3];
-    const R dp2 = dp * dp;
-    const R dd = dp2 + FVB_LIT(R, 0.1) * ps * ps;
-    R idS;
-    if constexpr (sizeof(R) == 8) {
-        // one FP64 reciprocal for the HLLE span and the sensor's
-        // denominator (dS >= 1e-10, dd >= 4e-29: the product is normal)
-        const R ip = frcp(dS * dd);
-        idS = dd * ip;
-        sd = dp2 * (dS * ip);
-    } else {
-        idS = frcp(dS);
-        sd = dp2 * frcp(dd);
-    }
-    const R SRL = SR * SL;
-    Fl[0] = (SR * mL - SL * mR + SRL * (rR - rL)) * idS;
-    Fl[1] = (SR * FL1 - SL * FR1 + SRL * (mR - mL)) * idS;
-    Fl[2] = (SR * FL2 - SL * FR2 + SRL * (rR * tR - rL * tL)) * idS;
-    Fl[3] = (SR * FL3 - SL * FR3 + SRL * (EWR - EWL)) * idS;
-}
-
-// Ducros blend (1 - s) Fh + s Fl
-template <class R>
-__device__ __forceinline__ void ducros_blend(const R Fh[4], const R Fl[4], R sd, R F[4])
-{
-#pragma unroll
-    for (int q = 0; q < 4; ++q) F[q] = Fh[q] + sd * (Fl[q] - Fh[q]);
-}
-
-template <class R, int RS = 0>
-__device__ __forceinline__ void face_flux_fast(const R L[4], const R Rv[4], const R WL[4], const R WR[4], R cWL,
-                                               R cWR, R EWL, R EWR, const GasF<R> &gs, R F[4])
-{
-    R Fh[4], Fl[4], sd;
-    recon_flux_fast<R, RS>(L, Rv, gs, Fh);
-    hlle_sensor_fast<R>(WL, WR, cWL, cWR, EWL, EWR, Fl, sd);
-    ducros_blend<R>(Fh, Fl, sd, F);
-}
 
 }  // namespace fvb

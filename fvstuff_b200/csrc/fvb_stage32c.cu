@@ -154,7 +154,9 @@ __global__ void __launch_bounds__(NT, MinBlocks32c<NT>::v) stage32c_kernel(const
     if (t < ntiles && batched) {
         if (tid < 32) {
             const TileRef r0 = a.tiles[t];
-            start_batched_tile<P32C, G, SW, SH, NT>(a, &s_hdr[0], r0, hdr_word(a, r0, tid), cur, IN, &s_bar, tid);
+            start_batched_tile<P32C>(a, &s_hdr[0], r0, hdr_word(a, r0, tid), &s_bar, tid, [&](const TileHdr &h) {
+                issue_tile_load<P32C, G, SW, SH, NT>(h.gd, a.stage, cur, r0.tile, IN, &s_bar, 0);
+            });
             if (tid == 0 && t + stride < ntiles) s_ref_next = a.tiles[t + stride];
         }
         wait_box(true);
@@ -200,7 +202,7 @@ __global__ void __launch_bounds__(NT, MinBlocks32c<NT>::v) stage32c_kernel(const
         const TileCtl ctl = batched ? s_hdr[slot].ctl : ctl1;
         const int n = gd.n;
         const int tx0 = (tile % gd.tiles_x) * TX, ty0 = (tile / gd.tiles_x) * TY;
-        const float gam = (float)gd.gam, gm1 = (float)gd.gam - 1.0f, igm1 = (float)(1.0 / (gd.gam - 1.0));
+        const float gam = (float)gd.gam, gm1 = (float)gd.gam - 1.0f, igm1 = (float)gd.igm1;
         // ---- 1. stage input U0 + d into W as primitives (+ c, E where the
         //         HLLE reads them, cemask) ------------------------------------
         if (ctl.run) {
@@ -239,8 +241,11 @@ __global__ void __launch_bounds__(NT, MinBlocks32c<NT>::v) stage32c_kernel(const
         if (has_next) {
             if (batched) {
                 if (tid < 32) {
-                    start_batched_tile<P32C, G, SW, SH, NT>(a, &s_hdr[slot ^ 1], ref_next, wnext, cur, IN, &s_bar,
-                                                            tid);
+                    start_batched_tile<P32C>(a, &s_hdr[slot ^ 1], ref_next, wnext, &s_bar, tid,
+                                             [&](const TileHdr &h) {
+                                                 issue_tile_load<P32C, G, SW, SH, NT>(h.gd, a.stage, cur,
+                                                                                      ref_next.tile, IN, &s_bar, 0);
+                                             });
                     if (tid == 0) s_ref_next = ref_after;
                 }
                 next_tma = true;
@@ -265,7 +270,7 @@ __global__ void __launch_bounds__(NT, MinBlocks32c<NT>::v) stage32c_kernel(const
             continue;
         }
         const float dt = (float)ctl.dt;
-        const float dt_h = dt * (float)(1.0 / gd.h);
+        const float dt_h = dt * (float)gd.inv_h;
 
         // ---- 3. face fluxes, x-face p and y-face p as one packed pair -------
         for (int p = tid; p < NP; p += NT) {
@@ -450,7 +455,9 @@ __global__ void __launch_bounds__(NT, MinBlocks32c<NT>::v) stage32p_kernel(const
     if (t < ntiles && batched) {
         if (tid < 32) {
             const TileRef r0 = a.tiles[t];
-            start_batched_tile<P32C, G, SW, SH, NT>(a, &s_hdr[0], r0, hdr_word(a, r0, tid), cur, IN, &s_bar, tid);
+            start_batched_tile<P32C>(a, &s_hdr[0], r0, hdr_word(a, r0, tid), &s_bar, tid, [&](const TileHdr &h) {
+                issue_tile_load<P32C, G, SW, SH, NT>(h.gd, a.stage, cur, r0.tile, IN, &s_bar, 0);
+            });
             if (tid == 0 && t + stride < ntiles) s_ref_next = a.tiles[t + stride];
         }
         wait_box(true);
@@ -490,7 +497,7 @@ __global__ void __launch_bounds__(NT, MinBlocks32c<NT>::v) stage32p_kernel(const
         const TileCtl ctl = batched ? s_hdr[slot].ctl : ctl1;
         const int n = gd.n;
         const int tx0 = (tile % gd.tiles_x) * TX, ty0 = (tile / gd.tiles_x) * TY;
-        const float gam = (float)gd.gam, gm1 = (float)gd.gam - 1.0f, igm1 = (float)(1.0 / (gd.gam - 1.0));
+        const float gam = (float)gd.gam, gm1 = (float)gd.gam - 1.0f, igm1 = (float)gd.igm1;
         // ---- 1. stage input U0 + d into W2 as primitive row pairs (+ c, E
         //         where the HLLE reads them) -----------------------------------
         if (ctl.run) {
@@ -535,8 +542,11 @@ __global__ void __launch_bounds__(NT, MinBlocks32c<NT>::v) stage32p_kernel(const
         if (has_next) {
             if (batched) {
                 if (tid < 32) {
-                    start_batched_tile<P32C, G, SW, SH, NT>(a, &s_hdr[slot ^ 1], ref_next, wnext, cur, IN, &s_bar,
-                                                            tid);
+                    start_batched_tile<P32C>(a, &s_hdr[slot ^ 1], ref_next, wnext, &s_bar, tid,
+                                             [&](const TileHdr &h) {
+                                                 issue_tile_load<P32C, G, SW, SH, NT>(h.gd, a.stage, cur,
+                                                                                      ref_next.tile, IN, &s_bar, 0);
+                                             });
                     if (tid == 0) s_ref_next = ref_after;
                 }
                 next_tma = true;
@@ -561,7 +571,7 @@ __global__ void __launch_bounds__(NT, MinBlocks32c<NT>::v) stage32p_kernel(const
             continue;
         }
         const float dt = (float)ctl.dt;
-        const float dt_h = dt * (float)(1.0 / gd.h);
+        const float dt_h = dt * (float)gd.inv_h;
 
         // ---- 3. face fluxes as row pairs: x-faces, then y-faces -------------
         const f2::V tiny = f2::splat(1e-14f);

@@ -112,6 +112,33 @@ __device__ __forceinline__ void issue_tile_load(const GridDev &gd, int stage, in
     }
 }
 
+// The FP64 kernel's halo box of a tile (fvb_stage64.cuh): SW columns from one
+// (XO) left of the tile's first padded column, which starts the box on an
+// even column; the stage input of `stage`.
+template <int G, int TX, int TY, int SW, int XO, int NT>
+__device__ __forceinline__ void issue_tile_load64(const GridDev &gd, int stage, int tile, double *IN, uint64_t *bar,
+                                                  int tid)
+{
+    constexpr int SH = TY + 2 * G, PL = SW * SH;
+    const int tx0 = (tile % gd.tiles_x) * TX, ty0 = (tile / gd.tiles_x) * TY;
+    if (gd.tmap) {
+        if (tid == 0) {
+            mbar_expect_tx(bar, 4u * PL * sizeof(double));
+            tma_load3(IN, gd.tmap + (stage == 2 ? TM_K1 : stage == 3 ? TM_K2 : TM_ST0), gd.xoff - XO + tx0, ty0, 0,
+                      bar);
+        }
+        return;
+    }
+    const double *src = (const double *)(stage == 2 ? gd.k1 : stage == 3 ? gd.k2 : gd.st[0]);
+    const int np = gd.n + 2 * G;
+    for (int k = tid; k < PL; k += NT) {
+        const int r = k / SW, c = k - r * SW, jp = ty0 + r, ip = tx0 + c - XO;
+        const bool in = jp < np && ip >= 0 && ip < np;
+        const long long e = (long long)jp * gd.pitch + ip + gd.xoff;
+        for (int q = 0; q < 4; ++q) IN[q * PL + k] = in ? src[e + q * gd.plane] : 0.0;
+    }
+}
+
 // Tile headers of a batched launch.  Warp 0 stages them one tile ahead:
 // the table entry of the CTA's next tile is loaded a tile early, and at the
 // top of each tile each lane of warp 0 loads one 8-byte word of the next
@@ -155,10 +182,11 @@ __device__ __forceinline__ unsigned long long hdr_word(const StageArgs &a, TileR
 }
 
 // warp 0: publish the header of tile r into h, evaluate its grid's step
-// control for this stage, and start its halo-box load
-template <int PREC, int G, int SW, int SH, int NT, class R>
+// control for this stage, and start its halo-box load (issue(header), by
+// lane 0, completing on `bar`)
+template <int PREC, class Issue>
 __device__ __forceinline__ void start_batched_tile(const StageArgs &a, TileHdr *h, TileRef r, unsigned long long w,
-                                                   int parity, R *IN, uint64_t *bar, int lane)
+                                                   uint64_t *bar, int lane, Issue issue)
 {
     if (lane < kHdrWords) reinterpret_cast<unsigned long long *>(h)[lane] = w;
     __syncwarp();
@@ -170,7 +198,7 @@ __device__ __forceinline__ void start_batched_tile(const StageArgs &a, TileHdr *
         if (a.stage == 3 && leader && h->ctl.run) leader_finish_from<PREC>(h->c, ctrl);
         if (h->gd.tmap) {
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            issue_tile_load<PREC, G, SW, SH, NT>(h->gd, a.stage, parity, r.tile, IN, bar, 0);
+            issue(*h);
         } else {
             // batched grids load through TMA only: never compute on a box
             // that was not loaded

@@ -46,11 +46,10 @@ float time_shape(int prec, int order, int n, int shape, cudaStream_t s)
         GridDev gd{};
         grid_pointers(gd, block, G, prec == P64 ? FVB_PREC_F64 : prec == P32 ? FVB_PREC_F32 : FVB_PREC_F32C);
         gd.bcx = gd.bcy = FVB_BC_PERIODIC;
-        gd.h = 1.0 / n;
-        gd.gam = 1.4;
+        set_scales(gd, 1.0 / n, 1.4);
         gd.ctrl = (Ctrl *)((char *)block + ctrl_off);
         int tiles;
-        tile_dims(shape, n, gd.tiles_x, tiles);
+        tile_dims(prec, shape, n, gd.tiles_x, tiles);
         CUtensorMap maps[TM_COUNT];
         gd.tmap = nullptr;
         if (encode_tile_maps(gd, prec, order, shape, maps)) {
@@ -142,15 +141,15 @@ int autotune_shape(int prec, int order, int n)
     float best_ms = -1.f;
     const bool log = std::getenv("FVB_AUTOTUNE_LOG") != nullptr;
     for (int shape = 0; shape < kNumTileShapes; ++shape) {
-        // the row-pair variant is used only when asked for: it matches
+        // FP32c's row-pair variant is used only when asked for: it matches
         // variant 5 on large grids within the timing spread, and its 14-row
         // tiles leave more of small grids' last tile row empty
-        if (shape == kRowPairShape) continue;
+        if (prec == P32C && shape == kRowPairShape) continue;
         float ms = time_shape(prec, order, nt, shape, s);
         if (log)
             std::fprintf(stderr, "fvb autotune: precision %d order %d n %d: tile %d (%dx%d, %d threads) %.4f ms\n",
-                         prec, order, nt, shape, kTileShapes[shape].tx, kTileShapes[shape].ty, kTileShapes[shape].nt,
-                         ms);
+                         prec, order, nt, shape, tile_shape(prec, shape).tx, tile_shape(prec, shape).ty,
+                         tile_shape(prec, shape).nt, ms);
         if (ms > 0 && (best_ms < 0 || ms < best_ms)) {
             best_ms = ms;
             best = shape;
