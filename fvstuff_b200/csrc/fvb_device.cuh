@@ -7,6 +7,24 @@
 
 namespace fvb {
 
+// Programmatic dependent launch.  A kernel of the step loops is launched with
+// launch_chained (fvb_internal.h), so its CTAs may become resident while the
+// kernel before it in the stream still runs; grid_dependency() is its first
+// statement that touches global memory: it waits until the kernel before has
+// finished and its writes are visible (also to the TMA loads that follow).
+// grid_release() lets the next kernel's CTAs come in the same way; a CTA
+// calls it before the update of its last tile, so that they take the places
+// of CTAs that are about to end and not those beside the ones that are not.
+__device__ __forceinline__ void grid_release()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void grid_dependency()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("fence.proxy.async;" ::: "memory");
+}
+
 template <int PREC> struct PrecT;
 template <> struct PrecT<P64> { using R = double; using RR = double; };
 template <> struct PrecT<P32> { using R = float; using RR = double; };

@@ -157,6 +157,9 @@ struct LaunchFacts {
     int ctas_per_sm;
     int sms;
 };
+// a launch whose CTAs may start, up to their grid_dependency(), while the
+// kernel before it in the stream ends (fvb_stage.cu)
+cudaError_t launch_chained(const void *fn, int ctas, int threads, size_t smem, cudaStream_t s, void **args);
 cudaError_t launch_facts(const void *fn, int threads, size_t smem, LaunchFacts &out);
 
 }  // namespace fvb

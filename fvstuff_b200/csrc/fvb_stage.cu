@@ -99,6 +99,7 @@ __global__ void __launch_bounds__(NT, MINB) stage32_kernel(const __grid_constant
         s_err = 0;
     }
     __syncthreads();
+    grid_dependency();
 
     // every thread waits on the mbarrier itself (the completed phase makes the
     // TMA bytes visible to it); the barrier after the wait also agrees on s_err
@@ -192,6 +193,7 @@ __global__ void __launch_bounds__(NT, MINB) stage32_kernel(const __grid_constant
         }
         __syncthreads();
 
+        if (!has_next) grid_release();
         // ---- 4. divergence, RK combination, stores ------------------------
         double lmax = 0.0;
 #pragma unroll
@@ -314,6 +316,21 @@ static StageKernel kernel_for(int prec, int order, int shape, int rs = 0)
     case 5: return entry32<5>();
     default: return entry32<6>();
     }
+}
+
+cudaError_t launch_chained(const void *fn, int ctas, int threads, size_t smem, cudaStream_t s, void **args)
+{
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelExC(&cfg, fn, args);
 }
 
 cudaError_t launch_facts(const void *fn, int threads, size_t smem, LaunchFacts &out)
@@ -448,7 +465,7 @@ cudaError_t launch_stage(int prec, int order, int shape, const StageArgs &a, int
     if (err != cudaSuccess) return err;
     if (grid_ctas <= 0) return cudaSuccess;
     void *args[] = {(void *)&a};
-    return cudaLaunchKernel(fn, dim3(grid_ctas), dim3(e.nt), args, e.smem, s);
+    return launch_chained(fn, grid_ctas, e.nt, e.smem, s, args);
 }
 
 }  // namespace fvb

@@ -102,13 +102,14 @@ __global__ void __launch_bounds__(NT, MinBlocks32c<NT>::v) stage32c_kernel(const
 
     const int tid = threadIdx.x;
     constexpr bool batched = BATCHED;
-    const int ntiles = batched ? *a.ntiles : a.ntiles_static;
     const int cur = a.parity, nxt = a.parity ^ 1;
     if (tid == 0) {
         mbar_init(&s_bar, 1);
         s_err = 0;
     }
     __syncthreads();
+    grid_dependency();
+    const int ntiles = batched ? *a.ntiles : a.ntiles_static;
 
     // every thread waits on the mbarrier itself (the completed phase makes the
     // TMA bytes visible to it); the barrier after the wait also agrees on s_err
@@ -312,6 +313,7 @@ __global__ void __launch_bounds__(NT, MinBlocks32c<NT>::v) stage32c_kernel(const
         }
         __syncthreads();
 
+        if (!has_next) grid_release();
         // ---- 4. divergence, RK combination, stores --------------------------
         float lmax = 0.0f;
         for (int k = tid; k < NC; k += NT) {
@@ -416,13 +418,14 @@ __global__ void __launch_bounds__(NT, MinBlocks32c<NT>::v) stage32p_kernel(const
 
     const int tid = threadIdx.x;
     constexpr bool batched = BATCHED;
-    const int ntiles = batched ? *a.ntiles : a.ntiles_static;
     const int cur = a.parity, nxt = a.parity ^ 1;
     if (tid == 0) {
         mbar_init(&s_bar, 1);
         s_err = 0;
     }
     __syncthreads();
+    grid_dependency();
+    const int ntiles = batched ? *a.ntiles : a.ntiles_static;
 
     uint32_t phase = 0;
     auto wait_box = [&](bool tma) {
@@ -627,6 +630,7 @@ __global__ void __launch_bounds__(NT, MinBlocks32c<NT>::v) stage32p_kernel(const
         }
         __syncthreads();
 
+        if (!has_next) grid_release();
         // ---- 4. divergence as pairs, then each cell's RK update -------------
         float lmax = 0.0f;
         const f2::V ndt = f2::splat(-dt_h);

@@ -84,12 +84,13 @@ __global__ void __launch_bounds__(NT, (L64<ORDER, TX, TY, NT>::MINB)) stage64_ke
     __shared__ TileRef s_ref_next;  // batched: table entry of the CTA's next tile
 
     const int tid = threadIdx.x;
-    const int ntiles = BATCHED ? *a.ntiles : a.ntiles_static;
     if (tid == 0) {
         for (int m = 0; m < 3; ++m) mbar_init(&s_bar[m], 1);
         s_err = 0;
     }
     __syncthreads();
+    grid_dependency();
+    const int ntiles = BATCHED ? *a.ntiles : a.ntiles_static;
 
     // every thread waits on the mbarrier itself (the completed phase makes the
     // TMA bytes visible to it); the barrier after the wait also agrees on s_err
@@ -297,6 +298,7 @@ __global__ void __launch_bounds__(NT, (L64<ORDER, TX, TY, NT>::MINB)) stage64_ke
         }
         __syncthreads();
 
+        if (!has_next) grid_release();
         // ---- 5. divergence, RK combination, stores: cells 2k and 2k + 1 of
         //      column c (split: one cell) -----------------------------------
         double lmax = 0.0;

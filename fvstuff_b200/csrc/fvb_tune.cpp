@@ -23,10 +23,13 @@ namespace {
 std::mutex g_mu;
 std::map<std::tuple<int, int, int, int>, int> g_cache;
 
+// <=64, <=96, <=128, <=192, ... <=1024, larger: below about 512^2 cells the
+// choice turns on how the tiles fill the SMs, which changes within a factor
+// of two in n
 int size_class(int n)
 {
     int c = 0;
-    for (int m = 64; m < n && c < 5; m *= 2) ++c;  // <=64, <=128, <=256, <=512, <=1024, larger
+    for (int m = 64; m < n && c < 9; ++c) m = c & 1 ? m / 3 * 4 : m / 2 * 3;
     return c;
 }
 
