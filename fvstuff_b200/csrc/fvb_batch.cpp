@@ -212,8 +212,7 @@ fvb_status fvb_batch_create(const fvb_batch_config *cfg, fvb_batch **out)
     if (e == cudaSuccess) e = cudaMallocHost(&b->ntiles_host, sizeof(int));
     if (e != cudaSuccess) { fvb_batch_destroy(b); return cuda_fail(e, "batch allocation"); }
     std::memset(b->desc_host, 0, sizeof(GridDev) * b->max_inst);
-    // a batched launch walks many tiles, as a large grid does: tune there
-    b->shape = cfg->tile >= 0 ? cfg->tile : autotune_shape(b->prec, 7, 4096);
+    b->shape = cfg->tile >= 0 ? cfg->tile : batch_shape(b->prec);
     int per_sm = stage_max_ctas_per_sm(b->prec, 7, b->shape);
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, cfg->device);

@@ -36,6 +36,13 @@ __device__ __forceinline__ long long gidx(const GridDev &gd, int q, int j, int i
     return (long long)q * gd.plane + (long long)(j + gd.g) * gd.pitch + (i + gd.g) + gd.xoff;
 }
 
+// The same within one plane, as a 32-bit index for the kernels' interior
+// accesses (a plane that fits the device has fewer than 2^32 elements).
+__device__ __forceinline__ unsigned cell_index(const GridDev &gd, int j, int i)
+{
+    return (unsigned)(j + gd.g) * (unsigned)gd.pitch + (unsigned)(i + gd.g + gd.xoff);
+}
+
 // Ghost images of cell i along one axis (index 0 is the cell itself).
 //   reflect:      i < g -> -1-i,  i >= n-g -> 2n-1-i  (normal momentum negated)
 //   periodic:     i < g -> i+n,   i >= n-g -> i-n
@@ -68,11 +75,11 @@ template <class R>
 __device__ __forceinline__ void put_cell(const GridDev &gd, R *buf, int j, int i, const R v[4])
 {
     const long long pl = gd.plane;
-    const long long c = gidx(gd, 0, j, i);
+    const unsigned c = cell_index(gd, j, i);
     buf[c] = v[0];
-    buf[c + pl] = v[1];
-    buf[c + 2 * pl] = v[2];
-    buf[c + 3 * pl] = v[3];
+    (buf + pl)[c] = v[1];
+    (buf + 2 * pl)[c] = v[2];
+    (buf + 3 * pl)[c] = v[3];
     const int g = gd.g, n = gd.n;
     if (i >= g && i < n - g && j >= g && j < n - g) return;
     const int nx = n_images(i, n, g, gd.bcx), ny = n_images(j, n, g, gd.bcy);
@@ -98,11 +105,11 @@ __device__ __forceinline__ void put_cell2(const GridDev &gd, R *bufA, R *bufB, i
                                           const R vb[4])
 {
     const long long pl = gd.plane;
-    const long long c = gidx(gd, 0, j, i);
+    const unsigned c = cell_index(gd, j, i);
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-        bufA[c + q * pl] = va[q];
-        bufB[c + q * pl] = vb[q];
+        (bufA + q * pl)[c] = va[q];
+        (bufB + q * pl)[c] = vb[q];
     }
     const int g = gd.g, n = gd.n;
     if (i >= g && i < n - g && j >= g && j < n - g) return;

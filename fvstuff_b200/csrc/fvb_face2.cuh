@@ -47,6 +47,19 @@ __device__ __forceinline__ V vrsqrt(V a) { return make_float2(rsqrtf(a.x), rsqrt
 // sqrt of x >= 1e-14 as x * rsqrt(x)
 __device__ __forceinline__ V vsqrt(V a) { return mul(a, vrsqrt(a)); }
 
+// error-free sum of double-floats (hi, lo) and float increments d, as df_add
+// (fvb_device.cuh)
+__device__ __forceinline__ void df_add(V &hi, V &lo, V d)
+{
+    const V s = add(hi, d);
+    const V bb = sub(s, hi);
+    const V err = add(sub(hi, sub(s, bb)), sub(d, bb));
+    const V l = add(lo, err);
+    const V h2 = add(s, l);
+    lo = sub(l, sub(h2, s));
+    hi = h2;
+}
+
 struct B {
     bool x, y;
 };
@@ -71,6 +84,16 @@ __device__ __forceinline__ void upface7(const V s[8], V &vL, V &vR)
     vR = fma(FVB_W7(25.), s[6], vR);
     vR = fma(FVB_W7(-3.), s[7], vR);
 #undef FVB_W7
+}
+
+// the floor 1e-14 on the reconstructed rho and p
+__device__ __forceinline__ void floors(V L[4], V R[4])
+{
+    const V tiny = splat(1e-14f);
+    L[0] = vmax(L[0], tiny);
+    R[0] = vmax(R[0], tiny);
+    L[3] = vmax(L[3], tiny);
+    R[3] = vmax(R[3], tiny);
 }
 
 // Blended flux of two faces, normal frame.  L, Rv: floored reconstructions

@@ -39,6 +39,7 @@ void case_defaults(fvb_case *c, int kind, double x0, double y0, double L);
 
 // tile variant for a grid size (fvb_tune.cpp)
 int autotune_shape(int prec, int order, int n);
+int batch_shape(int prec);
 
 // KEEP flux family (fvb_keep.cu): tiles of a grid, one stage (entropy-
 // distance pass + fused stage kernel), and the wave-speed max of a state

@@ -110,14 +110,15 @@ constexpr TileShape kTileShapes[kNumTileShapes] = {
 // face a thread, NT = 2 TX (TY + 1)
 constexpr TileShape kTileShapes64[kNumTileShapes] = {
     {32, 15, 256}, {32, 7, 128}, {64, 7, 256}, {16, 7, 256}, {16, 7, 64}, {32, 7, 512}, {16, 3, 128}};
+// the FP32-compensated kernels' (fvb_stage32c.cu): row pairs where the height
+// is even and NT = TX (TY / 2 + 1) / 2, else an x-face and a y-face a thread
+constexpr TileShape kTileShapes32c[kNumTileShapes] = {
+    {32, 30, 256}, {32, 7, 128}, {64, 14, 256}, {16, 15, 256}, {32, 14, 128}, {32, 16, 256}, {32, 22, 192}};
+constexpr bool row_pairs(const TileShape &t) { return t.ty % 4 == 2 && t.nt == t.tx * (t.ty / 2 + 1) / 2; }
 constexpr const TileShape &tile_shape(int prec, int shape)
 {
-    return prec == P64 ? kTileShapes64[shape] : kTileShapes[shape];
+    return prec == P64 ? kTileShapes64[shape] : prec == P32C ? kTileShapes32c[shape] : kTileShapes[shape];
 }
-// the variant whose FP32-compensated kernel evaluates faces and cells as
-// pairs of rows TY/2 apart (fvb_stage32c.cu, stage32p_kernel); the FP32 kernel
-// treats it as one more tile shape
-constexpr int kRowPairShape = 6;
 
 // TMA descriptors (fvb_stage.cu): encode the four maps of a grid for a
 // tile shape into host memory; false if this grid cannot use TMA
@@ -136,10 +137,8 @@ struct StageKernel {
 // reconstructed states (fvb_stage64.cuh); fn null: not built
 StageKernel stage64_kernel_of(int order, int shape, int rs);
 
-// the FP32-compensated stage kernel of a tile shape and its shared memory
-// (fvb_stage32c.cu)
-void *stage32c_fn(int shape, bool batched);
-size_t stage32c_smem(int shape);
+// the FP32-compensated stage kernel of a tile variant (fvb_stage32c.cu)
+StageKernel stage32c_kernel_of(int shape);
 
 // launchers (fvb_stage.cu).  rs: the solver on the reconstructed states of
 // the FP64 UP7 kernel -- 0 HLLC, 1 HLL, 2 Roe

@@ -304,9 +304,7 @@ static StageKernel kernel_for(int prec, int order, int shape, int rs = 0)
     if (shape < 0 || shape >= kNumTileShapes) return StageKernel{};
     if (prec == P64) return stage64_kernel_of(order, shape, rs);
     if (order != 7 || rs != 0) return StageKernel{};
-    if (prec == P32C)
-        return StageKernel{stage32c_fn(shape, false), stage32c_fn(shape, true), stage32c_smem(shape),
-                           kTileShapes[shape].nt};
+    if (prec == P32C) return stage32c_kernel_of(shape);
     switch (shape) {
     case 0: return entry32<0>();
     case 1: return entry32<1>();

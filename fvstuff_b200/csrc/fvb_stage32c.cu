@@ -6,11 +6,18 @@
 // is evaluated once; the RK combination stores the interior and its ghost
 // images; stage 3 max-reduces the wave speed into the step control.
 //
-// What differs, for FP32 throughput: the faces are evaluated in pairs --
-// x-face p in the low half and y-face p in the high half of packed FP32
-// registers (fvb_face2.cuh) -- so the face arithmetic issues one instruction
-// per two faces; and three CTAs of 256 threads share an SM (68 KB of shared
-// memory and <= 85 registers each).
+// What differs, for FP32 throughput: two faces, or two cells, share the lanes
+// of packed FP32 registers (fvb_face2.cuh), so that their arithmetic issues as
+// one instruction.  Two forms:
+//   * stage32c_kernel pairs x-face p with y-face p, one pair a thread; three
+//     CTAs of 256 threads share an SM (71 KB, 80 registers).  It serves small
+//     grids and batches.
+//   * stage32p_kernel pairs rows half a tile apart and gives a thread four
+//     faces of each direction; two CTAs of 256 threads (112 KB, 128
+//     registers).  It serves large grids.
+// Both give the same bits.  What bounds them is instruction issue and, at 16
+// to 24 warps an SM, the latency of dependent instructions, not memory (a
+// 2048^2 stage is 34 us at the copy bandwidth).
 //
 // State: conserved (rho, rho u, rho v, E) as an FP32 hi/lo pair per value;
 // the stages form increments d1 = dt L(U0), d2 = (d1 + dt L(U1)) / 4 and add
@@ -31,49 +38,146 @@ namespace fvb {
 // per SM, <= 85 registers a thread
 template <int NT> struct MinBlocks32c { static constexpr int v = 768 / NT; };
 
+// The operands of one cell's RK update beside dt L: the stage increment (d1
+// in stage 2, d2 in stage 3) and, in stage 3, the hi / lo pair of U0.
+struct Operands32c {
+    float d[4], h[4], l[4];
+};
+__device__ __forceinline__ void load_operands32c(const GridDev &gd, int stage, int cur, int j, int i, Operands32c &o)
+{
+    if (stage == 1) return;
+    const unsigned e = cell_index(gd, j, i);
+    const float *d = (const float *)(stage == 2 ? gd.k1 : gd.k2);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) o.d[q] = (d + q * gd.plane)[e];
+    if (stage == 3) {
+        const float *h = (const float *)gd.st[cur], *l = (const float *)gd.lo[cur];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            o.h[q] = (h + q * gd.plane)[e];
+            o.l[q] = (l + q * gd.plane)[e];
+        }
+    }
+}
+
+// The floors on a new state that is at one of them (rho, p >= 1e-14); returns
+// its wave speed.
+__device__ __noinline__ float floor_cell32c_(float vh0, float vh1, float vh2, float vh3, float gam, float gm1,
+                                             float *rho, float *E)
+{
+    float w[4];
+    const float ir = frcp(vh0);
+    w[0] = vh0; w[1] = vh1 * ir; w[2] = vh2 * ir;
+    w[3] = gm1 * (vh3 - 0.5f * (vh1 * vh1 + vh2 * vh2) * ir);
+    *rho = vh0;
+    *E = vh3;
+    if (!(w[0] > 1e-14f)) { *rho = 1e-14f; w[0] = 1e-14f; }
+    if (!(w[3] > 1e-14f)) {
+        const float ke = 0.5f * (vh1 * vh1 + vh2 * vh2) / *rho;
+        *E = 1e-14f / gm1 + ke;
+        w[3] = 1e-14f;
+    }
+    const float cs2 = gam * w[3] * frcp(w[0]);
+    return fabsf(w[1]) + fabsf(w[2]) + fsqrt(cs2 > 1e-14f ? cs2 : 1e-14f);
+}
+__device__ __forceinline__ float floor_cell32c(float vh[4], float vl[4], float gam, float gm1)
+{
+    float rho, E;
+    const float lam = floor_cell32c_(vh[0], vh[1], vh[2], vh[3], gam, gm1, &rho, &E);
+    if (rho != vh[0]) vl[0] = 0.f;
+    if (E != vh[3]) vl[3] = 0.f;
+    vh[0] = rho;
+    vh[3] = E;
+    return lam;
+}
+
 // The RK update of one cell from dres = dt L(U) (stage 1: d1 = dres; stage
 // 2: d2 = (d1 + dres) / 4; stage 3: U0 + 2/3 (d2 + dres) added to the hi /
 // lo pair with an error-free sum, floors, stores with ghost images, and the
 // cell's wave speed into lmax).
-__device__ __forceinline__ void update_cell32c(const GridDev &gd, int stage, int cur, int nxt, int j, int i,
-                                               const float dres[4], float gam, float gm1, float &lmax)
+__device__ __forceinline__ void update_cell32c(const GridDev &gd, int stage, int nxt, int j, int i,
+                                               const float dres[4], const Operands32c &o, float gam, float gm1,
+                                               float &lmax)
 {
     if (stage == 1) {
         put_cell<float>(gd, (float *)gd.k1, j, i, dres);
     } else if (stage == 2) {
         float d[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const float d1 = ((const float *)gd.k1)[gidx(gd, q, j, i)];
-            d[q] = 0.25f * (d1 + dres[q]);
-        }
+        for (int q = 0; q < 4; ++q) d[q] = 0.25f * (o.d[q] + dres[q]);
         put_cell<float>(gd, (float *)gd.k2, j, i, d);
     } else {
         float vh[4], vl[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            const long long e = gidx(gd, q, j, i);
-            const float d = (2.0f / 3.0f) * (((const float *)gd.k2)[e] + dres[q]);
-            vh[q] = ((const float *)gd.st[cur])[e];
-            vl[q] = ((const float *)gd.lo[cur])[e];
-            df_add(vh[q], vl[q], d);
+            vh[q] = o.h[q];
+            vl[q] = o.l[q];
+            df_add(vh[q], vl[q], (2.0f / 3.0f) * (o.d[q] + dres[q]));
         }
-        // floors rho, p >= 1e-14 on the new state
-        float w[4];
-        {
-            const float ir = frcp(vh[0]);
-            w[0] = vh[0]; w[1] = vh[1] * ir; w[2] = vh[2] * ir;
-            w[3] = gm1 * (vh[3] - 0.5f * (vh[1] * vh[1] + vh[2] * vh[2]) * ir);
-        }
-        if (!(w[0] > 1e-14f)) { vh[0] = 1e-14f; vl[0] = 0.f; w[0] = 1e-14f; }
-        if (!(w[3] > 1e-14f)) {
-            float ke = 0.5f * (vh[1] * vh[1] + vh[2] * vh[2]) / vh[0];
-            vh[3] = 1e-14f / gm1 + ke; vl[3] = 0.f; w[3] = 1e-14f;
-        }
+        // primitives and wave speed of the new state, floors rho, p >= 1e-14
+        const float ir = frcp(vh[0]);
+        const float u = vh[1] * ir, v = vh[2] * ir;
+        const float ke = __fmul_rn(__fmul_rn(0.5f, __fmaf_rn(vh[1], vh[1], __fmul_rn(vh[2], vh[2]))), ir);
+        const float pr = gm1 * __fsub_rn(vh[3], ke);
+        const float cs2 = gam * pr * ir;
+        const float x = fmaxf(cs2, 1e-14f);
+        float lam = fabsf(u) + fabsf(v) + __fmul_rn(x, rsqrtf(x));  // (not fused: as update_pair32c)
+        if (!(vh[0] > 1e-14f && pr > 1e-14f)) lam = floor_cell32c(vh, vl, gam, gm1);
         put_cell2<float>(gd, (float *)gd.st[nxt], (float *)gd.lo[nxt], j, i, vh, vl);
-        float cs2 = gam * w[3] * frcp(w[0]);
-        float lam = fabsf(w[1]) + fabsf(w[2]) + fsqrt(cs2 > 1e-14f ? cs2 : 1e-14f);
         lmax = fmaxf(lmax, lam);  // (NaN skipped; exact in FP64 below)
+    }
+}
+
+// The same update for two cells in the lanes of packed registers (cells
+// (j0, i) and (j1, i); in0 / in1: inside the grid): the arithmetic of
+// update_cell32c, one packed operation for both.
+__device__ __forceinline__ void update_pair32c(const GridDev &gd, int stage, int nxt, int j0, int j1, int i, bool in0,
+                                               bool in1, const f2::V dr[4], const Operands32c &o0,
+                                               const Operands32c &o1, float gam, float gm1, float &lmax)
+{
+    f2::V d[4];
+    if (stage == 1) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) d[q] = dr[q];
+    } else {
+        const f2::V c = f2::splat(stage == 2 ? 0.25f : 2.0f / 3.0f);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) d[q] = f2::mul(c, f2::add(make_float2(o0.d[q], o1.d[q]), dr[q]));
+    }
+    if (stage <= 2) {
+        float *out = (float *)(stage == 1 ? gd.k1 : gd.k2);
+        const float a[4] = {d[0].x, d[1].x, d[2].x, d[3].x}, b[4] = {d[0].y, d[1].y, d[2].y, d[3].y};
+        if (in0) put_cell<float>(gd, out, j0, i, a);
+        if (in1) put_cell<float>(gd, out, j1, i, b);
+        return;
+    }
+    f2::V h[4], l[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        h[q] = make_float2(o0.h[q], o1.h[q]);
+        l[q] = make_float2(o0.l[q], o1.l[q]);
+        f2::df_add(h[q], l[q], d[q]);
+    }
+    // primitives and wave speed of the new state, floors rho, p >= 1e-14
+    const f2::V ir = f2::rcp(h[0]);
+    const f2::V u = f2::mul(h[1], ir), v = f2::mul(h[2], ir);
+    const f2::V ke = f2::mul(f2::mul(f2::splat(0.5f), f2::fma(h[1], h[1], f2::mul(h[2], h[2]))), ir);
+    const f2::V pr = f2::mul(f2::splat(gm1), f2::sub(h[3], ke));
+    const f2::V cs2 = f2::mul(f2::mul(f2::splat(gam), pr), ir);
+    const f2::V cs = f2::vsqrt(f2::vmax(cs2, f2::splat(1e-14f)));
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+        if (!(m ? in1 : in0)) continue;
+        float vh[4], vl[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            vh[q] = m ? h[q].y : h[q].x;
+            vl[q] = m ? l[q].y : l[q].x;
+        }
+        float lam = fabsf(m ? u.y : u.x) + fabsf(m ? v.y : v.x) + (m ? cs.y : cs.x);
+        if (!(vh[0] > 1e-14f && (m ? pr.y : pr.x) > 1e-14f)) lam = floor_cell32c(vh, vl, gam, gm1);
+        put_cell2<float>(gd, (float *)gd.st[nxt], (float *)gd.lo[nxt], m ? j1 : j0, i, vh, vl);
+        lmax = fmaxf(lmax, lam);
     }
 }
 
@@ -292,9 +396,7 @@ __global__ void __launch_bounds__(NT, MinBlocks32c<NT>::v) stage32c_kernel(const
                 WL[m] = s[G - 1];
                 WR[m] = s[G];
             }
-            const f2::V tiny = f2::splat(1e-14f);
-            L[0] = f2::vmax(L[0], tiny); Rv[0] = f2::vmax(Rv[0], tiny);
-            L[3] = f2::vmax(L[3], tiny); Rv[3] = f2::vmax(Rv[3], tiny);
+            f2::floors(L, Rv);
             const float *cex = W + 4 * PL + bx, *cey = W + 4 * PL + by;
             f2::V F[4];
             f2::face_flux(L, Rv, WL, WR, make_float2(cex[-1], cey[-SW]), make_float2(cex[0], cey[0]),
@@ -326,7 +428,9 @@ __global__ void __launch_bounds__(NT, MinBlocks32c<NT>::v) stage32c_kernel(const
                 const float *fy = FY + q * (TY + 1) * TX + r * TX + c;
                 dres[q] = -((fx[1] - fx[0]) + (fy[TX] - fy[0])) * dt_h;
             }
-            update_cell32c(gd, a.stage, cur, nxt, j, i, dres, gam, gm1, lmax);
+            Operands32c o;
+            load_operands32c(gd, a.stage, cur, j, i, o);
+            update_cell32c(gd, a.stage, nxt, j, i, dres, o, gam, gm1, lmax);
         }
 
         // ---- 5. max wave speed of the new state (stage 3) ------------------
@@ -364,52 +468,67 @@ __global__ void __launch_bounds__(NT, MinBlocks32c<NT>::v) stage32c_kernel(const
 }
 
 // ---------------------------------------------------------------------------
-// Row-pair variant of the compensated stage kernel (tile variant 6).
+// Row-pair form of the compensated stage kernel.
 //
 // The two lanes of every packed register are the same face, or the same
 // cell, in two rows HT = TY / 2 apart: the working tile keeps each quantity
-// as float2 pairs (box row r', box row r' + HT) for r' in [0, HT + 2G), so
-// one 64-bit shared load fetches a stencil point for both faces, x-faces
-// pair with x-faces and y-faces with y-faces (the same index pattern and
-// component order in both lanes), and the face fluxes are stored and read
-// back as pairs.  The halo box, the tile walk, the step control and the
-// per-cell update are those of stage32c_kernel above; the rows the two
-// halves share (box rows HT .. 2G + HT - 1) are converted once per half.
+// as float2 pairs (box row r, box row r + HT) for r in [0, HT + 2G), so
+// x-faces pair with x-faces and y-faces with y-faces (one index pattern and
+// component order in both lanes).  On that tile of TX x HT pairs a thread
+// takes, as in the FP64 kernel (fvb_stage64.cuh), two neighbouring x-faces and
+// two neighbouring y-faces, four faces of each direction: the nine stencil
+// points of a variable are five 16-byte loads along x and nine 8-byte ones
+// along y for four faces, against sixteen 4-byte ones for two, and the y-fluxes
+// stay with the thread that updates their cells.  HT = 2 NK - 1 rows, TX NK
+// threads, each updating up to four cells as two packed pairs.  The halo box, the tile walk, the
+// step control and the per-cell update are those of stage32c_kernel above; the
+// rows the two halves share are converted once per half.
+//
+// Measured, KH 2048^2, stage 1 / 2 / 3: 109 / 118 / 145 us (430, 480, 570
+// instructions a cell) against 119 / 130 / 157 (616 in stage 2) for
+// stage32c_kernel; a step 0.347 against 0.376 ms.  In stage 3 the operands of
+// two cells are loaded before the barrier and those of the other two after
+// the first update (all four before it spill: 181 us), and the lo words,
+// which nothing has read yet, are prefetched into L2 at the tile's start
+// (145 against 152 us).
 // ---------------------------------------------------------------------------
 template <int TX, int TY>
 struct RowPair {
-    static constexpr int G = 4, HT = TY / 2;
+    static constexpr int G = 4, HT = TY / 2, NK = (HT + 1) / 2, NT = TX * NK;
     static constexpr int SW = TX + 2 * G, SH = TY + 2 * G, PL = SW * SH;
     static constexpr int PR = HT + 2 * G;             // pair rows of the working tile
     static constexpr int P2 = PR * SW;                // pairs per working plane
-    static constexpr int C2 = (HT + 2) * SW;          // pairs of the c / E planes: rows G-1 .. G+HT
-    static constexpr int NXP = HT * (TX + 1);         // x-face pairs
-    static constexpr int NYP = (HT + 1) * TX;         // y-face pairs (row HT is evaluated in both halves)
-    static constexpr int NC2 = HT * TX;               // cell pairs
-    static constexpr size_t smem = sizeof(float) * 8 * PL +
-                                   sizeof(float2) * (4 * P2 + 2 * C2 + 4 * HT * (TX + 1) + 4 * (HT + 1) * TX);
+    static constexpr int CW = TX + 2, C2 = (HT + 2) * CW;  // pairs of the c / E planes: cells -1 .. HT, -1 .. TX
+    static constexpr int XP = TX / 2 + 1, FW = 2 * XP;     // x-face pairs of a row, row of FX2
+    static constexpr int r16(int v) { return (v + 15) / 16 * 16; }  // in pairs: 128 bytes
+    static constexpr int oW = r16(8 * PL / 2), oCE = oW + r16(4 * P2), oFX = oCE + r16(2 * C2),
+                         oFY = oFX + r16(4 * HT * FW);
+    static constexpr size_t smem = sizeof(float2) * (size_t)(oFY + 4 * NK * TX);
+    static constexpr int fit = (int)(227 * 1024 / (smem + 2048)), regs = 512 / NT;
+    static constexpr int MINB = fit < regs ? fit : regs;  // resident CTAs an SM, at 128 registers a thread
 };
 
-template <int TX, int TY, int NT, bool BATCHED>
-__global__ void __launch_bounds__(NT, MinBlocks32c<NT>::v) stage32p_kernel(const __grid_constant__ StageArgs a)
+template <int TX, int TY, bool BATCHED>
+__global__ void __launch_bounds__((RowPair<TX, TY>::NT), (RowPair<TX, TY>::MINB))
+    stage32p_kernel(const __grid_constant__ StageArgs a)
 {
     using RP = RowPair<TX, TY>;
-    static_assert(TY % 2 == 0, "two halves of equal height");
-    constexpr int G = RP::G, HT = RP::HT, SW = RP::SW, SH = RP::SH, PL = RP::PL;
-    constexpr int P2 = RP::P2, C2 = RP::C2, NXP = RP::NXP, NYP = RP::NYP, NC2 = RP::NC2;
+    static_assert(TY % 2 == 0 && RP::HT % 2 == 1, "two halves of an odd height");
+    constexpr int G = RP::G, HT = RP::HT, NK = RP::NK, NT = RP::NT, SW = RP::SW, SH = RP::SH, PL = RP::PL;
+    constexpr int P2 = RP::P2, CW = RP::CW, C2 = RP::C2, XP = RP::XP, FW = RP::FW;
     constexpr int NC = TX * TY;
     constexpr int NW = NT / 32;
     constexpr int HS = HT * SW;  // box offset of the upper half's rows
 
     // IN: the halo box as loaded (hi + increment planes); W2: rho, u, v, p
-    // as row pairs; CE2: sound speed and energy as row pairs (pair rows G-1
-    // .. G+HT); FX2 / FY2: face fluxes as row pairs
+    // as row pairs; CE2: sound speed and energy as row pairs; FX2 / FY2: face
+    // fluxes as row pairs (FY2: the lower face of each thread's two)
     extern __shared__ __align__(128) unsigned char smem_raw[];
     float *IN = reinterpret_cast<float *>(smem_raw);
-    float2 *W2 = reinterpret_cast<float2 *>(IN + 8 * PL);
-    float2 *CE2 = W2 + 4 * P2;
-    float2 *FX2 = CE2 + 2 * C2;              // [4][HT][TX+1]
-    float2 *FY2 = FX2 + 4 * HT * (TX + 1);   // [4][HT+1][TX]
+    float2 *sm2 = reinterpret_cast<float2 *>(smem_raw);
+    float2 *W2 = sm2 + RP::oW, *CE2 = sm2 + RP::oCE;
+    float2 *FX2 = sm2 + RP::oFX;             // [4][HT][FW]
+    float2 *FY2 = sm2 + RP::oFY;             // [4][NK][TX]
     __shared__ double s_red[NW];
     __shared__ __align__(8) uint64_t s_bar;
     __shared__ int s_err;
@@ -471,17 +590,6 @@ __global__ void __launch_bounds__(NT, MinBlocks32c<NT>::v) stage32p_kernel(const
         wait_box(t < ntiles ? start_single(t) : false);
     }
     double lacc = 0.0;
-    // which of this thread's conversion pairs (k = tid + it NT) the HLLE reads
-    // the sound speed and energy of: pair rows G-1 .. G+HT, columns G-1 .. G+TX
-    constexpr int NCV = (P2 + NT - 1) / NT;
-    static_assert(NCV <= 32, "one mask bit per conversion pair");
-    unsigned cemask = 0;
-#pragma unroll
-    for (int it = 0; it < NCV; ++it) {
-        const int k = tid + it * NT, r = k / SW, c = k - r * SW;
-        const bool ce = (unsigned)(r - (G - 1)) < (unsigned)(HT + 2) && (unsigned)(c - (G - 1)) < (unsigned)(TX + 2);
-        cemask |= (ce && k < P2 ? 1u : 0u) << it;
-    }
     TileCtl ctl1{};
     if (!batched && t < ntiles) ctl1 = tile_control<P32C>(a.grid.ctrl, a.stage, tid == 0 && t == 0);
     for (; t < ntiles; t += stride, slot ^= 1) {
@@ -501,14 +609,15 @@ __global__ void __launch_bounds__(NT, MinBlocks32c<NT>::v) stage32p_kernel(const
         const int n = gd.n;
         const int tx0 = (tile % gd.tiles_x) * TX, ty0 = (tile / gd.tiles_x) * TY;
         const float gam = (float)gd.gam, gm1 = (float)gd.gam - 1.0f, igm1 = (float)gd.igm1;
+        // rows of the tile inside the grid: pair rows beyond them are skipped
+        const int rows = n - ty0 < HT ? n - ty0 : HT;
         // ---- 1. stage input U0 + d into W2 as primitive row pairs (+ c, E
         //         where the HLLE reads them) -----------------------------------
         if (ctl.run) {
             const f2::V nhalf = f2::splat(-0.5f), G1 = f2::splat(gm1), GA = f2::splat(gam);
-#pragma unroll
-            for (int it = 0; it < NCV; ++it) {
-                const int k = tid + it * NT;
-                if (k >= P2) break;
+            const int np2 = (rows + 2 * G) * SW;
+#pragma unroll 2
+            for (int k = tid; k < np2; k += NT) {
                 f2::V w0 = make_float2(IN[k], IN[k + HS]), w1 = make_float2(IN[PL + k], IN[PL + k + HS]);
                 f2::V w2 = make_float2(IN[2 * PL + k], IN[2 * PL + k + HS]);
                 f2::V w3 = make_float2(IN[3 * PL + k], IN[3 * PL + k + HS]);
@@ -524,9 +633,10 @@ __global__ void __launch_bounds__(NT, MinBlocks32c<NT>::v) stage32p_kernel(const
                 w2 = f2::mul(w2, ir);
                 // p = (gamma - 1)(E - rho (u^2 + v^2) / 2)
                 w3 = f2::mul(G1, f2::fma(f2::mul(nhalf, w0), f2::fma(w1, w1, f2::mul(w2, w2)), E));
-                if ((cemask >> it) & 1u) {
+                const int r = k / SW, c = k - r * SW;
+                if ((unsigned)(r - (G - 1)) < (unsigned)(HT + 2) && (unsigned)(c - (G - 1)) < (unsigned)CW) {
                     const f2::V cs2 = f2::mul(f2::mul(GA, w3), ir);
-                    const int kc = k - (G - 1) * SW;
+                    const int kc = (r - (G - 1)) * CW + (c - (G - 1));
                     CE2[kc] = f2::vsqrt(f2::vmax(cs2, f2::splat(1e-14f)));
                     CE2[C2 + kc] = E;
                 }
@@ -576,85 +686,111 @@ __global__ void __launch_bounds__(NT, MinBlocks32c<NT>::v) stage32p_kernel(const
         const float dt = (float)ctl.dt;
         const float dt_h = dt * (float)gd.inv_h;
 
-        // ---- 3. face fluxes as row pairs: x-faces, then y-faces -------------
-        const f2::V tiny = f2::splat(1e-14f);
-        for (int p = tid; p < NXP; p += NT) {
-            // x-faces of rows r and r + HT at column c (the face left of cell c)
-            const int r = p / (TX + 1), c = p - r * (TX + 1);
-            const int base = (r + G) * SW + (c + G);
-            f2::V L[4], Rv[4], WL[4], WR[4];
+        if (ctl.run && a.stage == 3) {
+            // the lo words come from DRAM: into L2 while the faces are computed
+            for (int m = tid; m < 4 * TY; m += NT) {
+                const int q = m / TY, j = ty0 + (m - q * TY);
+                if (j < n) {
+                    const float *pl = (const float *)gd.lo[cur] + gidx(gd, q, j, tx0);
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(pl));
+                }
+            }
+        }
+        // ---- 3. x-faces 2j, 2j + 1 of pair row r -------------------------------
+        for (int p = tid; p < XP * rows; p += NT) {
+            const int r = p / XP, j = p - r * XP;
+            f2::V LA[4], RA[4], LB[4], RB[4], V0[4], V1[4], V2[4];
 #pragma unroll
             for (int m = 0; m < 4; ++m) {
-                const f2::V *v = W2 + m * P2 + base;
-                f2::V s[8];
+                const float4 *v = reinterpret_cast<const float4 *>(W2 + m * P2 + (r + G) * SW + 2 * j);
+                f2::V s[2 * G + 2];
 #pragma unroll
-                for (int d = 0; d < 8; ++d) s[d] = v[d - G];
-                f2::upface7(s, L[m], Rv[m]);
-                WL[m] = s[G - 1];
-                WR[m] = s[G];
+                for (int d = 0; d <= G; ++d) {
+                    const float4 x = v[d];
+                    s[2 * d] = make_float2(x.x, x.y);
+                    s[2 * d + 1] = make_float2(x.z, x.w);
+                }
+                f2::upface7(s, LA[m], RA[m]);
+                f2::upface7(s + 1, LB[m], RB[m]);
+                V0[m] = s[G - 1];
+                V1[m] = s[G];
+                V2[m] = s[G + 1];
             }
-            L[0] = f2::vmax(L[0], tiny); Rv[0] = f2::vmax(Rv[0], tiny);
-            L[3] = f2::vmax(L[3], tiny); Rv[3] = f2::vmax(Rv[3], tiny);
-            const f2::V *ce = CE2 + (r + 1) * SW + (c + G - 1);
-            f2::V F[4];
-            f2::face_flux(L, Rv, WL, WR, ce[0], ce[1], ce[C2], ce[C2 + 1], gam, igm1, F);
-            f2::V *o = FX2 + p;
-            constexpr int os = HT * (TX + 1);
-            o[0] = F[0]; o[os] = F[1]; o[2 * os] = F[2]; o[3 * os] = F[3];
+            const f2::V *ce = CE2 + (r + 1) * CW + 2 * j;
+            f2::V FA[4], FB[4];
+            f2::floors(LA, RA);
+            f2::floors(LB, RB);
+            f2::face_flux(LA, RA, V0, V1, ce[0], ce[1], ce[C2], ce[C2 + 1], gam, igm1, FA);
+            f2::face_flux(LB, RB, V1, V2, ce[1], ce[2], ce[C2 + 1], ce[C2 + 2], gam, igm1, FB);
+            float4 *o = reinterpret_cast<float4 *>(FX2 + r * FW + 2 * j);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) o[q * (HT * FW / 2)] = make_float4(FA[q].x, FA[q].y, FB[q].x, FB[q].y);
         }
-        for (int p = tid; p < NYP; p += NT) {
-            // y-faces of rows r and r + HT (below cell rows r, r + HT) at column c
-            const int r = p / TX, c = p - r * TX;
-            const int base = (r + G) * SW + (c + G);
-            f2::V L[4], Rv[4], WL[4], WR[4];
+        // ---- 4. y-faces 2k, 2k + 1 of column c (normal velocity v) ------------
+        const int k = tid / TX, c = tid - k * TX, i = tx0 + c;
+        f2::V F0[4], F1[4];
+        if (2 * k <= rows) {
+            f2::V LA[4], RA[4], LB[4], RB[4], V0[4], V1[4], V2[4];
 #pragma unroll
             for (int m = 0; m < 4; ++m) {
-                // (rho, v, u, p): normal velocity v, tangential u
-                const f2::V *v = W2 + (m == 1 ? 2 : m == 2 ? 1 : m) * P2 + base;
-                f2::V s[8];
+                const f2::V *v = W2 + (m == 1 ? 2 : m == 2 ? 1 : m) * P2 + 2 * k * SW + (c + G);
+                f2::V s[2 * G + 1];
 #pragma unroll
-                for (int d = 0; d < 8; ++d) s[d] = v[(d - G) * SW];
-                f2::upface7(s, L[m], Rv[m]);
-                WL[m] = s[G - 1];
-                WR[m] = s[G];
+                for (int d = 0; d <= 2 * G; ++d) s[d] = v[d * SW];
+                f2::upface7(s, LA[m], RA[m]);
+                f2::upface7(s + 1, LB[m], RB[m]);
+                V0[m] = s[G - 1];
+                V1[m] = s[G];
+                V2[m] = s[G + 1];
             }
-            L[0] = f2::vmax(L[0], tiny); Rv[0] = f2::vmax(Rv[0], tiny);
-            L[3] = f2::vmax(L[3], tiny); Rv[3] = f2::vmax(Rv[3], tiny);
-            const f2::V *ce = CE2 + r * SW + (c + G);
-            f2::V F[4];
-            f2::face_flux(L, Rv, WL, WR, ce[0], ce[SW], ce[C2], ce[C2 + SW], gam, igm1, F);
-            f2::V *o = FY2 + p;
-            constexpr int os = (HT + 1) * TX;
-            // normal momentum is v, tangential u
-            o[0] = F[0]; o[os] = F[2]; o[2 * os] = F[1]; o[3 * os] = F[3];
+            const f2::V *ce = CE2 + 2 * k * CW + c + 1;
+            f2::V FA[4], FB[4];
+            f2::floors(LA, RA);
+            f2::floors(LB, RB);
+            f2::face_flux(LA, RA, V0, V1, ce[0], ce[CW], ce[C2], ce[C2 + CW], gam, igm1, FA);
+            f2::face_flux(LB, RB, V1, V2, ce[CW], ce[2 * CW], ce[C2 + CW], ce[C2 + 2 * CW], gam, igm1, FB);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int s = q == 1 ? 2 : q == 2 ? 1 : q;  // Cartesian components
+                F0[q] = FA[s];
+                F1[q] = FB[s];
+                FY2[(q * NK + k) * TX + c] = F0[q];
+            }
         }
+        // the operands of this thread's cells: pair rows 2k, 2k + 1, both halves
+        Operands32c ops[2];
+        auto load_ops = [&](int h) {
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+                const int r = 2 * k + h, j = ty0 + r + b * HT;
+                if (r < HT && i < n && j < n) load_operands32c(gd, a.stage, cur, j, i, ops[b]);
+            }
+        };
+        load_ops(0);
         __syncthreads();
 
         if (!has_next) grid_release();
-        // ---- 4. divergence as pairs, then each cell's RK update -------------
+        // ---- 5. divergence as pairs, then each cell's RK update ---------------
         float lmax = 0.0f;
         const f2::V ndt = f2::splat(-dt_h);
-        for (int cp = tid; cp < NC2; cp += NT) {
-            const int r = cp / TX, c = cp - r * TX, i = tx0 + c;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int r = 2 * k + h;
+            if (r >= rows) continue;
             f2::V dr[4];  // dt L of cells (r, c) and (r + HT, c)
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                const f2::V *fx = FX2 + q * HT * (TX + 1) + r * (TX + 1) + c;
-                const f2::V *fy = FY2 + q * (HT + 1) * TX + r * TX + c;
-                dr[q] = f2::mul(f2::add(f2::sub(fx[1], fx[0]), f2::sub(fy[TX], fy[0])), ndt);
+                const f2::V *fx = FX2 + (q * HT + r) * FW + c;
+                const f2::V dy = h == 0 ? f2::sub(F1[q], F0[q]) : f2::sub(FY2[(q * NK + k + 1) * TX + c], F1[q]);
+                dr[q] = f2::mul(f2::add(f2::sub(fx[1], fx[0]), dy), ndt);
             }
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int j = ty0 + r + h * HT;
-                if (i >= n || j >= n) continue;
-                float dres[4];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) dres[q] = h ? dr[q].y : dr[q].x;
-                update_cell32c(gd, a.stage, cur, nxt, j, i, dres, gam, gm1, lmax);
-            }
+            const int j = ty0 + r;
+            update_pair32c(gd, a.stage, nxt, j, j + HT, i, i < n, i < n && j + HT < n, dr, ops[0], ops[1], gam, gm1,
+                           lmax);
+            if (h == 0) load_ops(1);
         }
 
-        // ---- 5. max wave speed of the new state (stage 3) ------------------
+        // ---- 6. max wave speed of the new state (stage 3) ------------------
         if (a.stage == 3) {
             if (!batched && tid == 0 && tile == 0) leader_finish<P32C>(gd.ctrl);
             if (batched) {
@@ -666,7 +802,7 @@ __global__ void __launch_bounds__(NT, MinBlocks32c<NT>::v) stage32p_kernel(const
                 lacc = fmax(lacc, (double)lmax);
             }
         }
-        // ---- 6. next tile's halo box -----------------------------------------
+        // ---- 7. next tile's halo box -----------------------------------------
         wait_box_own(next_tma);
     }
     if (!batched && a.stage == 3) {
@@ -684,39 +820,34 @@ __global__ void __launch_bounds__(NT, MinBlocks32c<NT>::v) stage32p_kernel(const
 }
 
 template <int SHAPE>
-static void *fn32c(bool batched)
+static StageKernel entry32c()
 {
-    constexpr TileShape ts = kTileShapes[SHAPE];
-    if constexpr (SHAPE == kRowPairShape)
-        return batched ? (void *)stage32p_kernel<ts.tx, ts.ty, ts.nt, true>
-                       : (void *)stage32p_kernel<ts.tx, ts.ty, ts.nt, false>;
-    else
-        return batched ? (void *)stage32c_kernel<ts.tx, ts.ty, ts.nt, true>
-                       : (void *)stage32c_kernel<ts.tx, ts.ty, ts.nt, false>;
-}
-
-void *stage32c_fn(int shape, bool batched)
-{
-    switch (shape) {
-    case 0: return fn32c<0>(batched);
-    case 1: return fn32c<1>(batched);
-    case 2: return fn32c<2>(batched);
-    case 3: return fn32c<3>(batched);
-    case 4: return fn32c<4>(batched);
-    case 5: return fn32c<5>(batched);
-    case 6: return fn32c<6>(batched);
-    default: return nullptr;
+    constexpr TileShape ts = kTileShapes32c[SHAPE];
+    if constexpr (row_pairs(ts)) {
+        static_assert(ts.nt == RowPair<ts.tx, ts.ty>::NT, "one y-face pair a thread");
+        return StageKernel{(void *)stage32p_kernel<ts.tx, ts.ty, false>, (void *)stage32p_kernel<ts.tx, ts.ty, true>,
+                           RowPair<ts.tx, ts.ty>::smem, ts.nt};
+    } else {
+        constexpr int sw = ts.tx + 8, sh = ts.ty + 8;
+        constexpr size_t smem = sizeof(float) * ((size_t)14 * sw * sh + 4 * ts.ty * (ts.tx + 1) + 4 * (ts.ty + 1) * ts.tx);
+        return StageKernel{(void *)stage32c_kernel<ts.tx, ts.ty, ts.nt, false>,
+                           (void *)stage32c_kernel<ts.tx, ts.ty, ts.nt, true>, smem, ts.nt};
     }
 }
 
-size_t stage32c_smem(int shape)
+StageKernel stage32c_kernel_of(int shape)
 {
-    if (shape < 0 || shape >= kNumTileShapes) return 0;
-    if (shape == kRowPairShape)
-        return RowPair<kTileShapes[kRowPairShape].tx, kTileShapes[kRowPairShape].ty>::smem;
-    const TileShape &ts = kTileShapes[shape];
-    const int sw = ts.tx + 8, sh = ts.ty + 8;
-    return sizeof(float) * ((size_t)14 * sw * sh + 4 * ts.ty * (ts.tx + 1) + 4 * (ts.ty + 1) * ts.tx);
+    static_assert(kNumTileShapes == 7, "one entry a shape");
+    switch (shape) {
+    case 0: return entry32c<0>();
+    case 1: return entry32c<1>();
+    case 2: return entry32c<2>();
+    case 3: return entry32c<3>();
+    case 4: return entry32c<4>();
+    case 5: return entry32c<5>();
+    case 6: return entry32c<6>();
+    default: return StageKernel{};
+    }
 }
 
 }  // namespace fvb

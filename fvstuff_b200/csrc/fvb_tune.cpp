@@ -5,8 +5,7 @@
 // builds a scratch grid of a representative size (the grid's own size, at
 // most 2048^2), fills it with a smooth state, and times a few SSP-RK3 steps
 // of every tile variant that can be resident on the device with CUDA
-// events; the fastest wins and is cached for the process (the row-pair
-// variant 6 is not among the candidates).  FVB_TILE=<k>
+// events; the fastest wins and is cached for the process.  FVB_TILE=<k>
 // forces variant k; FVB_AUTOTUNE=0 selects variant 0 without measuring;
 // FVB_AUTOTUNE_LOG=1 prints each variant's time and the choice to stderr.
 #include <cstdio>
@@ -123,12 +122,32 @@ float time_shape(int prec, int order, int n, int shape, cudaStream_t s)
 
 }  // namespace
 
-int autotune_shape(int prec, int order, int n)
+// FVB_TILE's variant, or -1
+static int forced_shape()
 {
     if (const char *f = std::getenv("FVB_TILE")) {
-        int k = std::atoi(f);
+        const int k = std::atoi(f);
         if (k >= 0 && k < kNumTileShapes) return k;
     }
+    return -1;
+}
+
+// Tile variant of a batch, fixed before its grids are known.  FP32c: 32 x 16
+// (three CTAs an SM): grids of 64 ... 512 cells a side fill its 16 rows better
+// than the 30 of the row-pair tile that wins on one large grid.  us a stage on
+// B200, 32 x 16 against 32 x 30: 24 grids of 64-128 15 / 17, 32 of 100-200
+// 35 / 38, 64 of 64-256 74 / 82, 32 of 64-512 111 / 110, 128 of 64-512
+// 415 / 409.  FP64: as one large grid (32 x 15 was best on all of these).
+int batch_shape(int prec)
+{
+    const int f = forced_shape();
+    return f >= 0 ? f : prec == P32C ? 5 : autotune_shape(prec, 7, 4096);
+}
+
+int autotune_shape(int prec, int order, int n)
+{
+    const int forced = forced_shape();
+    if (forced >= 0) return forced;
     if (const char *a = std::getenv("FVB_AUTOTUNE"))
         if (a[0] == '0') return 0;
     int dev = 0;
@@ -144,10 +163,6 @@ int autotune_shape(int prec, int order, int n)
     float best_ms = -1.f;
     const bool log = std::getenv("FVB_AUTOTUNE_LOG") != nullptr;
     for (int shape = 0; shape < kNumTileShapes; ++shape) {
-        // FP32c's row-pair variant is used only when asked for: it matches
-        // variant 5 on large grids within the timing spread, and its 14-row
-        // tiles leave more of small grids' last tile row empty
-        if (prec == P32C && shape == kRowPairShape) continue;
         float ms = time_shape(prec, order, nt, shape, s);
         if (log)
             std::fprintf(stderr, "fvb autotune: precision %d order %d n %d: tile %d (%dx%d, %d threads) %.4f ms\n",
