@@ -401,10 +401,19 @@ fvb_status fvb_create(const fvb_config *cfg, fvb_solver **out)
     if (e != cudaSuccess) { fvb_destroy(s); return cuda_fail(e, "cudaMallocHost"); }
 
     if (keep || rec3 || d2av) {
-        // KEEP / rec3 / D2 viscosity: plain loads into their own tile kernels
+        // KEEP / rec3 / D2 viscosity: their own tile kernels
         if (keep) keep_tiles(s->n, s->gd.tiles_x, s->tiles);
         else if (rec3) rec3_tiles(s->n, s->gd.tiles_x, s->tiles);
         else d2av_tiles(s->n, s->gd.tiles_x, s->tiles);
+        int tx = 0, ty = 0;
+        if (rec3) rec3_tile(tx, ty);
+        CUtensorMap maps[TM_COUNT];
+        if (tx && encode_family_maps(s->gd, tx, ty, maps)) {
+            CUtensorMap *dmaps = (CUtensorMap *)((char *)s->block + tmap_off);
+            e = put_tile_maps(maps, dmaps, s->stream);
+            if (e != cudaSuccess) { fvb_destroy(s); return cuda_fail(e, "tensor maps"); }
+            s->gd.tmap = dmaps;
+        }
         s->graph_steps = 1;
         s->use_graph = cfg->n <= 512;
         e = ctrl_set(s->ctrl, 0.0, 1, 0.0, cfg->cfl, s->gd.h, s->stream);

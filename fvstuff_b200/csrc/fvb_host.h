@@ -51,6 +51,7 @@ cudaError_t keep_lam_into(const GridDev &gd, cudaStream_t s);
 // the limiter pass over a whole state, max wave speed, fv_rec3's initial
 // states (0 Sod, 1 paper vortex, 2 Gresho with background pressure p0)
 void rec3_tiles(int n, int &tiles_x, int &tiles);
+void rec3_tile(int &tx, int &ty);
 cudaError_t rec3_launch_stage(const GridDev &gd, int stage, int tiles, cudaStream_t s);
 cudaError_t rec3_limit_into(const GridDev &gd, void *buf, cudaStream_t s);
 cudaError_t rec3_lam_into(const GridDev &gd, cudaStream_t s);

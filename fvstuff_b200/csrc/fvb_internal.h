@@ -123,6 +123,8 @@ constexpr const TileShape &tile_shape(int prec, int shape)
 // TMA descriptors (fvb_stage.cu): encode the four maps of a grid for a
 // tile shape into host memory; false if this grid cannot use TMA
 bool encode_tile_maps(const GridDev &gd, int prec, int order, int shape, CUtensorMap out[TM_COUNT]);
+// the same for the kernels of BoxPipe (fvb_tma.cuh) with tx x ty tiles
+bool encode_family_maps(const GridDev &gd, int tx, int ty, CUtensorMap out[TM_COUNT]);
 // stream-ordered copy of encoded maps into device memory (dst 64-byte aligned)
 cudaError_t put_tile_maps(const CUtensorMap maps[TM_COUNT], CUtensorMap *dst, cudaStream_t s);
 

@@ -10,12 +10,13 @@
 // non-overlapping 2x2 blocks of the new state (block corners by bilinear
 // extrapolation, one common theta per block, block total conserved).
 //
-// One launch per stage does all of it for a tile of 32 x 32 cells: tiles
-// start on even cells, so every 2x2 block lies in one tile, and after the
-// face fluxes one thread takes one block -- the residuals and RK values of
-// its four cells, the limiter, the stores (interior + periodic ghost
-// images) -- with no barrier between; stage 3 max-reduces the wave speed of
-// the limited state.
+// One launch per stage does all of it for a tile of 32 x 14 cells: tiles
+// start on even cells, so every 2x2 block lies in one tile.  Two halo boxes
+// alternate (TMA, the next one in flight for a whole tile) and U0 arrives
+// during the faces; after the face fluxes a warp takes 2 rows of 16 cells, a
+// block being four of its lanes, so that residual, RK combination, limiter and
+// stores (interior + periodic ghost images) need no barrier between; stage 3
+// max-reduces the wave speed of the limited state.
 //
 // The reference scatters each face flux into its two cells with atomicAdd;
 // here every cell gathers its four face terms in the order a serial run of
@@ -30,21 +31,28 @@
 // needs no scaling and takes none of its code; the faces that do not are
 // listed and then handled one a thread: in place, each warp along the shock
 // went through 25 dependent steps for one or two of its lanes, face after
-// face, and the tiles of the ring held the launch up (84 us of it).  Sod
-// 1024^2: 225 -> 116 us a stage, bit-identical.
+// face, and the tiles of the ring held the launch up (84 us of it).  The
+// limiter's bisection likewise takes a block's four corners side by side.
+// us a stage at 1024^2, mean over ten steps of the Sod (a smooth state): 225
+// (242) as it was, 116 (97) with shared reciprocals, the list and plain loads
+// into 32 x 32 tiles, 105 (77) with the pipeline above.
 #include <algorithm>
 
 #include "fvb_aux.h"
 #include "fvb_device.cuh"
 #include "fvb_ieee.cuh"
+#include "fvb_tma.cuh"
 
 namespace fvb {
 namespace {
 
 constexpr double R3_GAM = 1.4, R3_PFLOOR = 1e-9, R3_RHOFLOOR = 1e-12;
-constexpr int RTX = 32, RTY = 32, RNT = 256, RG = 2;
-constexpr int RSW = RTX + 2 * RG, RSH = RTY + 2 * RG, RPL = RSW * RSH;
-constexpr int RNC = RTX * RTY;
+constexpr int RTX = 32, RTY = 14, RNT = 256, RG = 2;
+using RPipe = BoxPipe<RG, RTX, RTY, RNT>;
+constexpr int RSW = RPipe::SW, RPL = RPipe::PL;
+static_assert(RPipe::XO == 0, "the box starts at the tile's first padded column");
+// shared memory, in doubles: two boxes, U0, x-fluxes, y-fluxes
+constexpr int ROU0 = 2 * RPipe::BOX, ROFX = ROU0 + RPipe::U0, ROFY = ROFX + 4 * RTY * (RTX + 1);
 constexpr int RNF = RTY * (RTX + 1) + (RTY + 1) * RTX;  // faces of a tile
 
 // c = sqrt(gamma p / rho)                       fv_rec3_2d.cu:68-69
@@ -302,98 +310,106 @@ __device__ __noinline__ double r3_lam_any(double U0, double U1, double U2, doubl
     return fabs(W[1]) + fabs(W[2]) + r3_snd(W[0], W[3]);
 }
 
-__device__ __noinline__ bool r3_limit_any(double U[4][4], int *brutal) { return r3_limit_block(U, brutal); }
-
-// corner c of a 2x2 block by bilinear extrapolation: opposite cell 3 - c,
-// neighbours in the reference's order
-__device__ __forceinline__ void r3_corner(const double U[4][4], int c, double C[4])
+// Is this lane's corner of its 2x2 block (lanes l, l ^ 1, l ^ 16, l ^ 17) well
+// clear of the floors?  If all four are, the block needs no limiter: its mean,
+// the corners' average, then clears them too (the pressure is concave; with
+// rho, p >= 1e-6 and E <= 1e6 the rounding of any of these is below 1e-7).
+__device__ __forceinline__ bool r3_clear_corner(const double U[4])
 {
-    const int a = c ^ 1, b = c ^ 2;  // (1, 2), (0, 3), (3, 0), (2, 1)
+    double C[4], r, u, v;
 #pragma unroll
-    for (int q = 0; q < 4; q++) C[q] = (9. * U[c][q] - 3. * U[a][q] - 3. * U[b][q] + U[3 - c][q]) * 0.25;
-}
-
-// r3_limit_block of a block whose mean and corners clear the floors (nearly
-// all): left as it is; false: it needs the limiter
-__device__ __forceinline__ bool r3_clear_block(const double U[4][4])
-{
-    double Ub[4] = {0., 0., 0., 0.};
-#pragma unroll
-    for (int c = 0; c < 4; c++)
-#pragma unroll
-        for (int q = 0; q < 4; q++) Ub[q] += 0.25 * U[c][q];
-    bool ok = true;
-    double r, u, v;
-    double rmin = Ub[0], pmin = r3_p_near(Ub, r, u, v, ok);
-#pragma unroll
-    for (int c = 0; c < 4; c++) {
-        double C[4];
-        r3_corner(U, c, C);
-        const double p = r3_p_near(C, r, u, v, ok);
-        rmin = smin<double>(C[0], rmin);
-        pmin = smin<double>(p, pmin);
+    for (int q = 0; q < 4; ++q) {
+        const double a = __shfl_xor_sync(0xffffffffu, U[q], 1), b = __shfl_xor_sync(0xffffffffu, U[q], 16);
+        const double o = __shfl_xor_sync(0xffffffffu, U[q], 17);
+        C[q] = (9. * U[q] - 3. * a - 3. * b + o) * 0.25;
     }
-    return ok && rmin >= R3_RHOFLOOR && pmin >= R3_PFLOOR;
+    bool ok = true;
+    const double p = r3_p_near(C, r, u, v, ok);
+    return ok && C[0] >= 1e-6 && p >= 1e-6 && C[3] <= 1e6;
 }
 
-// the limiter of a block with an admissible mean, the four corners' pressures
-// of a bisection step side by side in the shared-reciprocal form; false (U
-// untouched): take r3_limit_any
-__device__ __forceinline__ bool r3_limit_near(double U[4][4])
+// The limiter (r3_limit_block) of a warp's eight 2x2 blocks, each lane on its
+// own cell and corner, so that a bisection step is one pressure for all four
+// corners and not four in a row (and in place of one lane a block: 9 us a warp
+// on the shock).  A block that turns out to need none is left as it is; one
+// whose mean is not admissible or whose values leave the quotients' range goes
+// to r3_limit_block, one lane.
+__device__ __noinline__ void r3_limit_warp_any(double U[4], bool take, int lane, int *brutal)
 {
-    double Ub[4] = {0., 0., 0., 0.}, C[4][4];
-#pragma unroll
+    const int base = lane & 14, mine = (lane >> 4) * 2 + (lane & 1);
+    double T[4][4];
     for (int c = 0; c < 4; c++)
-#pragma unroll
-        for (int q = 0; q < 4; q++) Ub[q] += 0.25 * U[c][q];
-    bool ok = true;
-    double r, u, v;
-    const double pb = r3_p_near(Ub, r, u, v, ok);
-    if (!ok || !(Ub[0] >= R3_RHOFLOOR) || !(pb >= R3_PFLOOR)) return false;
-    double th = 1.;
-#pragma unroll
-    for (int c = 0; c < 4; c++) {
-        r3_corner(U, c, C[c]);
-        if (C[c][0] < R3_RHOFLOOR) {
-            const double d = Ub[0] - C[c][0];
-            if (d > 0.) th = smin<double>((Ub[0] - R3_RHOFLOOR) / d, th);
+        for (int q = 0; q < 4; q++) T[c][q] = __shfl_sync(0xffffffffu, U[q], base + (c & 1) + 16 * (c >> 1));
+    if (take && mine == 0) r3_limit_block(T, brutal);
+    for (int c = 0; c < 4; c++)
+        for (int q = 0; q < 4; q++) {
+            const double v = __shfl_sync(0xffffffffu, T[c][q], base);
+            if (take && c == mine) U[q] = v;
         }
-    }
-    if (th < 1.)
+}
+
+__device__ __noinline__ void r3_limit_warp_(double U[4], bool in, int lane, int *brutal)
+{
+    const int base = lane & 14;
+    const unsigned block = 0x30003u << base;
+    double Ub[4], C[4], r, u, v;
+    bool ok = true;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        Ub[q] = 0.;
 #pragma unroll
         for (int c = 0; c < 4; c++)
+            Ub[q] += 0.25 * __shfl_sync(0xffffffffu, U[q], base + (c & 1) + 16 * (c >> 1));
+        const double a = __shfl_xor_sync(0xffffffffu, U[q], 1), b = __shfl_xor_sync(0xffffffffu, U[q], 16);
+        const double o = __shfl_xor_sync(0xffffffffu, U[q], 17);
+        C[q] = (9. * U[q] - 3. * a - 3. * b + o) * 0.25;
+    }
+    const double pb = r3_p_near(Ub, r, u, v, ok);
+    ok = ok && Ub[0] >= R3_RHOFLOOR && pb >= R3_PFLOOR;
+    double th = 1.;
+    if (C[0] < R3_RHOFLOOR) {
+        const double d = Ub[0] - C[0];
+        if (d > 0.) th = smin<double>((Ub[0] - R3_RHOFLOOR) / d, th);
+    }
+    th = smin<double>(__shfl_xor_sync(0xffffffffu, th, 1), th);
+    th = smin<double>(__shfl_xor_sync(0xffffffffu, th, 16), th);
+    if (th < 1.)
 #pragma unroll
-            for (int q = 0; q < 4; q++) C[c][q] = Ub[q] + th * (C[c][q] - Ub[q]);
-    bool bad = false;
-#pragma unroll
-    for (int c = 0; c < 4; c++) bad = bad || C[c][0] < R3_RHOFLOOR || r3_p_near(C[c], r, u, v, ok) < R3_PFLOOR;
+        for (int q = 0; q < 4; q++) C[q] = Ub[q] + th * (C[q] - Ub[q]);
+    const double pc = r3_p_near(C, r, u, v, ok);
+    const bool bad = (__ballot_sync(0xffffffffu, in && (C[0] < R3_RHOFLOOR || pc < R3_PFLOOR)) & block) != 0;
     double lo = 0., hi = 1.;
-    if (bad) {
+    if (__any_sync(0xffffffffu, bad)) {
 #pragma unroll 1
         for (int it = 0; it < 30; it++) {
             const double mid = 0.5 * (lo + hi);
-            bool out = false;
+            double V[4];
 #pragma unroll
-            for (int c = 0; c < 4; c++) {
-                double V[4];
-#pragma unroll
-                for (int q = 0; q < 4; q++) V[q] = Ub[q] + mid * (C[c][q] - Ub[q]);
-                const double p = r3_p_near(V, r, u, v, ok);
-                out = out || V[0] < R3_RHOFLOOR || p < R3_PFLOOR;
-            }
+            for (int q = 0; q < 4; q++) V[q] = Ub[q] + mid * (C[q] - Ub[q]);
+            const double p = r3_p_near(V, r, u, v, ok);
+            const bool out = (__ballot_sync(0xffffffffu, V[0] < R3_RHOFLOOR || p < R3_PFLOOR) & block) != 0;
             hi = out ? mid : hi;
             lo = out ? lo : mid;
         }
     }
-    if (!ok) return false;
-#pragma unroll
-    for (int c = 0; c < 4; c++)
+    const unsigned odd = __ballot_sync(0xffffffffu, in && !ok);
+    if (odd) r3_limit_warp_any(U, in && (odd & block) != 0, lane, brutal);
+    if ((odd & block) == 0)
 #pragma unroll
         for (int q = 0; q < 4; q++) {
-            if (th < 1.) U[c][q] = Ub[q] + th * (U[c][q] - Ub[q]);
-            if (bad) U[c][q] = Ub[q] + lo * (U[c][q] - Ub[q]);
+            if (th < 1.) U[q] = Ub[q] + th * (U[q] - Ub[q]);
+            if (bad) U[q] = Ub[q] + lo * (U[q] - Ub[q]);
         }
-    return true;
+}
+// (with copies, so that the usual path's state stays in registers)
+__device__ __forceinline__ void r3_limit_warp(double U[4], bool in, int lane, int &brutal)
+{
+    double X[4] = {U[0], U[1], U[2], U[3]};
+    int nb = 0;
+    r3_limit_warp_(X, in, lane, &nb);
+    brutal += nb;
+#pragma unroll
+    for (int q = 0; q < 4; q++) U[q] = X[q];
 }
 
 __device__ __forceinline__ long long r3_at(const GridDev &gd, int j, int i)
@@ -445,18 +461,18 @@ __device__ __forceinline__ bool r3_face(const double *Q, int f, double *FP)
 }
 
 // one SSP-RK3 stage                             fv_rec3_2d.cu:166-353
-__global__ void __launch_bounds__(RNT, 2) rec3_stage_kernel(const GridDev gd, int stage, int ntiles)
+__global__ void __launch_bounds__(RNT, 2) rec3_stage_kernel(const __grid_constant__ GridDev gd, int stage, int ntiles)
 {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    double *Q = reinterpret_cast<double *>(smem_raw);  // [4][RSH][RSW] stage input
-    double *FX = Q + 4 * RPL;                          // [4][RTY][RTX+1]
-    double *FY = FX + 4 * RTY * (RTX + 1);             // [4][RTY+1][RTX]
-    __shared__ TileCtl s_ctl;
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    double *sm = reinterpret_cast<double *>(smem_raw);
+    double *U0 = sm + ROU0;  // [4][RTY][RTX]
+    double *FX = sm + ROFX;  // [4][RTY][RTX+1]
+    double *FY = sm + ROFY;  // [4][RTY+1][RTX]
     __shared__ double s_red[RNT / 32];
-    __shared__ int s_nlist;
+    __shared__ __align__(8) uint64_t s_bar[3];
+    __shared__ int s_err, s_nlist;
     __shared__ unsigned short s_list[RNF];  // faces that need the scaling
-    const int tid = threadIdx.x, n = gd.n, np = n + 2 * RG;
-    const double *in = (const double *)(stage == 2 ? gd.k1 : stage == 3 ? gd.k2 : gd.st[0]);
+    const int tid = threadIdx.x, lane = tid & 31, n = gd.n;
     const double *u0 = (const double *)gd.st[0];
     double *out = (double *)(stage == 1 ? gd.k1 : stage == 2 ? gd.k2 : gd.st[0]);
     const double inv_h = 1. / gd.h;
@@ -465,33 +481,43 @@ __global__ void __launch_bounds__(RNT, 2) rec3_stage_kernel(const GridDev gd, in
     int brutal = 0;
     double lacc = 0.0;
 
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    RPipe pipe(s_bar, &s_err, tid);
+    grid_dependency();
+    int t = blockIdx.x, buf = 0;
+    if (t < ntiles) pipe.start_box(gd, stage, t, sm, 0, tid);
+    const TileCtl ctl = tile_control<P64>(gd.ctrl, stage, tid == 0 && t == 0);
+    pipe.finish_box(gd, 0, t < ntiles);
+    for (; t < ntiles; t += gridDim.x, buf ^= 1) {
         const int tx0 = (t % gd.tiles_x) * RTX, ty0 = (t / gd.tiles_x) * RTY;
-        if (tid == 0) {
-            s_ctl = tile_control<P64>(gd.ctrl, stage, t == 0);
-            s_nlist = 0;
+        const bool has_next = t + (int)gridDim.x < ntiles;
+        if (s_err) {
+            // a box never arrived: record it, stop
+            if (tid == 0) gd.ctrl->status = FVB_ERR_TIMEOUT;
+            break;
         }
-        __syncthreads();
-        const TileCtl ctl = s_ctl;
+        if (has_next) pipe.start_box(gd, stage, t + gridDim.x, sm + (buf ^ 1) * RPipe::BOX, buf ^ 1, tid);
+        const bool u0_tma = ctl.run && stage >= 2 && gd.tmap;
+        if (u0_tma) pipe.start_u0(gd, tx0, ty0, U0, tid);
         if (!ctl.run) {
-            __syncthreads();
+            pipe.finish_box(gd, buf ^ 1, has_next);
             continue;
         }
-        // ---- halo box of the stage input (an admissible dummy outside) ----
-        for (int k = tid; k < RPL; k += RNT) {
-            const int r = k / RSW, c = k - r * RSW, jp = ty0 + r, ip = tx0 + c;
-            const bool inb = jp < np && ip < np;
-            const long long e = (long long)jp * gd.pitch + ip + gd.xoff;
-            for (int q = 0; q < 4; ++q) Q[q * RPL + k] = inb ? in[e + q * gd.plane] : (q == 0 ? 1. : q == 3 ? 2.5 : 0.);
-        }
+        const double *Q = sm + buf * RPipe::BOX;  // [4][RSH][RSW] stage input
+        if (tid == 0) s_nlist = 0;
         __syncthreads();
         // ---- faces: x-face (r, c) lies between cells c-1 and c; a face with
         //      a state below the floors goes on the list ------------------------
-        for (int f = tid; f < RTY * (RTX + 1); f += RNT)
-            if (!r3_face<true, false>(Q, f, FX)) s_list[atomicAdd(&s_nlist, 1)] = (unsigned short)f;
-        for (int f = tid; f < (RTY + 1) * RTX; f += RNT)
-            if (!r3_face<false, false>(Q, f, FY))
+        //      (faces of cells outside the grid are left out)
+        for (int f = tid; f < RTY * (RTX + 1); f += RNT) {
+            const int r = f / (RTX + 1), c = f - r * (RTX + 1);
+            if (ty0 + r < n && tx0 + c <= n && !r3_face<true, false>(Q, f, FX))
+                s_list[atomicAdd(&s_nlist, 1)] = (unsigned short)f;
+        }
+        for (int f = tid; f < (RTY + 1) * RTX; f += RNT) {
+            const int r = f / RTX, c = f - r * RTX;
+            if (ty0 + r <= n && tx0 + c < n && !r3_face<false, false>(Q, f, FY))
                 s_list[atomicAdd(&s_nlist, 1)] = (unsigned short)(f + RTY * (RTX + 1));
+        }
         __syncthreads();
         // ---- the listed faces, one a thread, so that their bisections (25
         //      dependent steps a side) run side by side ---------------------------
@@ -504,18 +530,18 @@ __global__ void __launch_bounds__(RNT, 2) rec3_stage_kernel(const GridDev gd, in
             }
             __syncthreads();
         }
-        // ---- per 2x2 block, one thread: residual of its four cells in the
-        //      serial scatter's order, RK combination, the block limiter,
-        //      stores with the periodic ghost images, stage-3 wave speed -----
-        for (int kb = tid; kb < RNC / 4; kb += RNT) {
-            const int jb = kb / (RTX / 2), ib = kb - jb * (RTX / 2);
-            const int c0 = 2 * ib, r0 = 2 * jb;
-            if (tx0 + c0 >= n || ty0 + r0 >= n) continue;  // n even: the block is whole
-            double U[4][4];
-#pragma unroll
-            for (int cc = 0; cc < 4; cc++) {
-                const int r = r0 + (cc >> 1), c = c0 + (cc & 1), i = tx0 + c, j = ty0 + r;
-                const long long e = r3_at(gd, j, i);
+        // ---- cells, a warp on 2 rows of 16, so that a 2x2 block is four lanes:
+        //      residual in the serial scatter's order, RK combination, the
+        //      block limiter, stores with the periodic ghost images, stage-3
+        //      wave speed ------------------------------------------------------
+        if (!has_next) grid_release();
+        const bool u0_ok = !u0_tma || pipe.wait(2);
+        for (int w = tid >> 5; w < (RTY / 2) * (RTX / 16); w += RNT / 32) {
+            const int r = 2 * (w / (RTX / 16)) + (lane >> 4), c = 16 * (w % (RTX / 16)) + (lane & 15);
+            const int i = tx0 + c, j = ty0 + r;
+            const bool in = i < n && j < n && u0_ok;  // (n even: a block is inside as a whole)
+            double U[4] = {1., 0., 0., 2.5};
+            if (in) {
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {
                     const double *fx = FX + q * RTY * (RTX + 1) + r * (RTX + 1) + c;
@@ -527,42 +553,31 @@ __global__ void __launch_bounds__(RNT, 2) rec3_stage_kernel(const GridDev gd, in
                     else if (i == 0 && j > 0) L = ((tb + tr) + tt) + tl;
                     else if (i > 0) L = ((tl + tr) + tt) + tb;
                     else L = ((tr + tt) + tl) + tb;
-                    const double qa = u0[e + q * gd.plane];
                     const double qb = Q[q * RPL + (r + RG) * RSW + (c + RG)];
-                    U[cc][q] = ca * qa + cb * (qb + ctl.dt * L);
+                    const double qa = stage == 1 ? qb
+                                      : u0_tma   ? U0[(q * RTY + r) * RTX + c]
+                                                 : u0[r3_at(gd, j, i) + q * gd.plane];
+                    U[q] = ca * qa + cb * (qb + ctl.dt * L);
                 }
             }
-            if (!r3_clear_block(U) && !r3_limit_near(U)) {
-                double T[4][4];
-                int nb = 0;
-#pragma unroll
-                for (int c = 0; c < 4; c++)
-#pragma unroll
-                    for (int q = 0; q < 4; q++) T[c][q] = U[c][q];
-                r3_limit_any(T, &nb);
-                brutal += nb;
-#pragma unroll
-                for (int c = 0; c < 4; c++)
-#pragma unroll
-                    for (int q = 0; q < 4; q++) U[c][q] = T[c][q];
-            }
-#pragma unroll
-            for (int cc = 0; cc < 4; cc++) {
-                const int i = tx0 + c0 + (cc & 1), j = ty0 + r0 + (cc >> 1);
-                put_cell<double>(gd, out, j, i, U[cc]);
+            const bool clear = r3_clear_corner(U);  // (every lane: it shuffles)
+            if (__any_sync(0xffffffffu, in && !clear)) r3_limit_warp(U, in, lane, brutal);
+            if (in) {
+                put_cell<double>(gd, out, j, i, U);
                 if (stage == 3) {
-                    double r, u, v;
+                    double rr, u, v;
                     bool ok = true;
-                    const double p = smax<double>(r3_p_near(U[cc], r, u, v, ok), R3_PFLOOR);
-                    const double x = quot(R3_GAM * p, r, recip(r));
+                    const double p = smax<double>(r3_p_near(U, rr, u, v, ok), R3_PFLOOR);
+                    const double x = quot(R3_GAM * p, rr, recip(rr));
                     const double lam = fabs(u) + fabs(v) + root(x);
-                    lacc = smax<double>(ok && den_ok(x) ? lam : r3_lam_any(U[cc][0], U[cc][1], U[cc][2], U[cc][3]), lacc);
+                    lacc = smax<double>(ok && den_ok(x) ? lam : r3_lam_any(U[0], U[1], U[2], U[3]), lacc);
                 }
             }
         }
         if (stage == 3 && tid == 0 && t == 0) leader_finish<P64>(gd.ctrl);
-        __syncthreads();
+        pipe.finish_box(gd, buf ^ 1, has_next);
     }
+    pipe.drain();
     if (brutal) atomicAdd(&gd.ctrl->aux, (unsigned long long)brutal);
     if (stage == 3) {
         for (int o = 16; o > 0; o >>= 1) lacc = fmax(lacc, __shfl_xor_sync(0xffffffffu, lacc, o));
@@ -682,10 +697,7 @@ __global__ void rec3_ic_kernel(const GridDev gd, double *buf, int icase, double 
     }
 }
 
-size_t rec3_smem()
-{
-    return sizeof(double) * (4 * RPL + 4 * RTY * (RTX + 1) + 4 * (RTY + 1) * RTX);
-}
+size_t rec3_smem() { return sizeof(double) * (ROFY + 4 * (RTY + 1) * RTX); }
 
 int sm_count()
 {
@@ -703,14 +715,20 @@ void rec3_tiles(int n, int &tiles_x, int &tiles)
     tiles = tiles_x * ((n + RTY - 1) / RTY);
 }
 
+void rec3_tile(int &tx, int &ty)
+{
+    tx = RTX;
+    ty = RTY;
+}
+
 cudaError_t rec3_launch_stage(const GridDev &gd, int stage, int tiles, cudaStream_t s)
 {
     LaunchFacts f{};
     cudaError_t e = launch_facts((const void *)rec3_stage_kernel, RNT, rec3_smem(), f);
     if (e != cudaSuccess) return e;
     const int cap = f.ctas_per_sm * f.sms;
-    rec3_stage_kernel<<<tiles < cap ? tiles : cap, RNT, rec3_smem(), s>>>(gd, stage, tiles);
-    return cudaGetLastError();
+    void *args[] = {(void *)&gd, (void *)&stage, (void *)&tiles};
+    return launch_chained((const void *)rec3_stage_kernel, tiles < cap ? tiles : cap, RNT, rec3_smem(), s, args);
 }
 
 cudaError_t rec3_limit_into(const GridDev &gd, void *buf, cudaStream_t s)

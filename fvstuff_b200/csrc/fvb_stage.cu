@@ -385,31 +385,26 @@ static EncodeTiledFn encode_fn()
     return fn;
 }
 
-// Descriptors of the (TX+2g) x (TY+2g) x 4 halo box of each padded buffer.
-// The tensor is (x = memory column, y = padded row, z = variable plane);
-// x starts at column 0 of the pitched row, so a tile's box starts at
-// x = xoff + tx0.  Every such x, the pitch and the plane stride must be
-// 16-byte multiples; out-of-range parts of ragged tiles are zero-filled.
-// The FP64 kernel's box starts one column earlier where that x is odd and is
-// two columns wider (fvb_stage64.cuh), and its U0 tile has a map of its own.
-bool encode_tile_maps(const GridDev &gd, int prec, int order, int shape, CUtensorMap out[TM_COUNT])
+// Descriptors of the (tx+2g) x (ty+2g) x 4 halo box of each padded buffer and
+// of the tx x ty tile of U0 (out[TM_U0]).  The tensor is (x = memory column,
+// y = padded row, z = variable plane); x starts at column 0 of the pitched
+// row, so a tile's box starts at x = xoff + tx0, or with xo = 1 (where that x
+// is odd, FP64) one column earlier and is two columns wider.  Every such x,
+// the pitch and the plane stride must be 16-byte multiples; out-of-range
+// parts of ragged tiles are zero-filled.
+static bool encode_maps(const GridDev &gd, size_t es, int g, int tx, int ty, int xo, CUtensorMap out[TM_COUNT])
 {
     EncodeTiledFn enc = encode_fn();
-    if (!enc || shape < 0 || shape >= kNumTileShapes) return false;
-    const TileShape &ts = tile_shape(prec, shape);
-    const int g = (order + 1) / 2, np = gd.n + 2 * g;
-    const size_t es = prec == P64 ? 8 : 4;
-    const int xo = prec == P64 ? (16 - g) & 1 : 0;
-    const int sw = ts.tx + 2 * g + 2 * xo, sh = ts.ty + 2 * g;
+    if (!enc) return false;
+    const int np = gd.n + 2 * g, sw = tx + 2 * g + 2 * xo, sh = ty + 2 * g;
     if (((size_t)gd.pitch * es) % 16 || ((size_t)gd.plane * es) % 16 || gd.xoff < xo ||
-        ((size_t)(gd.xoff - xo) * es) % 16 || ((size_t)ts.tx * es) % 16 || ((size_t)sw * es) % 16 || sw > 256 ||
-        sh > 256)
+        ((size_t)(gd.xoff - xo) * es) % 16 || ((size_t)tx * es) % 16 || ((size_t)sw * es) % 16 || sw > 256 || sh > 256)
         return false;
-    if (prec == P64 && ((size_t)(gd.xoff + g) * es) % 16) return false;
+    if (es == 8 && ((size_t)(gd.xoff + g) * es) % 16) return false;
     cuuint64_t dims[3] = {(cuuint64_t)(gd.xoff + np), (cuuint64_t)np, 4};
     cuuint64_t strides[2] = {(cuuint64_t)gd.pitch * es, (cuuint64_t)gd.plane * es};
     cuuint32_t box[3] = {(cuuint32_t)sw, (cuuint32_t)sh, 4};
-    cuuint32_t tile[3] = {(cuuint32_t)ts.tx, (cuuint32_t)ts.ty, 4};
+    cuuint32_t tile[3] = {(cuuint32_t)tx, (cuuint32_t)ty, 4};
     cuuint32_t estr[3] = {1, 1, 1};
     void *bufs[TM_COUNT] = {gd.st[0], gd.st[1] ? gd.st[1] : gd.st[0], gd.k1, gd.k2, gd.st[0]};
     for (int m = 0; m < TM_COUNT; ++m) {
@@ -421,6 +416,19 @@ bool encode_tile_maps(const GridDev &gd, int prec, int order, int shape, CUtenso
         if (r != CUDA_SUCCESS) return false;
     }
     return true;
+}
+
+bool encode_tile_maps(const GridDev &gd, int prec, int order, int shape, CUtensorMap out[TM_COUNT])
+{
+    if (shape < 0 || shape >= kNumTileShapes) return false;
+    const TileShape &ts = tile_shape(prec, shape);
+    const int g = (order + 1) / 2;
+    return encode_maps(gd, prec == P64 ? 8 : 4, g, ts.tx, ts.ty, prec == P64 ? (16 - g) & 1 : 0, out);
+}
+
+bool encode_family_maps(const GridDev &gd, int tx, int ty, CUtensorMap out[TM_COUNT])
+{
+    return encode_maps(gd, 8, gd.g, tx, ty, (16 - gd.g) & 1, out);
 }
 
 // Copy a grid's tensor maps into device memory from a kernel parameter, so

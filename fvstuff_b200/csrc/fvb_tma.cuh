@@ -139,6 +139,66 @@ __device__ __forceinline__ void issue_tile_load64(const GridDev &gd, int stage, 
     }
 }
 
+// The loads of a single-grid FP64 kernel that walks tiles with two alternating
+// halo boxes (barriers 0, 1) and, in stages 2 and 3, the tile's U0 (barrier
+// 2): the KEEP, rec3 and D2-viscosity kernels.  Without descriptors the boxes
+// are loaded cooperatively and U0 is read where it is used.
+template <int G, int TX, int TY, int NT>
+struct BoxPipe {
+    static constexpr int XO = (16 - G) & 1;  // a box starts on an even column (16 bytes)
+    static constexpr int SW = TX + 2 * G + 2 * XO, SH = TY + 2 * G, PL = SW * SH;
+    static constexpr int BOX = (4 * PL + 15) / 16 * 16, U0 = 4 * TX * TY;  // doubles, 128-byte multiples
+    uint64_t *bar;
+    int *err;
+    uint32_t phase = 0, lost = 0;  // bit m: the phase of bar[m] to wait for; a wait on it gave up
+
+    __device__ BoxPipe(uint64_t *b, int *e, int tid) : bar(b), err(e)
+    {
+        if (tid == 0) {
+            for (int m = 0; m < 3; ++m) mbar_init(bar + m, 1);
+            *err = 0;
+        }
+        __syncthreads();
+    }
+    __device__ __forceinline__ bool wait(int m)
+    {
+        if (!mbar_wait(bar + m, (phase >> m) & 1u)) {
+            *err = 1;
+            lost |= 1u << m;
+            return false;
+        }
+        phase ^= 1u << m;
+        return true;
+    }
+    // box of tile t into dst; its last readers are behind a block barrier
+    __device__ __forceinline__ void start_box(const GridDev &gd, int stage, int t, double *dst, int m, int tid)
+    {
+        if (tid == 0 && gd.tmap) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        issue_tile_load64<G, TX, TY, SW, XO, NT>(gd, stage, t, dst, bar + m, tid);
+    }
+    __device__ __forceinline__ void start_u0(const GridDev &gd, int tx0, int ty0, double *dst, int tid)
+    {
+        if (tid != 0) return;
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        mbar_expect_tx(bar + 2, U0 * sizeof(double));
+        tma_load3(dst, gd.tmap + TM_U0, gd.xoff + G + tx0, G + ty0, 0, bar + 2);
+    }
+    // the box of barrier m: wait for it; the block barrier also makes a
+    // cooperative load visible and agrees on *err
+    __device__ __forceinline__ void finish_box(const GridDev &gd, int m, bool issued)
+    {
+        if (issued && gd.tmap) wait(m);
+        __syncthreads();
+    }
+    // a load whose wait gave up may still be in flight: wait once more, so no
+    // copy into this CTA's shared memory outlives it
+    __device__ __forceinline__ void drain()
+    {
+        for (int m = 0; m < 3; ++m)
+            if ((lost >> m) & 1u) mbar_wait(bar + m, (phase >> m) & 1u);
+    }
+};
+
 // Tile headers of a batched launch.  Warp 0 stages them one tile ahead:
 // the table entry of the CTA's next tile is loaded a tile early, and at the
 // top of each tile each lane of warp 0 loads one 8-byte word of the next
