@@ -338,7 +338,7 @@ __device__ __noinline__ void d2_cell_any(const double *Q, const double *FX, cons
 // one SSP-RK3 stage                        fv_up7_ducros_2d.cu.bak:287-446
 template <int ORDER>
 __global__ void __launch_bounds__(DNT, D2Shape<ORDER>::MINB)
-    d2av_stage_kernel(const GridDev gd, int stage, int ntiles, D2Params av)
+    d2av_stage_kernel(const __grid_constant__ GridDev gd, int stage, int ntiles, D2Params av)
 {
     using S = D2Shape<ORDER>;
     constexpr int HW = S::HW, HB = S::HB, BW = S::BW, PL = S::PL;
@@ -351,7 +351,6 @@ __global__ void __launch_bounds__(DNT, D2Shape<ORDER>::MINB)
     double *CS = LY + PL;                              // c
     double *FX = CS + PL;                              // [4][DTY][DTX+1]
     double *FY = FX + 4 * S::NFX;                      // [4][DTY+1][DTX]
-    __shared__ TileCtl s_ctl;
     __shared__ double s_red[DNT / 32];
     const int tid = threadIdx.x, n = gd.n, np = n + 2 * HB;
     const double gam = gd.gam, h = gd.h;
@@ -361,22 +360,16 @@ __global__ void __launch_bounds__(DNT, D2Shape<ORDER>::MINB)
     double lacc = 0.0;
     // (in shared memory: 18 registers a thread would hold across the faces)
     __shared__ D2Cell ck;
+    grid_dependency();
+    // the step control, the same for every tile
+    const TileCtl ctl = tile_control<P64>(gd.ctrl, stage, tid == 0 && blockIdx.x == 0);
     if (tid == 0)
-        ck = D2Cell{h, recip(h), 60. * h, recip(60. * h), av.c2 / h, av.cg / h, av.sc / (h * h), 0.0, stage,
+        ck = D2Cell{h, recip(h), 60. * h, recip(60. * h), av.c2 / h, av.cg / h, av.sc / (h * h), ctl.dt, stage,
                     av.cg != 0.0};
     const bool hok = den_ok(h) && den_ok(60. * h);
 
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    for (int t = blockIdx.x; t < ntiles && ctl.run; t += gridDim.x) {
         const int tx0 = (t % gd.tiles_x) * DTX, ty0 = (t / gd.tiles_x) * DTY;
-        if (tid == 0) {
-            s_ctl = tile_control<P64>(gd.ctrl, stage, t == 0);
-            ck.dt = s_ctl.dt;
-        }
-        __syncthreads();
-        if (!s_ctl.run) {
-            __syncthreads();
-            continue;
-        }
         // ---- halo box of the stage input and its per-cell quantities: the
         //      sensor's velocities in the rows / columns it reaches, the wave
         //      speeds on the cells and their direct neighbours --------------
@@ -432,6 +425,7 @@ __global__ void __launch_bounds__(DNT, D2Shape<ORDER>::MINB)
             o[3 * os] = Fn[3];
         }
         __syncthreads();
+        if (t + (int)gridDim.x >= ntiles) grid_release();
         // ---- cells: residual, sensor, viscosity, RK combination, stores ---
         for (int k = tid; k < DTX * DTY; k += DNT) {
             const int r = k / DTX, c = k - r * DTX, i = tx0 + c, j = ty0 + r;
@@ -548,8 +542,8 @@ cudaError_t launch_order(const GridDev &gd, int stage, int tiles, const D2Params
     cudaError_t e = launch_facts((const void *)d2av_stage_kernel<ORDER>, DNT, smem, f);
     if (e != cudaSuccess) return e;
     const int cap = f.ctas_per_sm * f.sms;
-    d2av_stage_kernel<ORDER><<<tiles < cap ? tiles : cap, DNT, smem, s>>>(gd, stage, tiles, av);
-    return cudaGetLastError();
+    void *args[] = {(void *)&gd, (void *)&stage, (void *)&tiles, (void *)&av};
+    return launch_chained((const void *)d2av_stage_kernel<ORDER>, tiles < cap ? tiles : cap, DNT, smem, s, args);
 }
 
 }  // namespace

@@ -187,7 +187,7 @@ __device__ __forceinline__ void load_cell(const double *buf, const GridDev &gd, 
     for (int q = 0; q < 4; ++q) U[q] = buf[e + q * gd.plane];
 }
 
-constexpr int KTX = 32, KTY = 16, KNT = 256, KG = 2;
+constexpr int KTX = 32, KTY = 15, KNT = 256, KG = 2;
 constexpr int KSW = KTX + 2 * KG, KSH = KTY + 2 * KG, KPL = KSW * KSH;
 constexpr int EW = KTX + 1, EH = KTY + 1, EPL = EW * EH;  // a tile and its right / top neighbours
 
@@ -329,6 +329,13 @@ __device__ __noinline__ void k_face_any(const double *U, const double *Wuvp, con
     }
 }
 
+// where the sensor pass of a stage leaves its max; the pass of the stage before
+// clears it, so no launch does that alone
+__device__ __forceinline__ unsigned long long *sensor_word(Ctrl *c, int stage)
+{
+    return stage == 1 ? &c->aux : &c->aux23[stage - 2];
+}
+
 // store a per-cell scalar and its ghost images (no sign: it is even in the
 // velocities)
 __device__ __forceinline__ void put_scalar(const GridDev &gd, double *buf, int j, int i, double v)
@@ -349,15 +356,20 @@ __device__ __forceinline__ void put_scalar(const GridDev &gd, double *buf, int j
 // state and entropy variables in shared memory)   keep_fv_euler_2d.cu:249-277
 // Each cell's entropy, its log and pow the costliest operations of the
 // scheme, goes to the plane `ent`, from which the stage kernel reads it.
-__global__ void __launch_bounds__(KNT) keep_ed_kernel(const GridDev gd, const double *buf, double *ent, int ntiles)
+__global__ void __launch_bounds__(KNT) keep_ed_kernel(const __grid_constant__ GridDev gd, int stage,
+                                                      const double *buf, double *ent, int ntiles)
 {
     __shared__ double sU[4][EPL], sV[4][EPL];
     __shared__ double sh[KNT / 32];
     const int tid = threadIdx.x, n = gd.n;
     const double gam = gd.gam, ygm1 = recip(gam - 1.);
     double m = 0.0;
+    grid_dependency();
+    // the sensor word of the next stage: nothing reads it during this one
+    if (blockIdx.x == 0 && tid == 0) *sensor_word(gd.ctrl, stage % 3 + 1) = 0ull;
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const int tx0 = (t % gd.tiles_x) * KTX, ty0 = (t / gd.tiles_x) * KTY;
+        if (t + (int)gridDim.x >= ntiles) grid_release();
         for (int k = tid; k < EPL; k += KNT) {
             const int r = k / EW, c = k - r * EW, j = ty0 + r, i = tx0 + c;
             double U[4] = {1, 0, 0, 2.5};  // admissible filler beyond the ghost layer
@@ -394,12 +406,12 @@ __global__ void __launch_bounds__(KNT) keep_ed_kernel(const GridDev gd, const do
     if (tid == 0) {
         double b = 0.0;
         for (int w = 0; w < KNT / 32; ++w) b = fmax(b, sh[w]);
-        atomicMax(&gd.ctrl->aux, (unsigned long long)__double_as_longlong(b));
+        atomicMax(sensor_word(gd.ctrl, stage), (unsigned long long)__double_as_longlong(b));
     }
 }
 
 // one SSP-RK3 stage of the KEEP scheme               keep_fv_euler_2d.cu:298-393
-__global__ void __launch_bounds__(KNT, 2) keep_stage_kernel(const GridDev gd, int stage, int ntiles)
+__global__ void __launch_bounds__(KNT, 2) keep_stage_kernel(const __grid_constant__ GridDev gd, int stage, int ntiles)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double *U = reinterpret_cast<double *>(smem_raw);  // [4][KSH][KSW] conserved, rho floored
@@ -407,7 +419,6 @@ __global__ void __launch_bounds__(KNT, 2) keep_stage_kernel(const GridDev gd, in
     double *V = W + 3 * KPL;                           // [4] entropy variables (Cartesian)
     double *FX = V + 4 * KPL;                          // [4][KTY][KTX+1]
     double *FY = FX + 4 * KTY * (KTX + 1);             // [4][KTY+1][KTX]
-    __shared__ TileCtl s_ctl;
     __shared__ double s_red[KNT / 32];
     const int tid = threadIdx.x, n = gd.n, np = n + 2 * KG;
     const double gam = gd.gam;
@@ -415,19 +426,15 @@ __global__ void __launch_bounds__(KNT, 2) keep_stage_kernel(const GridDev gd, in
     const double *u0 = (const double *)gd.st[0];
     double *out = (double *)(stage == 1 ? gd.k1 : stage == 2 ? gd.k2 : gd.st[0]);
     const double *ent = (const double *)gd.lo[0];  // the stage input's entropies (keep_ed_kernel)
-    const double edmax = __longlong_as_double((long long)gd.ctrl->aux);
+    grid_dependency();
+    const double edmax = __longlong_as_double((long long)*sensor_word(gd.ctrl, stage));
     const double inv_h = 1. / gd.h;
+    // the step control, the same for every tile
+    const TileCtl ctl = tile_control<P64>(gd.ctrl, stage, tid == 0 && blockIdx.x == 0);
     const KFace kf{gam, recip(gam - 1.), edmax, 12. / (edmax + 1e-30)};
 
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+    for (int t = blockIdx.x; t < ntiles && ctl.run; t += gridDim.x) {
         const int tx0 = (t % gd.tiles_x) * KTX, ty0 = (t / gd.tiles_x) * KTY;
-        if (tid == 0) s_ctl = tile_control<P64>(gd.ctrl, stage, t == 0);
-        __syncthreads();
-        const TileCtl ctl = s_ctl;
-        if (!ctl.run) {
-            __syncthreads();
-            continue;
-        }
         // conserved state of the box; primitives and entropy variables of the
         // cells next to a face (the outer ring is the JST stencil's alone)
         for (int k = tid; k < KPL; k += KNT) {
@@ -488,6 +495,7 @@ __global__ void __launch_bounds__(KNT, 2) keep_stage_kernel(const GridDev gd, in
             for (int q = 0; q < 4; ++q) o[q * (KTY + 1) * KTX] = F[q];
         }
         __syncthreads();
+        if (t + (int)gridDim.x >= ntiles) grid_release();
         double lmax = 0.0;
         for (int k = tid; k < KTX * KTY; k += KNT) {
             const int r = k / KTX, c = k - r * KTX, i = tx0 + c, j = ty0 + r;
@@ -568,22 +576,21 @@ void keep_tiles(int n, int &tiles_x, int &tiles)
     tiles = tiles_x * ((n + KTY - 1) / KTY);
 }
 
-// one KEEP stage: clear the sensor max, the entropy-distance pass, then the
-// fused flux / RK / ghost kernel
+// one KEEP stage: the entropy-distance pass, then the fused flux / RK / ghost
+// kernel
 cudaError_t keep_launch_stage(const GridDev &gd, int stage, int tiles, cudaStream_t s)
 {
     LaunchFacts f{};
     cudaError_t e = launch_facts((const void *)keep_stage_kernel, KNT, keep_smem(), f);
     if (e != cudaSuccess) return e;
-    const int ctas_per_sm = f.ctas_per_sm, sms = f.sms;
-    const void *in = stage == 2 ? gd.k1 : stage == 3 ? gd.k2 : gd.st[0];
-    e = cudaMemsetAsync(&gd.ctrl->aux, 0, sizeof(unsigned long long), s);
+    const double *in = (const double *)(stage == 2 ? gd.k1 : stage == 3 ? gd.k2 : gd.st[0]);
+    double *ent = (double *)gd.lo[0];
+    const int eb = tiles < 4 * f.sms ? tiles : 4 * f.sms, cap = f.ctas_per_sm * f.sms;
+    void *ea[] = {(void *)&gd, (void *)&stage, (void *)&in, (void *)&ent, (void *)&tiles};
+    e = launch_chained((const void *)keep_ed_kernel, eb, KNT, 0, s, ea);
     if (e != cudaSuccess) return e;
-    const int eb = tiles < 4 * sms ? tiles : 4 * sms;
-    keep_ed_kernel<<<eb, KNT, 0, s>>>(gd, (const double *)in, (double *)gd.lo[0], tiles);
-    const int grid = tiles < ctas_per_sm * sms ? tiles : ctas_per_sm * sms;
-    keep_stage_kernel<<<grid, KNT, keep_smem(), s>>>(gd, stage, tiles);
-    return cudaGetLastError();
+    void *sa[] = {(void *)&gd, (void *)&stage, (void *)&tiles};
+    return launch_chained((const void *)keep_stage_kernel, tiles < cap ? tiles : cap, KNT, keep_smem(), s, sa);
 }
 
 cudaError_t keep_lam_into(const GridDev &gd, cudaStream_t s)
