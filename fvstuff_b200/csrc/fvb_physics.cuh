@@ -91,110 +91,6 @@ template <class R> __device__ __forceinline__ void c2p(const R c[4], R w[4], con
     w[3] = gs.gm1 * (c[3] - FVB_LIT(R, 0.5) * (c[1] * c[1] + c[2] * c[2]) / c[0]);
 }
 
-// pressure-jump sensor s = dp^2 / (dp^2 + 0.1 (pa+pb)^2)
-//                                               fv_up7_ducros_2d.cu:114-133
-template <class R> __device__ __forceinline__ R ducros(R pa, R pb)
-{
-    R dp = pb - pa, ps = pb + pa;
-    return dp * dp / (dp * dp + FVB_LIT(R, 0.1) * ps * ps);
-}
-
-// Upwind-biased face values from the 2g-point stencil s[0..2g-1] along the
-// normal (the face lies between s[g-1] and s[g]); arithmetic in RR, result
-// rounded to R.                                 fv_up7_ducros_2d.cu:149-186
-template <class R, class RR, int ORDER>
-__device__ __forceinline__ void upface(const R *s, R &vL, R &vR)
-{
-    if constexpr (ORDER == 3) {
-        vL = R((-RR(s[0]) + RR(5.0) * s[1] + RR(2.0) * s[2]) / RR(6.0));
-        vR = R((RR(2.0) * s[1] + RR(5.0) * s[2] - RR(s[3])) / RR(6.0));
-    } else if constexpr (ORDER == 5) {
-        vL = R((RR(2.0) * s[0] - RR(13.0) * s[1] + RR(47.0) * s[2] + RR(27.0) * s[3] - RR(3.0) * s[4]) / RR(60.0));
-        vR = R((-RR(3.0) * s[1] + RR(27.0) * s[2] + RR(47.0) * s[3] - RR(13.0) * s[4] + RR(2.0) * s[5]) / RR(60.0));
-    } else if constexpr (ORDER == 9) {
-        // the published UP9 weights, as they stand (the left-biased set sums
-        // to 4217/2520, not one)                 fv_up7_ducros_2d.cu:176-186
-        vL = R((RR(3.0) * s[0] - RR(25.0) * s[1] + RR(101.0) * s[2] - RR(319.0) * s[3] + RR(2765.0) * s[4]
-                + RR(2139.0) * s[5] - RR(533.0) * s[6] + RR(97.0) * s[7] - RR(11.0) * s[8]) / RR(2520.0));
-        vR = R((-RR(11.0) * s[1] + RR(97.0) * s[2] - RR(533.0) * s[3] + RR(2139.0) * s[4] + RR(2765.0) * s[5]
-                - RR(319.0) * s[6] + RR(101.0) * s[7] - RR(25.0) * s[8] + RR(3.0) * s[9]) / RR(2520.0));
-    } else {
-        static_assert(ORDER == 7, "ORDER must be 3, 5, 7 or 9");
-        vL = R((-RR(3.0) * s[0] + RR(25.0) * s[1] - RR(101.0) * s[2] + RR(319.0) * s[3]
-                + RR(214.0) * s[4] - RR(38.0) * s[5] + RR(4.0) * s[6]) / RR(420.0));
-        vR = R((RR(4.0) * s[1] - RR(38.0) * s[2] + RR(214.0) * s[3] + RR(319.0) * s[4]
-                - RR(101.0) * s[5] + RR(25.0) * s[6] - RR(3.0) * s[7]) / RR(420.0));
-    }
-}
-
-// total energy of a normal-frame state with the kinetic term summed in the
-// Cartesian order u^2 + v^2, as the reference sums it for every face: for a
-// y-face (YF) the normal component is v, so the tangential square comes
-// first (the two orders round differently under a fused multiply-add)
-template <bool YF, class R>
-__device__ __forceinline__ R etot_cart(R r, R un, R ut, R p, const Gas<R> &gs)
-{
-    return YF ? etot(r, ut, un, p, gs) : etot(r, un, ut, p, gs);
-}
-
-// HLLC with Davis wave-speed bounds, normal frame (YF: a y-face)
-//                                               fv_up7_ducros_2d.cu:237-292
-template <class R, bool YF = false>
-__device__ __forceinline__ void hllc(const R L[4], const R Rr[4], R F[4], const Gas<R> &gs)
-{
-    R rL = L[0], uL = L[1], tL = L[2], pL = L[3];
-    R rR = Rr[0], uR = Rr[1], tR = Rr[2], pR = Rr[3];
-    R cL = sound(pL, rL, gs), cR = sound(pR, rR, gs);
-    R EL = etot_cart<YF>(rL, uL, tL, pL, gs), ER = etot_cart<YF>(rR, uR, tR, pR, gs);
-    R SL = dmin<R>(uL - cL, uR - cR);
-    R SR = dmax<R>(uL + cL, uR + cR);
-    const R zero = R(0);
-    if (SL >= zero) {
-        F[0] = rL * uL; F[1] = rL * uL * uL + pL; F[2] = rL * uL * tL; F[3] = (EL + pL) * uL;
-        return;
-    }
-    if (SR <= zero) {
-        F[0] = rR * uR; F[1] = rR * uR * uR + pR; F[2] = rR * uR * tR; F[3] = (ER + pR) * uR;
-        return;
-    }
-    R dL = rL * (SL - uL), dR = rR * (SR - uR);
-    R Ss = (pR - pL + dL * uL - dR * uR) / (dL - dR);
-    bool left = (Ss >= zero);
-    R rK = left ? rL : rR, uK = left ? uL : uR, tK = left ? tL : tR;
-    R pK = left ? pL : pR, EK = left ? EL : ER, SK = left ? SL : SR;
-    R fact = rK * (SK - uK) / (SK - Ss);
-    R Us1 = fact * Ss, Us2 = fact * tK;
-    R Us3 = fact * (EK / rK + (Ss - uK) * (Ss + pK / (rK * (SK - uK))));
-    F[0] = rK * uK + SK * (fact - rK);
-    F[1] = rK * uK * uK + pK + SK * (Us1 - rK * uK);
-    F[2] = rK * uK * tK + SK * (Us2 - rK * tK);
-    F[3] = (EK + pK) * uK + SK * (Us3 - EK);
-}
-
-// HLLE on the two adjacent cell averages, normal frame (YF: a y-face)
-//                                               fv_up7_ducros_2d.cu:296-328
-template <class R, bool YF = false>
-__device__ __forceinline__ void hlle(const R L[4], const R Rr[4], R F[4], const Gas<R> &gs)
-{
-    R rL = L[0], uL = L[1], tL = L[2], pL = L[3];
-    R rR = Rr[0], uR = Rr[1], tR = Rr[2], pR = Rr[3];
-    R cL = sound(pL, rL, gs), cR = sound(pR, rR, gs);
-    R EL = etot_cart<YF>(rL, uL, tL, pL, gs), ER = etot_cart<YF>(rR, uR, tR, pR, gs);
-    R FL0 = rL * uL, FL1 = rL * uL * uL + pL, FL2 = rL * uL * tL, FL3 = (EL + pL) * uL;
-    R FR0 = rR * uR, FR1 = rR * uR * uR + pR, FR2 = rR * uR * tR, FR3 = (ER + pR) * uR;
-    R SL = dmin<R>(uL - cL, uR - cR);
-    R SR = dmax<R>(uL + cL, uR + cR);
-    const R zero = R(0);
-    if (SL >= zero) { F[0] = FL0; F[1] = FL1; F[2] = FL2; F[3] = FL3; return; }
-    if (SR <= zero) { F[0] = FR0; F[1] = FR1; F[2] = FR2; F[3] = FR3; return; }
-    R dS = dmax<R>(SR - SL, FVB_LIT(R, 1e-10));
-    R SRL = SR * SL;
-    F[0] = (SR * FL0 - SL * FR0 + SRL * (rR - rL)) / dS;
-    F[1] = (SR * FL1 - SL * FR1 + SRL * (rR * uR - rL * uL)) / dS;
-    F[2] = (SR * FL2 - SL * FR2 + SRL * (rR * tR - rL * tL)) / dS;
-    F[3] = (SR * FL3 - SL * FR3 + SRL * (ER - EL)) / dS;
-}
-
 // Reciprocal and square root per arithmetic type.  Every argument on these
 // paths is a positive normal number (densities and pressures are floored at
 // 1e-14, wave-speed spans at 1e-10, sound speeds squared at 1e-14).

@@ -29,40 +29,62 @@
 #include "fvb_physics.cuh"
 #include "fvb_device.cuh"
 #include "fvb_tma.cuh"
+#include "fvb_face32.cuh"
 
 namespace fvb {
 
-// Flux through one face of the working tile W ([4][SH][SW]: rho, u, v, p)
-// whose right/top cell is at `base`; XDIR: x-face (normal u), else
-// y-face (normal v).  Writes the 4 Cartesian components to out[q * ostride].
-template <int ORDER, int SW, int PL, bool XDIR>
-__device__ __forceinline__ void face_one(const float *W, int base, float *out, int ostride, const Gas<float> &gs)
+// Flux through one face of the working tile W ([4][SH][SW]: rho, u, v, p in
+// FP64) whose right/top cell is at `base`, its sound speed at ce[0] and its
+// energy for x- and y-faces at ce[CP], ce[2 CP] (the left/bottom cell's cs
+// before); XDIR: x-face (normal u),
+// else y-face (normal v).  Writes the 4 Cartesian components to
+// out[q * ostride].
+template <int SW, int PL, int CP, bool XDIR>
+__device__ __forceinline__ void face_one(const double *W, int base, const float *ce, int cs, float *out, int ostride,
+                                         const f32::Gas &gs)
 {
-    using R = float;
-    using RR = double;  // the reconstruction's arithmetic, as shipped
-    constexpr int G = (ORDER + 1) / 2;
+    constexpr int G = 4;
     constexpr int ST = XDIR ? 1 : SW;
+    constexpr int EO = XDIR ? CP : 2 * CP;
     constexpr int QN = XDIR ? 1 : 2, QT = XDIR ? 2 : 1;
     constexpr int QS[4] = {0, QN, QT, 3};
-    R L[4], Rv[4], WL[4], WR[4];
+    float L[4], Rv[4], WL[4], WR[4];
 #pragma unroll
     for (int m = 0; m < 4; ++m) {
-        const R *v = W + QS[m] * PL + base;
-        R s[2 * G];
+        const double *v = W + QS[m] * PL + base;
+        double s[2 * G];
 #pragma unroll
         for (int d = 0; d < 2 * G; ++d) s[d] = v[(d - G) * ST];
-        upface<R, RR, ORDER>(s, L[m], Rv[m]);
-        WL[m] = s[G - 1];
-        WR[m] = s[G];
+        f32::upface7(s, L[m], Rv[m]);
+        WL[m] = (float)s[G - 1];
+        WR[m] = (float)s[G];
     }
-    L[0] = floor14(L[0]); Rv[0] = floor14(Rv[0]);
-    L[3] = floor14(L[3]); Rv[3] = floor14(Rv[3]);
-    R Fn[4];
-    R Fh[4], Fl[4];
-    hllc<R, !XDIR>(L, Rv, Fh, gs);
-    hlle<R, !XDIR>(WL, WR, Fl, gs);
-    const R sd = ducros<R>(WL[3], WR[3]);
-    const R one_m = R(1) - sd;
+    // (a NaN here may stand for an infinity of the operators)
+    const float z = (L[0] + Rv[0]) + (L[1] + Rv[1]) + (L[2] + Rv[2]) + (L[3] + Rv[3]);
+    if (z != z) {
+#pragma unroll 1
+        for (int m = 0; m < 4; ++m) {
+            double s[2 * G], tL, tR;
+            const double *v = W + (m == 1 ? QN : m == 2 ? QT : m) * PL + base;
+#pragma unroll
+            for (int d = 0; d < 2 * G; ++d) s[d] = v[(d - G) * ST];
+            f32::sums7(s, tL, tR);
+            const float l = (float)(tL / 420.0), r = (float)(tR / 420.0);
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (k == m) {
+                    L[k] = l;
+                    Rv[k] = r;
+                }
+        }
+    }
+    L[0] = f32::fl14(L[0]); Rv[0] = f32::fl14(Rv[0]);
+    L[3] = f32::fl14(L[3]); Rv[3] = f32::fl14(Rv[3]);
+    float Fn[4], Fh[4], Fl[4];
+    f32::hllc(L, Rv, Fh, gs);
+    f32::hlle(WL, WR, ce[-cs], ce[0], ce[EO - cs], ce[EO], Fl);
+    const float sd = f32::ducros(WL[3], WR[3]);
+    const float one_m = 1.f - sd;
 #pragma unroll
     for (int q = 0; q < 4; ++q) Fn[q] = one_m * Fh[q] + sd * Fl[q];
     out[0] = Fn[0];
@@ -71,21 +93,39 @@ __device__ __forceinline__ void face_one(const float *W, int base, float *out, i
     out[3 * ostride] = Fn[3];
 }
 
-template <int ORDER, int TX, int TY, int NT, int MINB>
+// shared memory of a tile shape: the box as loaded, the working tile in FP64,
+// sound speed and energy of the cells -1 .. TX, -1 .. TY, the fluxes
+template <int TX, int TY>
+struct L32 {
+    static constexpr int SW = TX + 8, SH = TY + 8, PL = SW * SH, CW = TX + 2, CP = CW * (TY + 2);
+    static constexpr size_t smem = sizeof(double) * 4 * PL + sizeof(float) * (4 * PL + 3 * CP + 4 * TY * (TX + 1) +
+                                                                              4 * (TY + 1) * TX);
+};
+
+// The FP32 form as shipped.  What bounds it is instruction issue: per face the
+// reference's order asks for 64 FP64 operations of the reconstruction and the
+// roundings back, 5 divisions and 2 roots.  The working tile is FP64, so a cell
+// is converted once and not by each of its 64 stencil uses (an eighth-rate
+// instruction), the divisions by 420 and by the HLLE's span come from
+// reciprocals with the same bits (fvb_face32.cuh), and each cell's HLLE sound
+// speed and energy are formed once: 2107 -> 1568 instructions a cell, 34 -> 21 us a stage
+// at 400^2 (351 tiles), bit-identical.
+template <int TX, int TY, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB) stage32_kernel(const __grid_constant__ StageArgs a)
 {
     constexpr int PREC = P32;
     using R = float;
-    constexpr int G = (ORDER + 1) / 2;
-    constexpr int SW = TX + 2 * G, SH = TY + 2 * G, PL = SW * SH;
+    using LS = L32<TX, TY>;
+    constexpr int G = 4, SW = LS::SW, SH = LS::SH, PL = LS::PL, CW = LS::CW, CP = LS::CP;
     constexpr int NXF = (TX + 1) * TY, NYF = TX * (TY + 1);
     constexpr int NW = NT / 32;
     // IN: the tile as loaded (TMA lands here); W: the primitives the faces
     // are computed from, so IN can take the next tile meanwhile
     extern __shared__ __align__(128) unsigned char smem_raw[];
     R *IN = reinterpret_cast<R *>(smem_raw);
-    R *W = IN + 4 * PL;
-    R *FX = W + 4 * PL;               // [4][TY][TX+1]
+    double *W = reinterpret_cast<double *>(IN + 4 * PL);
+    R *CE = reinterpret_cast<R *>(W + 4 * PL);  // [3][TY+2][TX+2]
+    R *FX = CE + 3 * CP;              // [4][TY][TX+1]
     R *FY = FX + 4 * TY * (TX + 1);   // [4][TY+1][TX]
     __shared__ double s_red[NW];
     __shared__ __align__(8) uint64_t s_bar;
@@ -137,6 +177,7 @@ __global__ void __launch_bounds__(NT, MINB) stage32_kernel(const __grid_constant
     // tile is tile 0)
     double lacc = 0.0;
     TileCtl ctl{};
+    const R ygm1 = __frcp_rn(R(a.grid.gam) - R(1));
     if (t < ntiles) ctl = tile_control<PREC>(a.grid.ctrl, a.stage, tid == 0 && t == 0);
     for (; t < ntiles; t += stride) {
         const bool has_next = t + stride < ntiles;
@@ -145,13 +186,26 @@ __global__ void __launch_bounds__(NT, MINB) stage32_kernel(const __grid_constant
         const int n = gd.n;
         const int tx0 = (tile % gd.tiles_x) * TX, ty0 = (tile / gd.tiles_x) * TY;
         const Gas<R> gs{R(gd.gam), R(gd.gam) - R(1)};
+        const f32::Gas g32{gs.gam, gs.gm1, ygm1};
         if (s_err) {
             // a halo load never arrived: record it, skip the tile
             if (tid == 0 && gd.ctrl) gd.ctrl->status = FVB_ERR_TIMEOUT;
             break;
         }
         if (ctl.run && a.stage >= 0) {
-            for (int k = tid; k < 4 * PL; k += NT) W[k] = IN[k];
+            for (int k = tid; k < PL; k += NT) {
+                const R w0 = IN[k], w1 = IN[PL + k], w2 = IN[2 * PL + k], w3 = IN[3 * PL + k];
+                W[k] = w0;
+                W[PL + k] = w1;
+                W[2 * PL + k] = w2;
+                W[3 * PL + k] = w3;
+                const int r = k / SW - (G - 1), c = k % SW - (G - 1);
+                if ((unsigned)r < (unsigned)(TY + 2) && (unsigned)c < (unsigned)CW) {
+                    CE[r * CW + c] = f32::sound(w3, w0, g32);
+                    CE[CP + r * CW + c] = f32::energy(w0, w1, w2, w3, g32);
+                    CE[2 * CP + r * CW + c] = f32::energy(w0, w2, w1, w3, g32);
+                }
+            }
         }
         __syncthreads();
         // ---- 2. load the next tile into IN (asynchronous through TMA) -------
@@ -185,11 +239,13 @@ __global__ void __launch_bounds__(NT, MINB) stage32_kernel(const __grid_constant
         // ---- 3. face fluxes: x-faces, then y-faces (compile-time strides) ---
         for (int f = tid; f < NXF; f += NT) {
             const int r = f / (TX + 1), c = f - r * (TX + 1);
-            face_one<ORDER, SW, PL, true>(W, (r + G) * SW + (c + G), FX + r * (TX + 1) + c, TY * (TX + 1), gs);
+            face_one<SW, PL, CP, true>(W, (r + G) * SW + (c + G), CE + (r + 1) * CW + c + 1, 1,
+                                       FX + r * (TX + 1) + c, TY * (TX + 1), g32);
         }
         for (int f = tid; f < NYF; f += NT) {
             const int r = f / TX, c = f - r * TX;
-            face_one<ORDER, SW, PL, false>(W, (r + G) * SW + (c + G), FY + r * TX + c, (TY + 1) * TX, gs);
+            face_one<SW, PL, CP, false>(W, (r + G) * SW + (c + G), CE + (r + 1) * CW + c + 1, CW, FY + r * TX + c,
+                                        (TY + 1) * TX, g32);
         }
         __syncthreads();
 
@@ -214,14 +270,15 @@ __global__ void __launch_bounds__(NT, MINB) stage32_kernel(const __grid_constant
                 R *rhs = (R *)a.rhs;
                 size_t n2 = (size_t)n * n, kk = (size_t)j * n + i;
                 for (int q = 0; q < 4; ++q) rhs[q * n2 + kk] = res[q];
-                ((R *)a.lam)[kk] = dabs<R>(W[PL + sc]) + dabs<R>(W[2 * PL + sc]) + sound<R>(W[3 * PL + sc], W[sc], gs);
+                ((R *)a.lam)[kk] = dabs<R>((R)W[PL + sc]) + dabs<R>((R)W[2 * PL + sc]) +
+                                   sound<R>((R)W[3 * PL + sc], (R)W[sc], gs);
                 continue;
             }
             {
                 // the reference's update
                 R wk[4], w0[4], c0[4], cv[4], w[4];
 #pragma unroll
-                for (int q = 0; q < 4; ++q) wk[q] = W[q * PL + sc];
+                for (int q = 0; q < 4; ++q) wk[q] = (R)W[q * PL + sc];
                 if (a.stage == 1) {
 #pragma unroll
                     for (int q = 0; q < 4; ++q) w0[q] = wk[q];
@@ -290,11 +347,8 @@ template <int SHAPE>
 static StageKernel entry32()
 {
     constexpr TileShape ts = kTileShapes[SHAPE];
-    constexpr int G = 4;
-    constexpr size_t smem = sizeof(float) * (8 * (ts.ty + 2 * G) * (ts.tx + 2 * G) + 4 * ts.ty * (ts.tx + 1) +
-                                             4 * (ts.ty + 1) * ts.tx);
     // three CTAs an SM, the registers' budget (80 at 256 threads)
-    return StageKernel{(void *)stage32_kernel<7, ts.tx, ts.ty, ts.nt, 3>, nullptr, smem, ts.nt};
+    return StageKernel{(void *)stage32_kernel<ts.tx, ts.ty, ts.nt, 3>, nullptr, L32<ts.tx, ts.ty>::smem, ts.nt};
 }
 
 // the kernel of a form, an order, a tile variant and a solver on the
