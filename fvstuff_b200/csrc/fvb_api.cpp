@@ -868,6 +868,38 @@ fvb_status fvb_set_graph(fvb_solver *s, int enable)
 
 // ---- kernel-level contract ---------------------------------------------
 
+}  // extern "C"
+
+// Tile shape and CTAs of a residual launch, by rule (one call: nothing to
+// tune).  A grid whose small tiles fit the SMs at once is latency-bound and
+// takes the most tiles: FP64 16x7 split (one CTA an SM; 100^2: 8.2 us against
+// 10.2 with 32x15, 150^2: equal), then 32x7 while 32x15 would leave CTA slots
+// empty (257^2: 12.3 against 14.3, 362^2: equal); FP32 16x15 (100^2: 12.3
+// against 14.3, 257^2: 14.3 against 16.4, 362^2: equal).  Beyond, 32x15: in
+// FP64 one CTA a slot, which loads its next tile under the current one (1000^2:
+// 57 us, one CTA a tile 60); the FP32 kernel has one buffer and gains nothing
+// from it (1000^2: 70 and 70; 2048^2: 244, one CTA a tile 241).
+static cudaError_t rhs_launch_shape(int prec, int order, int n, int &shape, int &ctas)
+{
+    int dev = 0, sms = 0, tx, tiles;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    tile_dims(prec, shape = 3, n, tx, tiles);
+    ctas = tiles;
+    if (tiles <= (prec == P64 ? 1 : 3) * sms) return cudaSuccess;
+    tile_dims(prec, shape = 0, n, tx, tiles);
+    ctas = tiles;
+    if (prec == P32) return cudaSuccess;
+    if (tiles <= 2 * sms) tile_dims(prec, shape = 1, n, tx, tiles);
+    const int slots = stage_max_ctas_per_sm(prec, order, shape) * sms;
+    if (slots <= 0) return cudaErrorInvalidConfiguration;
+    ctas = std::min(tiles, slots);
+    return cudaSuccess;
+}
+
+extern "C" {
+
 fvb_status fvb_up_rhs(const void *Qp, void *rhs, void *lam, int n, int np, int order, double h, double gamma,
                       int dtype, void *stream)
 {
@@ -886,14 +918,16 @@ fvb_status fvb_up_rhs(const void *Qp, void *rhs, void *lam, int n, int np, int o
     set_scales(gd, h, gamma);
     gd.st[0] = (void *)Qp;
     gd.ctrl = nullptr;
-    const int shape = 0, prec = dtype == FVB_F64 ? P64 : P32;
-    int tiles;
+    const int prec = dtype == FVB_F64 ? P64 : P32;
+    int shape, ctas, tiles;
+    cudaError_t e = rhs_launch_shape(prec, order, n, shape, ctas);
+    if (e != cudaSuccess) return cuda_fail(e, "fvb_up_rhs");
     tile_dims(prec, shape, n, gd.tiles_x, tiles);
     a.ntiles_static = tiles;
     a.stage = 0;
     a.rhs = rhs;
     a.lam = lam;
-    cudaError_t e = launch_stage(prec, order, shape, a, tiles, (cudaStream_t)stream);
+    e = launch_stage(prec, order, shape, a, ctas, (cudaStream_t)stream);
     return e == cudaSuccess ? FVB_OK : cuda_fail(e, "fvb_up_rhs");
 }
 

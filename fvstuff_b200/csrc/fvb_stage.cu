@@ -148,6 +148,8 @@ __global__ void __launch_bounds__(NT, MINB) stage32_kernel(const __grid_constant
         if (tma) {
             if (mbar_wait(&s_bar, phase)) phase ^= 1;
             else s_err = 1;
+        } else {
+            cp_async_wait();
         }
         __syncthreads();
     };

@@ -107,6 +107,7 @@ __global__ void __launch_bounds__(NT, (L64<ORDER, TX, TY, NT>::MINB)) stage64_ke
     };
     auto wait_box = [&](int m, bool tma) {
         if (tma) wait_bar(m);
+        else cp_async_wait();
         __syncthreads();
     };
     // single grid: start the halo-box load of tile t (every thread: the

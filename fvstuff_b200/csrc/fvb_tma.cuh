@@ -74,8 +74,22 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity)
     }
 }
 
+// asynchronous copy of one value global -> shared (in == false: a zero), for
+// arrays that have no tensor map (a caller's own, of any pitch and alignment);
+// cp_async_wait() before the block barrier that publishes the copies
+template <class R>
+__device__ __forceinline__ void cp_async(R *dst, const R *src, bool in)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(smem_u32(dst)), "l"(src), "n"(sizeof(R)),
+                 "r"(in ? (int)sizeof(R) : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // The halo box of a tile in one grid: TMA when the grid has descriptors,
-// else cooperative loads by the whole CTA (the caller's IDX_P arrays).
+// else cooperative loads by the whole CTA (the caller's IDX_P arrays);
+// asynchronous ones in the FP32 kernel, the only form that the residual of a
+// caller's arrays takes through here.
 template <int PREC, int G, int SW, int SH, int NT, class R>
 __device__ __forceinline__ void issue_tile_load(const GridDev &gd, int stage, int parity, int tile, R *IN,
                                                 uint64_t *bar, int tid)
@@ -106,6 +120,10 @@ __device__ __forceinline__ void issue_tile_load(const GridDev &gd, int stage, in
         bool in = jp < np && ip < np;
         long long e = (long long)jp * gd.pitch + ip + gd.xoff;
         for (int q = 0; q < 4; ++q) {
+            if (PREC == P32) {
+                cp_async(IN + q * SH * SW + k, in ? src + e + q * gd.plane : src, in);
+                continue;
+            }
             IN[q * SH * SW + k] = in ? src[e + q * gd.plane] : R(0);
             if (two) IN[(4 + q) * SH * SW + k] = in ? inc[e + q * gd.plane] : R(0);
         }
@@ -134,8 +152,9 @@ __device__ __forceinline__ void issue_tile_load64(const GridDev &gd, int stage, 
     for (int k = tid; k < PL; k += NT) {
         const int r = k / SW, c = k - r * SW, jp = ty0 + r, ip = tx0 + c - XO;
         const bool in = jp < np && ip >= 0 && ip < np;
-        const long long e = (long long)jp * gd.pitch + ip + gd.xoff;
-        for (int q = 0; q < 4; ++q) IN[q * PL + k] = in ? src[e + q * gd.plane] : 0.0;
+        const double *v = in ? src + ((long long)jp * gd.pitch + ip + gd.xoff) : src;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) cp_async(IN + q * PL + k, in ? v + q * gd.plane : src, in);
     }
 }
 
@@ -188,6 +207,7 @@ struct BoxPipe {
     __device__ __forceinline__ void finish_box(const GridDev &gd, int m, bool issued)
     {
         if (issued && gd.tmap) wait(m);
+        else cp_async_wait();
         __syncthreads();
     }
     // a load whose wait gave up may still be in flight: wait once more, so no
