@@ -212,8 +212,10 @@ __global__ void __launch_bounds__(NT, MinBlocks32c<NT>::v) stage32c_kernel(const
         s_err = 0;
     }
     __syncthreads();
-    grid_dependency();
     const int ntiles = batched ? *a.ntiles : a.ntiles_static;
+    BatchHead head{};
+    if (batched && tid < 32) head = batch_head(a, &s_hdr[0], ntiles, tid);
+    grid_dependency();
 
     // every thread waits on the mbarrier itself (the completed phase makes the
     // TMA bytes visible to it); the barrier after the wait also agrees on s_err
@@ -258,11 +260,11 @@ __global__ void __launch_bounds__(NT, MinBlocks32c<NT>::v) stage32c_kernel(const
     int t = blockIdx.x, slot = 0;
     if (t < ntiles && batched) {
         if (tid < 32) {
-            const TileRef r0 = a.tiles[t];
-            start_batched_tile<P32C>(a, &s_hdr[0], r0, hdr_word(a, r0, tid), &s_bar, tid, [&](const TileHdr &h) {
+            const TileRef r0 = head.first;
+            start_first_tile<P32C>(a, &s_hdr[0], r0, &s_bar, tid, [&](const TileHdr &h) {
                 issue_tile_load<P32C, G, SW, SH, NT>(h.gd, a.stage, cur, r0.tile, IN, &s_bar, 0);
             });
-            if (tid == 0 && t + stride < ntiles) s_ref_next = a.tiles[t + stride];
+            if (tid == 0) s_ref_next = head.next;
         }
         wait_box(true);
     } else if (drop) {
@@ -543,8 +545,10 @@ __global__ void __launch_bounds__((RowPair<TX, TY>::NT), (RowPair<TX, TY>::MINB)
         s_err = 0;
     }
     __syncthreads();
-    grid_dependency();
     const int ntiles = batched ? *a.ntiles : a.ntiles_static;
+    BatchHead head{};
+    if (batched && tid < 32) head = batch_head(a, &s_hdr[0], ntiles, tid);
+    grid_dependency();
 
     uint32_t phase = 0;
     auto wait_box = [&](bool tma) {
@@ -576,11 +580,11 @@ __global__ void __launch_bounds__((RowPair<TX, TY>::NT), (RowPair<TX, TY>::MINB)
     int t = blockIdx.x, slot = 0;
     if (t < ntiles && batched) {
         if (tid < 32) {
-            const TileRef r0 = a.tiles[t];
-            start_batched_tile<P32C>(a, &s_hdr[0], r0, hdr_word(a, r0, tid), &s_bar, tid, [&](const TileHdr &h) {
+            const TileRef r0 = head.first;
+            start_first_tile<P32C>(a, &s_hdr[0], r0, &s_bar, tid, [&](const TileHdr &h) {
                 issue_tile_load<P32C, G, SW, SH, NT>(h.gd, a.stage, cur, r0.tile, IN, &s_bar, 0);
             });
-            if (tid == 0 && t + stride < ntiles) s_ref_next = a.tiles[t + stride];
+            if (tid == 0) s_ref_next = head.next;
         }
         wait_box(true);
     } else if (drop) {

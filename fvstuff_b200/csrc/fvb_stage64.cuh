@@ -89,8 +89,10 @@ __global__ void __launch_bounds__(NT, (L64<ORDER, TX, TY, NT>::MINB)) stage64_ke
         s_err = 0;
     }
     __syncthreads();
-    grid_dependency();
     const int ntiles = BATCHED ? *a.ntiles : a.ntiles_static;
+    BatchHead head{};
+    if (BATCHED && tid < 32) head = batch_head(a, &s_hdr[0], ntiles, tid);
+    grid_dependency();
 
     // every thread waits on the mbarrier itself (the completed phase makes the
     // TMA bytes visible to it); the barrier after the wait also agrees on s_err
@@ -127,11 +129,11 @@ __global__ void __launch_bounds__(NT, (L64<ORDER, TX, TY, NT>::MINB)) stage64_ke
     int t = blockIdx.x, buf = 0;
     if (t < ntiles && BATCHED) {
         if (tid < 32) {
-            const TileRef r0 = a.tiles[t];
-            start_batched_tile<P64>(a, &s_hdr[0], r0, hdr_word(a, r0, tid), &s_bar[0], tid, [&](const TileHdr &h) {
+            const TileRef r0 = head.first;
+            start_first_tile<P64>(a, &s_hdr[0], r0, &s_bar[0], tid, [&](const TileHdr &h) {
                 issue_tile_load64<G, TX, TY, SW, XO, NT>(h.gd, a.stage, r0.tile, sm, &s_bar[0], 0);
             });
-            if (tid == 0 && t + stride < ntiles) s_ref_next = a.tiles[t + stride];
+            if (tid == 0) s_ref_next = head.next;
         }
         wait_box(0, true);
     } else if (drop) {
