@@ -33,7 +33,7 @@ struct Ctrl {
                                 // issues no first halo-box load (its wait must run out)
     unsigned long long aux;     // KEEP: bit pattern of the entropy-distance max of stage 1's
                                 // input; rec3: count of 2x2 blocks given the brutal mean fix
-    unsigned long long aux23[2];  // KEEP: the same of stages 2 and 3
+    unsigned long long aux23[2];  // KEEP: the same of stages 2 and 3; rec3: the stages' tile counters
 };
 
 // Device view of one grid.  Element (q, jp, ip) of a padded buffer, padded

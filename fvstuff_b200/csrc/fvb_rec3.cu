@@ -460,6 +460,16 @@ __device__ __forceinline__ bool r3_face(const double *Q, int f, double *FP)
     return true;
 }
 
+// Tiles of a stage are handed out as CTAs come free: the shock's tiles, with
+// bisected faces and limited blocks, cost several times the others, and with
+// a fixed share of the tiles a CTA the SMs were busy 79 % of a stage (1024^2
+// circular Sod: a stage 105 us, now 94).  The counter of `stage`, zero when it begins: the stage after
+// it clears it.
+__device__ __forceinline__ int *rec3_queue(Ctrl *c, int stage)
+{
+    return reinterpret_cast<int *>(c->aux23) + (stage - 1);
+}
+
 // one SSP-RK3 stage                             fv_rec3_2d.cu:166-353
 __global__ void __launch_bounds__(RNT, 2) rec3_stage_kernel(const __grid_constant__ GridDev gd, int stage, int ntiles)
 {
@@ -470,7 +480,7 @@ __global__ void __launch_bounds__(RNT, 2) rec3_stage_kernel(const __grid_constan
     double *FY = sm + ROFY;  // [4][RTY+1][RTX]
     __shared__ double s_red[RNT / 32];
     __shared__ __align__(8) uint64_t s_bar[3];
-    __shared__ int s_err, s_nlist;
+    __shared__ int s_err, s_nlist, s_next;
     __shared__ unsigned short s_list[RNF];  // faces that need the scaling
     const int tid = threadIdx.x, lane = tid & 31, n = gd.n;
     const double *u0 = (const double *)gd.st[0];
@@ -486,22 +496,20 @@ __global__ void __launch_bounds__(RNT, 2) rec3_stage_kernel(const __grid_constan
     int t = blockIdx.x, buf = 0;
     if (t < ntiles) pipe.start_box(gd, stage, t, sm, 0, tid);
     const TileCtl ctl = tile_control<P64>(gd.ctrl, stage, tid == 0 && t == 0);
+    // (the launch before is over, and the next one is two waits away)
+    int *queue = rec3_queue(gd.ctrl, stage);
+    if (tid == 0 && t == 0) *rec3_queue(gd.ctrl, stage == 1 ? 3 : stage - 1) = 0;
     pipe.finish_box(gd, 0, t < ntiles);
-    for (; t < ntiles; t += gridDim.x, buf ^= 1) {
+    if (t < ntiles && s_err) {
+        // the box never arrived: record it, stop
+        if (tid == 0) gd.ctrl->status = FVB_ERR_TIMEOUT;
+        t = ntiles;
+    }
+    if (!ctl.run) t = ntiles;
+    while (t < ntiles) {
         const int tx0 = (t % gd.tiles_x) * RTX, ty0 = (t / gd.tiles_x) * RTY;
-        const bool has_next = t + (int)gridDim.x < ntiles;
-        if (s_err) {
-            // a box never arrived: record it, stop
-            if (tid == 0) gd.ctrl->status = FVB_ERR_TIMEOUT;
-            break;
-        }
-        if (has_next) pipe.start_box(gd, stage, t + gridDim.x, sm + (buf ^ 1) * RPipe::BOX, buf ^ 1, tid);
-        const bool u0_tma = ctl.run && stage >= 2 && gd.tmap;
+        const bool u0_tma = stage >= 2 && gd.tmap;
         if (u0_tma) pipe.start_u0(gd, tx0, ty0, U0, tid);
-        if (!ctl.run) {
-            pipe.finish_box(gd, buf ^ 1, has_next);
-            continue;
-        }
         const double *Q = sm + buf * RPipe::BOX;  // [4][RSH][RSW] stage input
         if (tid == 0) s_nlist = 0;
         __syncthreads();
@@ -513,12 +521,18 @@ __global__ void __launch_bounds__(RNT, 2) rec3_stage_kernel(const __grid_constan
             if (ty0 + r < n && tx0 + c <= n && !r3_face<true, false>(Q, f, FX))
                 s_list[atomicAdd(&s_nlist, 1)] = (unsigned short)f;
         }
+        // the next tile, taken while the y-faces are computed
+        const int q = tid == 0 && ntiles > (int)gridDim.x ? (int)gridDim.x + atomicAdd(queue, 1) : ntiles;
         for (int f = tid; f < (RTY + 1) * RTX; f += RNT) {
             const int r = f / RTX, c = f - r * RTX;
             if (ty0 + r <= n && tx0 + c < n && !r3_face<false, false>(Q, f, FY))
                 s_list[atomicAdd(&s_nlist, 1)] = (unsigned short)(f + RTY * (RTX + 1));
         }
+        if (tid == 0) s_next = q;
         __syncthreads();
+        const int next = s_next;
+        const bool has_next = next < ntiles;
+        if (has_next) pipe.start_box(gd, stage, next, sm + (buf ^ 1) * RPipe::BOX, buf ^ 1, tid);
         // ---- the listed faces, one a thread, so that their bisections (25
         //      dependent steps a side) run side by side ---------------------------
         const int nl = s_nlist;
@@ -576,6 +590,12 @@ __global__ void __launch_bounds__(RNT, 2) rec3_stage_kernel(const __grid_constan
         }
         if (stage == 3 && tid == 0 && t == 0) leader_finish<P64>(gd.ctrl);
         pipe.finish_box(gd, buf ^ 1, has_next);
+        if (s_err) {
+            if (tid == 0) gd.ctrl->status = FVB_ERR_TIMEOUT;
+            break;
+        }
+        t = next;
+        buf ^= 1;
     }
     pipe.drain();
     if (brutal) atomicAdd(&gd.ctrl->aux, (unsigned long long)brutal);
