@@ -25,6 +25,20 @@ __device__ __forceinline__ void grid_dependency()
     asm volatile("fence.proxy.async;" ::: "memory");
 }
 
+// Tile counters of a single grid's stages (in Ctrl::aux23): a kernel whose
+// CTAs take their tiles as they come free counts the tiles taken beyond the
+// first of each CTA.  The counter of a stage is 0 when its launch begins: the
+// launch after it, whichever stage that is, clears it once its own wait on
+// the stream is over, and the next launch that counts on it waits for that one.
+__device__ __forceinline__ int *tile_queue(Ctrl *c, int stage)
+{
+    return reinterpret_cast<int *>(c->aux23) + (stage - 1);
+}
+__device__ __forceinline__ void clear_tile_queue(Ctrl *c, int stage)
+{
+    *tile_queue(c, stage == 1 ? 3 : stage - 1) = 0;
+}
+
 template <int PREC> struct PrecT;
 template <> struct PrecT<P64> { using R = double; using RR = double; };
 template <> struct PrecT<P32> { using R = float; using RR = double; };

@@ -33,7 +33,7 @@ struct Ctrl {
                                 // issues no first halo-box load (its wait must run out)
     unsigned long long aux;     // KEEP: bit pattern of the entropy-distance max of stage 1's
                                 // input; rec3: count of 2x2 blocks given the brutal mean fix
-    unsigned long long aux23[2];  // KEEP: the same of stages 2 and 3; rec3: the stages' tile counters
+    unsigned long long aux23[2];  // KEEP: the same of stages 2 and 3; else: tile counters of the stages (tile_queue)
 };
 
 // Device view of one grid.  Element (q, jp, ip) of a padded buffer, padded
@@ -135,6 +135,7 @@ struct StageKernel {
     void *fn, *fn_batched;
     size_t smem;
     int nt;
+    void *fn_queued = nullptr;  // single grids on tensor maps, tiles taken as CTAs come free
 };
 // the FP64 stage kernel of an order, a tile variant and a solver on the
 // reconstructed states (fvb_stage64.cuh); fn null: not built

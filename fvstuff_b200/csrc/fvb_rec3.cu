@@ -460,17 +460,11 @@ __device__ __forceinline__ bool r3_face(const double *Q, int f, double *FP)
     return true;
 }
 
-// Tiles of a stage are handed out as CTAs come free: the shock's tiles, with
-// bisected faces and limited blocks, cost several times the others, and with
-// a fixed share of the tiles a CTA the SMs were busy 79 % of a stage (1024^2
-// circular Sod: a stage 105 us, now 94).  The counter of `stage`, zero when it begins: the stage after
-// it clears it.
-__device__ __forceinline__ int *rec3_queue(Ctrl *c, int stage)
-{
-    return reinterpret_cast<int *>(c->aux23) + (stage - 1);
-}
-
-// one SSP-RK3 stage                             fv_rec3_2d.cu:166-353
+// One SSP-RK3 stage                             fv_rec3_2d.cu:166-353
+// The shock's tiles, with bisected faces and limited blocks, cost several
+// times the others: with a fixed share of the tiles a CTA the SMs were busy
+// 79 % of a stage (1024^2 circular Sod: a stage 105 us, now 94), so a CTA takes
+// its next tile when it comes to it (tile_queue, fvb_device.cuh).
 __global__ void __launch_bounds__(RNT, 2) rec3_stage_kernel(const __grid_constant__ GridDev gd, int stage, int ntiles)
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -496,9 +490,8 @@ __global__ void __launch_bounds__(RNT, 2) rec3_stage_kernel(const __grid_constan
     int t = blockIdx.x, buf = 0;
     if (t < ntiles) pipe.start_box(gd, stage, t, sm, 0, tid);
     const TileCtl ctl = tile_control<P64>(gd.ctrl, stage, tid == 0 && t == 0);
-    // (the launch before is over, and the next one is two waits away)
-    int *queue = rec3_queue(gd.ctrl, stage);
-    if (tid == 0 && t == 0) *rec3_queue(gd.ctrl, stage == 1 ? 3 : stage - 1) = 0;
+    int *queue = tile_queue(gd.ctrl, stage);
+    if (tid == 0 && t == 0) clear_tile_queue(gd.ctrl, stage);
     pipe.finish_box(gd, 0, t < ntiles);
     if (t < ntiles && s_err) {
         // the box never arrived: record it, stop

@@ -412,11 +412,15 @@ cudaError_t launch_facts(const void *fn, int threads, size_t smem, LaunchFacts &
     return cudaSuccess;
 }
 
-// resident CTAs per SM of a kernel: the fewer of its two forms
+// resident CTAs per SM of a kernel: the fewest of its forms
 static cudaError_t prepare(const StageKernel &e, int &max_ctas)
 {
     LaunchFacts a{}, b{};
     cudaError_t err = launch_facts(e.fn, e.nt, e.smem, a);
+    if (err == cudaSuccess && e.fn_queued) {
+        err = launch_facts(e.fn_queued, e.nt, e.smem, b);
+        a.ctas_per_sm = std::min(a.ctas_per_sm, b.ctas_per_sm);
+    }
     if (err == cudaSuccess) err = e.fn_batched ? launch_facts(e.fn_batched, e.nt, e.smem, b) : cudaSuccess;
     if (err != cudaSuccess) return err;
     max_ctas = e.fn_batched ? std::min(a.ctas_per_sm, b.ctas_per_sm) : a.ctas_per_sm;
@@ -520,7 +524,11 @@ int stage_max_ctas_per_sm(int prec, int order, int shape, int rs)
 cudaError_t launch_stage(int prec, int order, int shape, const StageArgs &a, int grid_ctas, cudaStream_t s, int rs)
 {
     const StageKernel e = kernel_for(prec, order, shape, rs);
-    void *fn = a.grids ? e.fn_batched : e.fn;
+    // a queue of tiles from two whole waves up: below, the later box costs more
+    // than the balance gives (FP64, us a stage, fixed / queued: 400^2 12.9 / 13.8,
+    // 512^2 17.3 / 18.0; 560^2 19.8 / 18.3, 700^2 26.8 / 23.9)
+    const bool queued = e.fn_queued && !a.grids && a.grid.tmap && a.stage > 0 && a.ntiles_static > 2 * grid_ctas;
+    void *fn = a.grids ? e.fn_batched : queued ? e.fn_queued : e.fn;
     if (!fn) return cudaErrorInvalidValue;
     int max_ctas = 0;
     cudaError_t err = prepare(e, max_ctas);

@@ -64,9 +64,19 @@ struct L64 {
     static constexpr int MINB = fit < regs ? fit : regs;
 };
 
-template <int ORDER, int TX, int TY, int NT, bool BATCHED, int RS>
+// How a launch's tiles reach its CTAs.  FIXED: each CTA a fixed share, in turn,
+// the next box loaded from the top of a tile.  QUEUED (single grids on tensor
+// maps): a CTA takes its next tile (tile_queue) when it comes to its
+// y-faces, so that none is left with a whole tile while others are done; the
+// box has the y-faces and the update to arrive.  us a stage, fixed / queued:
+// 2048^2 179 / 164, 1024^2 50.5 / 47.2, 777^2 33.0 / 28.9.  BATCHED: a fixed
+// share of a tile table.
+enum { M64_FIXED, M64_BATCHED, M64_QUEUED };
+
+template <int ORDER, int TX, int TY, int NT, int MODE, int RS>
 __global__ void __launch_bounds__(NT, (L64<ORDER, TX, TY, NT>::MINB)) stage64_kernel(const __grid_constant__ StageArgs a)
 {
+    constexpr bool BATCHED = MODE == M64_BATCHED, QUEUED = MODE == M64_QUEUED;
     using P = L64<ORDER, TX, TY, NT>;
     constexpr bool SPLIT = P::SPLIT;
     constexpr int G = P::G, NK = P::NK, XO = P::XO, SW = P::SW, SH = P::SH, PL = P::PL;
@@ -79,7 +89,7 @@ __global__ void __launch_bounds__(NT, (L64<ORDER, TX, TY, NT>::MINB)) stage64_ke
     double *U0 = sm + P::oU0;  // [4][TY][TX]
     __shared__ double s_red[NW];
     __shared__ __align__(8) uint64_t s_bar[3];  // two boxes, U0
-    __shared__ int s_err;
+    __shared__ int s_err, s_next;
     __shared__ __align__(16) TileHdr s_hdr[2];
     __shared__ TileRef s_ref_next;  // batched: table entry of the CTA's next tile
 
@@ -148,10 +158,13 @@ __global__ void __launch_bounds__(NT, (L64<ORDER, TX, TY, NT>::MINB)) stage64_ke
     double lacc = 0.0;
     TileCtl ctl1{};
     if (!BATCHED && t < ntiles) ctl1 = tile_control<P64>(a.grid.ctrl, a.stage, tid == 0 && t == 0);
-    for (; t < ntiles; t += stride, buf ^= 1) {
+    if (QUEUED && tid == 0 && t == 0) clear_tile_queue(a.grid.ctrl, a.stage);
+    if (QUEUED && !ctl1.run && !s_err) t = ntiles;
+    for (int next; t < ntiles; t = next, buf ^= 1) {
+        next = t + stride;
         // warp 0 of a batched launch: the next tile's descriptor word and the
         // entry of the tile after it, in flight while c and E are formed
-        const bool has_next = t + stride < ntiles;
+        bool has_next = next < ntiles;
         unsigned long long wnext = 0ull;
         TileRef ref_next{}, ref_after{};
         if (BATCHED && tid < 32) {
@@ -175,7 +188,7 @@ __global__ void __launch_bounds__(NT, (L64<ORDER, TX, TY, NT>::MINB)) stage64_ke
         // ---- 1. start the next tile's box (its buffer was last read before
         //         the barrier that ended the previous tile) and this tile's U0 --
         bool next_tma = false;
-        if (!BATCHED && has_next) next_tma = start_single(t + stride, buf ^ 1);
+        if (!BATCHED && !QUEUED && has_next) next_tma = start_single(next, buf ^ 1);
         const bool u0_tma = P::U0S && ctl.run && a.stage >= 2 && gd.tmap;
         if (u0_tma && tid == 0) {
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -210,6 +223,14 @@ __global__ void __launch_bounds__(NT, (L64<ORDER, TX, TY, NT>::MINB)) stage64_ke
             continue;
         }
 
+        int taken = ntiles;
+        if (QUEUED && tid == 0) taken = stride + atomicAdd(tile_queue(a.grid.ctrl, a.stage), 1);
+        // the box of the tile taken: its buffer was last read before the barrier that ended the previous tile
+        auto start_taken = [&] {
+            if (!QUEUED || tid != 0) return;
+            s_next = taken;
+            if (taken < ntiles) start_single(taken, buf ^ 1);
+        };
         double F0[4], F1[4];  // this thread's y-pair
         if constexpr (SPLIT) {
             // ---- 3s. one face a thread: x-faces in the lower half of the
@@ -270,6 +291,7 @@ __global__ void __launch_bounds__(NT, (L64<ORDER, TX, TY, NT>::MINB)) stage64_ke
 #pragma unroll
                 for (int q = 0; q < 4; ++q) o[q * (TY * FW / 2)] = make_double2(FA[q], FB[q]);
             }
+            start_taken();
             // ---- 4. y-faces 2k, 2k + 1 of column c (normal velocity v) ------------
             {
                 const int k = tid / TX, c = tid - k * TX;
@@ -300,6 +322,10 @@ __global__ void __launch_bounds__(NT, (L64<ORDER, TX, TY, NT>::MINB)) stage64_ke
             }
         }
         __syncthreads();
+        if (QUEUED) {
+            next = s_next;
+            has_next = next_tma = next < ntiles;
+        }
 
         if (!has_next) grid_release();
         // ---- 5. divergence, RK combination, stores: cells 2k and 2k + 1 of
@@ -401,9 +427,13 @@ static StageKernel entry64()
 {
     constexpr TileShape ts = kTileShapes64[SHAPE];
     void *batched = nullptr;
-    if constexpr (ORDER == 7 && RS == 0) batched = (void *)stage64_kernel<ORDER, ts.tx, ts.ty, ts.nt, true, RS>;
-    return StageKernel{(void *)stage64_kernel<ORDER, ts.tx, ts.ty, ts.nt, false, RS>, batched, L64<ORDER, ts.tx, ts.ty, ts.nt>::smem,
-                       ts.nt};
+    if constexpr (ORDER == 7 && RS == 0) batched = (void *)stage64_kernel<ORDER, ts.tx, ts.ty, ts.nt, M64_BATCHED, RS>;
+    // (the split form is for grids of few tiles: no queue)
+    void *queued = nullptr;
+    if constexpr (!L64<ORDER, ts.tx, ts.ty, ts.nt>::SPLIT)
+        queued = (void *)stage64_kernel<ORDER, ts.tx, ts.ty, ts.nt, M64_QUEUED, RS>;
+    return StageKernel{(void *)stage64_kernel<ORDER, ts.tx, ts.ty, ts.nt, M64_FIXED, RS>, batched,
+                       L64<ORDER, ts.tx, ts.ty, ts.nt>::smem, ts.nt, queued};
 }
 
 template <int ORDER, int RS>
