@@ -510,7 +510,16 @@ struct RowPair {
     static constexpr int MINB = fit < regs ? fit : regs;  // resident CTAs an SM, at 128 registers a thread
 };
 
-template <int TX, int TY, bool BATCHED>
+// How a launch's tiles reach its CTAs (as the FP64 kernel's M64_ modes): a fixed
+// share each, a table's, or, on single grids of more than two waves, taken
+// from the stage's counter (tile_queue) between the x- and the y-faces.
+// us a stage, fixed / queued: 1800^2 92.7 / 89.6, 2048^2 116 / 111, 4096^2
+// 448 / 406; 1024^2 (3.8 waves) 34.3 / 34.5.  (The x/y pair kernel above, for
+// smaller grids, has one face loop, so the box would start with nothing but the
+// update left: taken with the conversion, -4 ... +2 %, so it has no such mode.)
+enum { M32P_FIXED, M32P_BATCHED, M32P_QUEUED };
+
+template <int TX, int TY, int MODE>
 __global__ void __launch_bounds__((RowPair<TX, TY>::NT), (RowPair<TX, TY>::MINB))
     stage32p_kernel(const __grid_constant__ StageArgs a)
 {
@@ -533,12 +542,12 @@ __global__ void __launch_bounds__((RowPair<TX, TY>::NT), (RowPair<TX, TY>::MINB)
     float2 *FY2 = sm2 + RP::oFY;             // [4][NK][TX]
     __shared__ double s_red[NW];
     __shared__ __align__(8) uint64_t s_bar;
-    __shared__ int s_err;
+    __shared__ int s_err, s_next;
     __shared__ __align__(16) TileHdr s_hdr[2];
     __shared__ TileRef s_ref_next;
 
     const int tid = threadIdx.x;
-    constexpr bool batched = BATCHED;
+    constexpr bool batched = MODE == M32P_BATCHED, QUEUED = MODE == M32P_QUEUED;
     const int cur = a.parity, nxt = a.parity ^ 1;
     if (tid == 0) {
         mbar_init(&s_bar, 1);
@@ -596,8 +605,10 @@ __global__ void __launch_bounds__((RowPair<TX, TY>::NT), (RowPair<TX, TY>::MINB)
     double lacc = 0.0;
     TileCtl ctl1{};
     if (!batched && t < ntiles) ctl1 = tile_control<P32C>(a.grid.ctrl, a.stage, tid == 0 && t == 0);
-    for (; t < ntiles; t += stride, slot ^= 1) {
-        const bool has_next = t + stride < ntiles;
+    if (QUEUED && tid == 0 && t == 0) clear_tile_queue(a.grid.ctrl, a.stage);
+    for (int next; t < ntiles; t = next, slot ^= 1) {
+        next = t + stride;
+        bool has_next = next < ntiles;
         unsigned long long wnext = 0ull;
         TileRef ref_next{}, ref_after{};
         if (batched && tid < 32) {
@@ -607,7 +618,7 @@ __global__ void __launch_bounds__((RowPair<TX, TY>::NT), (RowPair<TX, TY>::MINB)
             }
             if (t + 2 * stride < ntiles) ref_after = a.tiles[t + 2 * stride];
         }
-        const GridDev &gd = tile_grid<BATCHED>(s_hdr[slot], a);
+        const GridDev &gd = tile_grid<batched>(s_hdr[slot], a);
         const int tile = batched ? s_hdr[slot].tile : t;
         const TileCtl ctl = batched ? s_hdr[slot].ctl : ctl1;
         const int n = gd.n;
@@ -667,8 +678,8 @@ __global__ void __launch_bounds__((RowPair<TX, TY>::NT), (RowPair<TX, TY>::MINB)
                     if (tid == 0) s_ref_next = ref_after;
                 }
                 next_tma = true;
-            } else {
-                next_tma = start_single(t + stride);
+            } else if (!QUEUED || !ctl.run) {
+                next_tma = start_single(next);
             }
         }
         if (!ctl.run) {
@@ -700,6 +711,8 @@ __global__ void __launch_bounds__((RowPair<TX, TY>::NT), (RowPair<TX, TY>::MINB)
                 }
             }
         }
+        int taken = ntiles;
+        if (QUEUED && tid == 0) taken = stride + atomicAdd(tile_queue(a.grid.ctrl, a.stage), 1);
         // ---- 3. x-faces 2j, 2j + 1 of pair row r -------------------------------
         for (int p = tid; p < XP * rows; p += NT) {
             const int r = p / XP, j = p - r * XP;
@@ -729,6 +742,10 @@ __global__ void __launch_bounds__((RowPair<TX, TY>::NT), (RowPair<TX, TY>::MINB)
             float4 *o = reinterpret_cast<float4 *>(FX2 + r * FW + 2 * j);
 #pragma unroll
             for (int q = 0; q < 4; ++q) o[q * (HT * FW / 2)] = make_float4(FA[q].x, FA[q].y, FB[q].x, FB[q].y);
+        }
+        if (QUEUED && tid == 0) {
+            s_next = taken;
+            if (taken < ntiles) start_single(taken);
         }
         // ---- 4. y-faces 2k, 2k + 1 of column c (normal velocity v) ------------
         const int k = tid / TX, c = tid - k * TX, i = tx0 + c;
@@ -772,6 +789,10 @@ __global__ void __launch_bounds__((RowPair<TX, TY>::NT), (RowPair<TX, TY>::MINB)
         };
         load_ops(0);
         __syncthreads();
+        if (QUEUED) {
+            next = s_next;
+            has_next = next_tma = next < ntiles;
+        }
 
         if (!has_next) grid_release();
         // ---- 5. divergence as pairs, then each cell's RK update ---------------
@@ -829,8 +850,9 @@ static StageKernel entry32c()
     constexpr TileShape ts = kTileShapes32c[SHAPE];
     if constexpr (row_pairs(ts)) {
         static_assert(ts.nt == RowPair<ts.tx, ts.ty>::NT, "one y-face pair a thread");
-        return StageKernel{(void *)stage32p_kernel<ts.tx, ts.ty, false>, (void *)stage32p_kernel<ts.tx, ts.ty, true>,
-                           RowPair<ts.tx, ts.ty>::smem, ts.nt};
+        return StageKernel{(void *)stage32p_kernel<ts.tx, ts.ty, M32P_FIXED>,
+                           (void *)stage32p_kernel<ts.tx, ts.ty, M32P_BATCHED>, RowPair<ts.tx, ts.ty>::smem, ts.nt,
+                           (void *)stage32p_kernel<ts.tx, ts.ty, M32P_QUEUED>};
     } else {
         constexpr int sw = ts.tx + 8, sh = ts.ty + 8;
         constexpr size_t smem = sizeof(float) * ((size_t)14 * sw * sh + 4 * ts.ty * (ts.tx + 1) + 4 * (ts.ty + 1) * ts.tx);
