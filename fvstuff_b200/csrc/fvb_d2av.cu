@@ -24,7 +24,8 @@
 // roots were most of it: 60 divisions a cell, 4970 instructions and 1530 FP64
 // ones, 235 us a stage.  Rounding the same quotients from shared reciprocals
 // (fvb_ieee.cuh: one reciprocal of a density for the three quotients by it,
-// none for the constant denominators and h) takes a stage to 105 us.
+// none for the constant denominators and h) took a stage to 105 us; step
+// control once a CTA, chained launches and tiles taken as CTAs come free to 87.
 #include <algorithm>
 
 #include "fvb_aux.h"

@@ -12,8 +12,8 @@
 //
 // One launch per stage does all of it for a tile of 32 x 14 cells: tiles
 // start on even cells, so every 2x2 block lies in one tile.  Two halo boxes
-// alternate (TMA, the next one in flight for a whole tile) and U0 arrives
-// during the faces; after the face fluxes a warp takes 2 rows of 16 cells, a
+// alternate (TMA, the next one in flight from the end of a tile's faces) and U0
+// arrives during the faces; after the face fluxes a warp takes 2 rows of 16 cells, a
 // block being four of its lanes, so that residual, RK combination, limiter and
 // stores (interior + periodic ghost images) need no barrier between; stage 3
 // max-reduces the wave speed of the limited state.
@@ -35,7 +35,8 @@
 // limiter's bisection likewise takes a block's four corners side by side.
 // us a stage at 1024^2, mean over ten steps of the Sod (a smooth state): 225
 // (242) as it was, 116 (97) with shared reciprocals, the list and plain loads
-// into 32 x 32 tiles, 105 (77) with the pipeline above.
+// into 32 x 32 tiles, 105 (77) with the pipeline above, 94 with tiles taken as
+// CTAs come free.
 #include <algorithm>
 
 #include "fvb_aux.h"

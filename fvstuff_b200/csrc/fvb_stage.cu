@@ -1,7 +1,6 @@
-// fvb_stage.cu -- the fused SSP-RK3 stage kernel of the FP64 plain method
-// (and of the FP32 form as shipped), the step-control kernel of batched
-// launches, the tile-variant tables and the TMA descriptors.  The FP32-
-// compensated form has its own kernel (fvb_stage32c.cu).
+// fvb_stage.cu -- the fused SSP-RK3 stage kernel of the FP32 form as shipped,
+// the choice and the launch of every form's stage kernel (FP64:
+// fvb_stage64.cuh, FP32-compensated: fvb_stage32c.cu) and the TMA descriptors.
 //
 // One launch = one RK stage of one grid (or of every grid of a batch, through
 // a tile table).  Per tile of TX x TY interior cells a CTA
