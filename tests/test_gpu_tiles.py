@@ -133,3 +133,24 @@ def test_d2av_tile_edges_and_taken_tiles(n, order, steps):
     ref = U.copy()
     O.d2av_run(ref, n, 1.0 / n, 0.4, 0, steps, 1e30, order, 0.5, 0.0, 0.05)
     assert rel_linf(s.get_state(layout="cons", interior=True), ref[:, g:-g, g:-g]) <= 1e-13
+
+
+@pytest.mark.parametrize("precision,n", [("f64", 601), ("f32c", 781)])
+def test_taken_tiles_after_a_lost_load(precision, n):
+    """A stage that stops early (its first load is not issued, so the bounded
+    wait runs out) leaves tiles untaken; the stages after it clear its counter,
+    so the solver given a new state advances as a fresh one."""
+    w = smooth(n, seed=n)
+    out = []
+    for lost in (True, False):
+        s = F.Solver(n, precision=precision, bc="periodic", tile=0)
+        s.set_state(w, interior=True)
+        if lost:
+            s.debug_drop_load()
+            s.step(1)
+            assert s.sync().status != 0
+            s.set_state(w, interior=True)
+        s.step(3)
+        assert s.sync().steps == 3
+        out.append(s.get_state())
+    assert np.array_equal(out[0], out[1])
