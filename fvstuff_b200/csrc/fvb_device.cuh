@@ -10,8 +10,10 @@ namespace fvb {
 // Programmatic dependent launch.  A kernel of the step loops is launched with
 // launch_chained (fvb_internal.h), so its CTAs may become resident while the
 // kernel before it in the stream still runs; grid_dependency() is its first
-// statement that touches global memory: it waits until the kernel before has
-// finished and its writes are visible (also to the TMA loads that follow).
+// statement that touches global memory that a kernel writes: it waits until
+// the kernel before has finished and its writes are visible (also to the TMA
+// loads that follow).  (Batched launches read their tile table and grid
+// descriptors ahead of it: only stream-ordered copies write those.)
 // grid_release() lets the next kernel's CTAs come in the same way; a CTA
 // calls it before the update of its last tile, so that they take the places
 // of CTAs that are about to end and not those beside the ones that are not.

@@ -1,6 +1,6 @@
 // fvb_stage32c.cu -- the SSP-RK3 stage kernel of the FP32-compensated form.
 //
-// Same tile pipeline as the FP64 kernel (fvb_stage.cu): persistent CTAs walk
+// Same tile pipeline as the FP64 kernel (fvb_stage64.cuh): persistent CTAs walk
 // the tiles of one grid or of a batch's tile table; the halo box of the next
 // tile streams in through TMA while the current one is computed; every face
 // is evaluated once; the RK combination stores the interior and its ghost
