@@ -605,6 +605,8 @@ __global__ void ctrl_set_kernel(Ctrl *c, double t_stop, int reset, double t0, do
         c->clamped = 0;
         c->cfl = cfl;
         c->h = h;
+        // (between steps the tile counters, or KEEP's sensor words, hold nothing)
+        c->aux23[0] = c->aux23[1] = 0;
     }
     c->t_stop = t_stop;
 }

@@ -64,7 +64,9 @@ float time_shape(int prec, int order, int n, int shape, cudaStream_t s)
         const int internal = prec_internal(prec == P64 ? FVB_PREC_F64 : prec == P32 ? FVB_PREC_F32 : FVB_PREC_F32C);
         ExtView ev{1, g, n + 2 * g, FVB_LAYOUT_PRIM, FVB_F64};
         BufView v = view_of(gd);
-        if (cudaMemsetAsync(block, 0, G.bytes, s) != cudaSuccess) break;
+        // (the step control too: its tile counters and its lost-load flag are
+        // read by the first launches and set by nothing before them)
+        if (cudaMemsetAsync(block, 0, ctrl_off + sizeof(Ctrl), s) != cudaSuccess) break;
         if (init_case_prim64((double *)stage, n, 0.0, 0.0, gd.h, 1.4, c, s) != cudaSuccess) break;
         if (import_state(stage, ev, gd.st[0], gd.lo[0], v, internal, 1.4, s) != cudaSuccess) break;
         cudaError_t e = internal == INT_PRIM64 ? bc_fill<double>((double *)gd.st[0], v, 1, 1, s)
