@@ -184,14 +184,16 @@ __device__ __forceinline__ void hllc(const double L[4], const double R[4], const
     const double pK = left ? pL : pR, SK = left ? SL : SR;
     const double EK = energy(rK, uK, tK, pK, gs);
     // star state; in a supersonic fan S = u_K with SK - u_K and SK - S taken
-    // as 1, which gives K's own state exactly (those differences could be 0
-    // beside a floored sound speed)
+    // as 1, which gives K's own state (those differences could be 0 beside a
+    // floored sound speed).  S - u_K is then an exact 0, so p* and E* are p_K and
+    // E_K to the bit: E* formed with p* S - p_K u_K would put a term of other
+    // units beside E_K there, and lose its digits as velocities grow
     const double S = sup ? uK : Ss;
     const double w = sup ? 1. : SK - uK;
     const double q = frcp(sup ? 1. : SK - Ss);
-    const double dK = rK * w;
-    const double ps = fma(dK, S - uK, pK);
-    const double Es = fma(-pK, uK, fma(ps, S, EK * w)) * q;
+    const double dK = rK * w, du = S - uK;
+    const double ps = fma(dK, du, pK);
+    const double Es = fma(du, fma(dK, S, pK), EK * w) * q;
     F[0] = dK * q * S;
     F[1] = fma(F[0], S, ps);
     F[2] = F[0] * tK;
