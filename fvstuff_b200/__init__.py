@@ -185,6 +185,11 @@ class Solver:
         FVB_ERR_TIMEOUT (see fvb_debug_drop_load)."""
         check(lib().fvb_debug_drop_load(self._h), "fvb_debug_drop_load")
 
+    def debug_drop(self, load: str) -> None:
+        """The same for the load named: 'box', or 'u0' in the FP64 forms that
+        load U0 by its own copy (see fvb_debug_drop)."""
+        check(lib().fvb_debug_drop(self._h, L.DROP[load]), "fvb_debug_drop")
+
     def limiter_fixes(self) -> int:
         """rec3 family: blocks whose mean needed the floor fix since the
         state was set (see fvb_limiter_fixes); 0 for the other families."""

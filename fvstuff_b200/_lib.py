@@ -66,6 +66,7 @@ class ServeConfig(C.Structure):
                 ("max_seconds", C.c_double)]
 
 
+DROP = {"box": 1, "u0": 2}
 SERVE_POLICY = {"fifo": 0, "shortest": 1}
 
 
@@ -85,6 +86,7 @@ _SIG = {
     "fvb_get_state_hilo": (C.c_int, [_P, _P, _P]),
     "fvb_frame_begin": (C.c_int, [_P]),
     "fvb_debug_drop_load": (C.c_int, [_P]),
+    "fvb_debug_drop": (C.c_int, [_P, C.c_int]),
     "fvb_set_d2av": (C.c_int, [_P, C.c_double, C.c_double, C.c_double]),
     "fvb_limiter_fixes": (C.c_int, [_P, C.POINTER(C.c_int64)]),
     "fvb_frame_end": (C.c_int, [_P, _P]),

@@ -592,8 +592,16 @@ fvb_status fvb_debug_drop_load(fvb_solver *s)
     if (!s) return fail(FVB_ERR_INVALID, "null argument");
     if (s->keep || s->rec3 || s->d2av || !s->gd.tmap)
         return fail(FVB_ERR_INVALID, "the hook needs a TMA-fed UP grid");
-    static const int one = 1;
-    cudaError_t e = cudaMemcpyAsync(&s->ctrl->drop_load, &one, sizeof one, cudaMemcpyHostToDevice, s->stream);
+    return fvb_debug_drop(s, FVB_DROP_BOX);
+}
+
+fvb_status fvb_debug_drop(fvb_solver *s, int load)
+{
+    if (!s || (load != FVB_DROP_BOX && load != FVB_DROP_U0)) return fail(FVB_ERR_INVALID, "null solver or bad load %d", load);
+    if (s->keep || s->d2av || !s->gd.tmap) return fail(FVB_ERR_INVALID, "the hook needs a TMA-fed grid");
+    if (load == FVB_DROP_U0 && !s->rec3 && (s->prec != P64 || s->order == 9))
+        return fail(FVB_ERR_INVALID, "no U0 load in this form");
+    cudaError_t e = cudaMemcpyAsync(&s->ctrl->drop_load, &load, sizeof load, cudaMemcpyHostToDevice, s->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
     return e == cudaSuccess ? FVB_OK : cuda_fail(e, "arm");
 }

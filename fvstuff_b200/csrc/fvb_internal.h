@@ -29,8 +29,9 @@ struct Ctrl {
     int active;                 // the step in progress runs
     int status;                 // fvb_status of the step control
     int clamped;                // dt was clamped to land on t_stop
-    int drop_load;              // failure-injection hook: the next single-grid stage launch
-                                // issues no first halo-box load (its wait must run out)
+    int drop_load;              // failure-injection hook (fvb_debug_drop): CTA 0 of the next
+                                // single-grid stage that makes that load does not issue it
+                                // (its wait must run out)
     unsigned long long aux;     // KEEP: bit pattern of the entropy-distance max of stage 1's
                                 // input; rec3: count of 2x2 blocks given the brutal mean fix
     unsigned long long aux23[2];  // KEEP: the same of stages 2 and 3; else: tile counters of the stages (tile_queue)

@@ -489,11 +489,15 @@ __global__ void __launch_bounds__(RNT, 2) rec3_stage_kernel(const __grid_constan
     RPipe pipe(s_bar, &s_err, tid);
     grid_dependency();
     int t = blockIdx.x, buf = 0;
-    if (t < ntiles) pipe.start_box(gd, stage, t, sm, 0, tid);
+    // failure injection (fvb_debug_drop): CTA 0 issues no first box load, or no U0 load for its first tile
+    const int armed = blockIdx.x == 0 && gd.tmap ? *(volatile int *)&gd.ctrl->drop_load : 0;
+    const bool drop = armed == FVB_DROP_BOX, drop_u0 = armed == FVB_DROP_U0 && stage >= 2;
+    if (t < ntiles && !drop) pipe.start_box(gd, stage, t, sm, 0, tid);
     const TileCtl ctl = tile_control<P64>(gd.ctrl, stage, tid == 0 && t == 0);
     int *queue = tile_queue(gd.ctrl, stage);
     if (tid == 0 && t == 0) clear_tile_queue(gd.ctrl, stage);
     pipe.finish_box(gd, 0, t < ntiles);
+    if ((drop || drop_u0) && tid == 0) gd.ctrl->drop_load = 0;
     if (t < ntiles && s_err) {
         // the box never arrived: record it, stop
         if (tid == 0) gd.ctrl->status = FVB_ERR_TIMEOUT;
@@ -503,7 +507,7 @@ __global__ void __launch_bounds__(RNT, 2) rec3_stage_kernel(const __grid_constan
     while (t < ntiles) {
         const int tx0 = (t % gd.tiles_x) * RTX, ty0 = (t / gd.tiles_x) * RTY;
         const bool u0_tma = stage >= 2 && gd.tmap;
-        if (u0_tma) pipe.start_u0(gd, tx0, ty0, U0, tid);
+        if (u0_tma && !drop_u0) pipe.start_u0(gd, tx0, ty0, U0, tid);
         const double *Q = sm + buf * RPipe::BOX;  // [4][RSH][RSW] stage input
         if (tid == 0) s_nlist = 0;
         __syncthreads();
@@ -591,7 +595,7 @@ __global__ void __launch_bounds__(RNT, 2) rec3_stage_kernel(const __grid_constan
         t = next;
         buf ^= 1;
     }
-    pipe.drain();
+    if (!drop && !drop_u0) pipe.drain();
     if (brutal) atomicAdd(&gd.ctrl->aux, (unsigned long long)brutal);
     if (stage == 3) {
         for (int o = 16; o > 0; o >>= 1) lacc = fmax(lacc, __shfl_xor_sync(0xffffffffu, lacc, o));

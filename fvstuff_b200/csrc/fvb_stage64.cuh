@@ -129,12 +129,14 @@ __global__ void __launch_bounds__(NT, (L64<ORDER, TX, TY, NT>::MINB)) stage64_ke
         issue_tile_load64<G, TX, TY, SW, XO, NT>(a.grid, a.stage, t, sm + m * P::BOX, &s_bar[m], tid);
         return a.grid.tmap != nullptr;
     };
-    // failure injection (fvb_debug_drop_load): CTA 0 of a single-grid launch
-    // issues no first box load, so its bounded wait runs out and the grid's
-    // status becomes FVB_ERR_TIMEOUT; the flag is read by every thread of
-    // that CTA before thread 0 clears it behind the first barrier
-    const bool drop = !BATCHED && blockIdx.x == 0 && a.stage > 0 && a.grid.ctrl && a.grid.tmap &&
-                      *(volatile int *)&a.grid.ctrl->drop_load;
+    // failure injection (fvb_debug_drop): CTA 0 of a single-grid launch
+    // issues no first box load, or no U0 load for its first tile, so its bounded
+    // wait runs out and the grid's status becomes FVB_ERR_TIMEOUT; the flag is
+    // read by every thread of that CTA before thread 0 clears it behind the
+    // first barrier
+    const int armed = !BATCHED && blockIdx.x == 0 && a.stage > 0 && a.grid.ctrl && a.grid.tmap
+                          ? *(volatile int *)&a.grid.ctrl->drop_load : 0;
+    const bool drop = armed == FVB_DROP_BOX, drop_u0 = armed == FVB_DROP_U0 && a.stage >= 2;
     const int stride = gridDim.x;
     int t = blockIdx.x, buf = 0;
     if (t < ntiles && BATCHED) {
@@ -155,6 +157,7 @@ __global__ void __launch_bounds__(NT, (L64<ORDER, TX, TY, NT>::MINB)) stage64_ke
     // single grid: the stage-3 wave-speed max is reduced once per CTA, and the
     // step control, the same for every tile, is read once (the leader is CTA
     // 0, whose first tile is tile 0)
+    if (drop_u0 && tid == 0) a.grid.ctrl->drop_load = 0;
     double lacc = 0.0;
     TileCtl ctl1{};
     if (!BATCHED && t < ntiles) ctl1 = tile_control<P64>(a.grid.ctrl, a.stage, tid == 0 && t == 0);
@@ -181,8 +184,14 @@ __global__ void __launch_bounds__(NT, (L64<ORDER, TX, TY, NT>::MINB)) stage64_ke
         const int tx0 = (tile % gd.tiles_x) * TX, ty0 = (tile / gd.tiles_x) * TY;
         const f64::Gas gf{gd.gam, gd.igm1, gd.gam - 1.0};
         if (s_err) {
-            // a load never arrived: record it, stop
-            if (tid == 0 && gd.ctrl) gd.ctrl->status = FVB_ERR_TIMEOUT;
+            // a load never arrived: no tile of this CTA from here on is computed;
+            // record it for their grids, stop
+            if constexpr (BATCHED) {
+                for (int k = t + tid * stride; k < ntiles; k += NT * stride)
+                    a.ctrls[a.tiles[k].grid].status = FVB_ERR_TIMEOUT;
+            } else if (tid == 0 && gd.ctrl) {
+                gd.ctrl->status = FVB_ERR_TIMEOUT;
+            }
             break;
         }
         // ---- 1. start the next tile's box (its buffer was last read before
@@ -192,8 +201,10 @@ __global__ void __launch_bounds__(NT, (L64<ORDER, TX, TY, NT>::MINB)) stage64_ke
         const bool u0_tma = P::U0S && ctl.run && a.stage >= 2 && gd.tmap;
         if (u0_tma && tid == 0) {
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            mbar_expect_tx(&s_bar[2], 4u * TY * TX * sizeof(double));
-            tma_load3(U0, gd.tmap + TM_U0, gd.xoff + G + tx0, G + ty0, 0, &s_bar[2]);
+            if (!drop_u0) {
+                mbar_expect_tx(&s_bar[2], 4u * TY * TX * sizeof(double));
+                tma_load3(U0, gd.tmap + TM_U0, gd.xoff + G + tx0, G + ty0, 0, &s_bar[2]);
+            }
         }
         // ---- 2. sound speed and energy of the cells the HLLE reads ----------
         const double *IN = sm + buf * P::BOX;
@@ -332,7 +343,9 @@ __global__ void __launch_bounds__(NT, (L64<ORDER, TX, TY, NT>::MINB)) stage64_ke
         //      column c (split: one cell) -----------------------------------
         double lmax = 0.0;
         const double inv_h = gd.inv_h, dth = ctl.dt * inv_h;
+        // (a lost U0 is recorded here: there may be no next tile)
         const bool u0_ok = !u0_tma || wait_bar(2);
+        if (!u0_ok && gd.ctrl) gd.ctrl->status = FVB_ERR_TIMEOUT;
         const int k = tid / TX, c = tid - k * TX, i = tx0 + c;
 #pragma unroll
         for (int h = 0; h < (SPLIT ? 1 : 2); ++h) {
@@ -417,7 +430,7 @@ __global__ void __launch_bounds__(NT, (L64<ORDER, TX, TY, NT>::MINB)) stage64_ke
     }
     // a load whose wait gave up may still be in flight: wait once more
     // (bounded) so no copy into this CTA's shared memory outlives it
-    if (lost && !drop)
+    if (lost && !drop && !drop_u0)
         for (int m = 0; m < 3; ++m)
             if ((lost >> m) & 1u) mbar_wait(&s_bar[m], (phase >> m) & 1u);
 }

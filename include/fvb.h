@@ -230,6 +230,12 @@ FVB_API fvb_status fvb_set_d2av(fvb_solver *s, double c2, double cg, double sc);
  * the path a lost asynchronous copy would take.  The GPU context stays
  * usable; the solver stops stepping, as after a blow-up. */
 FVB_API fvb_status fvb_debug_drop_load(fvb_solver *s);
+
+/* The same for a chosen load of the next stage that makes it: FVB_DROP_BOX, the
+ * first halo box of CTA 0 (UP and rec3 grids), or FVB_DROP_U0, the U0 tile that
+ * stages 2 and 3 of the FP64 forms load beside it (UP orders 3, 5, 7 and rec3). */
+enum { FVB_DROP_BOX = 1, FVB_DROP_U0 = 2 };
+FVB_API fvb_status fvb_debug_drop(fvb_solver *s, int load);
 /* As fvb_sync, plus FP64 conserved sums over the interior. */
 FVB_API fvb_status fvb_stats_sums(fvb_solver *s, fvb_stats *st);
 /* Record the whole step (three stage kernels) as a CUDA graph and replay it
