@@ -481,17 +481,25 @@ cudaError_t sums_partials(const void *st, const void *lo, const BufView &v, int 
 // and max reduction (fv_up7_ducros_2d.cu:593-612)
 // ---------------------------------------------------------------------------
 // Quotients of one denominator.  FP64: from one reciprocal with the operator's
-// bits (fvb_ieee.cuh), the operator itself out of that form's range.
+// bits (fvb_ieee.cuh) while `ok`, which collects the range tests, stays true.
 template <class R> struct Over {
     R b;
-    __device__ __forceinline__ explicit Over(R x) : b(x) {}
-    __device__ __forceinline__ R operator()(R a) const { return a / b; }
+    __device__ __forceinline__ Over(R x, bool &) : b(x) {}
+    __device__ __forceinline__ R operator()(R a, bool &) const { return a / b; }
 };
 template <> struct Over<double> {
     double b, y;
-    bool ok;
-    __device__ __forceinline__ explicit Over(double x) : b(x), y(recip(x)), ok(den_ok(x)) {}
-    __device__ __forceinline__ double operator()(double a) const { return ok && num_ok(a) ? quot(a, b, y) : a / b; }
+    __device__ __forceinline__ Over(double x, bool &ok) : b(x), y(recip(x)) { ok = ok && pos_ok(x); }
+    __device__ __forceinline__ double operator()(double a, bool &ok) const
+    {
+        ok = ok && num_ok(a);
+        return quot(a, b, y);
+    }
+};
+template <class R> struct OverPlain {
+    R b;
+    __device__ __forceinline__ OverPlain(R x, bool &) : b(x) {}
+    __device__ __forceinline__ R operator()(R a, bool &) const { return a / b; }
 };
 
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
@@ -508,40 +516,49 @@ __global__ void rk3_kernel(int stage, R *Uo, const R *U0, const R *Uk, const R *
                            Gas<R> gs)
 {
     const long long n2 = (long long)n * n, np2 = (long long)np * np;
-    const Over<R> og(gs.gm1);
+    bool gok = true;
+    const Over<R> og(gs.gm1, gok);
+    const OverPlain<R> pg(gs.gm1, gok);
     const R wa = stage == 2 ? FVB_LIT(R, 0.75) : FVB_LIT(R, 1.) / FVB_LIT(R, 3.);
     const R wb = stage == 2 ? FVB_LIT(R, 0.25) : FVB_LIT(R, 2.) / FVB_LIT(R, 3.);
-    auto energy = [&](const R *w) {
-        return fma(FVB_LIT(R, 0.5) * w[0], fma(w[2], w[2], mul_rn(w[1], w[1])), og(w[3]));
-    };
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k < n2;
          k += (long long)blockDim.x * gridDim.x) {
         int j, i;
         cell_rc(k, n, j, i);
         const long long c = (long long)(j + g) * np + (i + g);
-        R w0[4], wk[4], l[4], cv[4], w[4];
+        R w0[4], wk[4], l[4], w[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             w0[q] = U0[q * np2 + c];
             wk[q] = stage != 1 ? Uk[q * np2 + c] : w0[q];
             l[q] = L[q * n2 + k];
         }
-        // U_k + dt L of the conserved variables, then the combination
-        cv[0] = fma(dt, l[0], wk[0]);
-        cv[1] = fma(wk[0], wk[1], mul_rn(dt, l[1]));
-        cv[2] = fma(wk[0], wk[2], mul_rn(dt, l[2]));
-        cv[3] = fma(dt, l[3], energy(wk));
-        if (stage != 1) {
-            const R c0[4] = {w0[0], mul_rn(w0[0], w0[1]), mul_rn(w0[0], w0[2]), energy(w0)};
+        // U_k + dt L of the conserved variables, then the combination and its
+        // primitives; `rho` is the quotient by the new density
+        auto advance = [&](const auto &gm1, auto rho, bool &ok) {
+            auto energy = [&](const R *v) {
+                return fma(FVB_LIT(R, 0.5) * v[0], fma(v[2], v[2], mul_rn(v[1], v[1])), gm1(v[3], ok));
+            };
+            R cv[4];
+            cv[0] = fma(dt, l[0], wk[0]);
+            cv[1] = fma(wk[0], wk[1], mul_rn(dt, l[1]));
+            cv[2] = fma(wk[0], wk[2], mul_rn(dt, l[2]));
+            cv[3] = fma(dt, l[3], energy(wk));
+            if (stage != 1) {
+                const R c0[4] = {w0[0], mul_rn(w0[0], w0[1]), mul_rn(w0[0], w0[2]), energy(w0)};
 #pragma unroll
-            for (int q = 0; q < 4; ++q) cv[q] = fma(wa, c0[q], mul_rn(wb, cv[q]));
-        }
-        const Over<R> orho(cv[0]);
-        w[0] = floor14(cv[0]);
-        w[1] = orho(cv[1]);
-        w[2] = orho(cv[2]);
-        const R ke = orho(FVB_LIT(R, 0.5) * fma(cv[1], cv[1], mul_rn(cv[2], cv[2])));
-        w[3] = floor14(gs.gm1 * (cv[3] - ke));
+                for (int q = 0; q < 4; ++q) cv[q] = fma(wa, c0[q], mul_rn(wb, cv[q]));
+            }
+            const auto by = rho(cv[0], ok);
+            w[0] = floor14(cv[0]);
+            w[1] = by(cv[1], ok);
+            w[2] = by(cv[2], ok);
+            const R ke = by(FVB_LIT(R, 0.5) * fma(cv[1], cv[1], mul_rn(cv[2], cv[2])), ok);
+            w[3] = floor14(gs.gm1 * (cv[3] - ke));
+        };
+        bool ok = gok;
+        advance(og, [](R x, bool &o) { return Over<R>(x, o); }, ok);
+        if (sizeof(R) == 8 && !ok) advance(pg, [](R x, bool &o) { return OverPlain<R>(x, o); }, ok);
 #pragma unroll
         for (int q = 0; q < 4; ++q) Uo[q * np2 + c] = w[q];
     }

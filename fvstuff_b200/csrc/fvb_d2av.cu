@@ -120,6 +120,12 @@ struct D2State {
     double p, c, u, v, y;  // y: reciprocal of the density
 };
 
+// The forms of a face and of a cell: quotients from shared reciprocals, for tiles
+// without small momenta (see the kernel); the same with small numerators looked
+// after; the operators, for whatever leaves the range.
+enum { D2_NEAR, D2_SMALL, D2_PLAIN };
+
+// (a velocity whose quotient underflows is off, which p and |u| + c do not notice)
 __device__ __forceinline__ bool d2_prim_near(double gam, const double U[4], D2State &w)
 {
     const double y = recip(U[0]);
@@ -130,14 +136,22 @@ __device__ __forceinline__ bool d2_prim_near(double gam, const double U[4], D2St
     const double gp = gam * w.p, cs2 = quot(gp, U[0], y);
     const double x = cs2 > 1e-14 ? cs2 : 1e-14;
     w.c = root(x);
-    return den_ok(U[0]) && num_ok(U[1], U[2], gp) && num_ok(x);
+    return pos_ok(U[0]) && fin_ok(U[1], U[2]) && pos_ok(gp) && fin_ok(x);
 }
 
+template <int FORM>
 __device__ __forceinline__ bool d2_hllc_near(double gam, const double UL[4], const double UR[4], double F[4])
 {
     D2State l, r;
     bool ok = d2_prim_near(gam, UL, l);
     ok = d2_prim_near(gam, UR, r) && ok;
+    if constexpr (FORM == D2_SMALL) {
+        // (p and c of either side take nothing from a small momentum)
+        if (is_small(UL[1])) l.u = small_quot(UL[1], UL[0], l.y);
+        if (is_small(UL[2])) l.v = small_quot(UL[2], UL[0], l.y);
+        if (is_small(UR[1])) r.u = small_quot(UR[1], UR[0], r.y);
+        if (is_small(UR[2])) r.v = small_quot(UR[2], UR[0], r.y);
+    }
     const double SL = smin<double>(l.u - l.c, r.u - r.c);
     const double SR = smax<double>(l.u + l.c, r.u + r.c);
     if (SL >= 0.0) {
@@ -149,8 +163,9 @@ __device__ __forceinline__ bool d2_hllc_near(double gam, const double UL[4], con
         return ok;
     }
     const double dL = UL[0] * (SL - l.u), dR = UR[0] * (SR - r.u);
-    const double sn = r.p - l.p + dL * l.u - dR * r.u, sd = dL - dR;
-    const double Ss = quot(sn, sd, recip(sd));
+    const double sn = r.p - l.p + dL * l.u - dR * r.u, sd = dL - dR, yd = recip(sd);
+    double Ss = squot(sn, sd, yd);
+    if (FORM == D2_SMALL && is_small(sn)) Ss = small_quot(sn, sd, yd);
     const bool left = Ss >= 0.0;
     const double K0 = left ? UL[0] : UR[0], K1 = left ? UL[1] : UR[1];
     const double K2 = left ? UL[2] : UR[2], K3 = left ? UL[3] : UR[3];
@@ -158,40 +173,43 @@ __device__ __forceinline__ bool d2_hllc_near(double gam, const double UL[4], con
     const double yK = left ? l.y : r.y;
     const double dK = left ? dL : dR;  // K0 (SK - uK), the same product
     const double sq = SK - Ss;
-    const double f = quot(dK, sq, recip(sq));
-    const double s3 = f * (quot(K3, K0, yK) + (Ss - uK) * (Ss + quot(pK, dK, recip(dK))));
+    const double f = squot(dK, sq, recip(sq));
+    const double s3 = f * (quot(K3, K0, yK) + (Ss - uK) * (Ss + squot(pK, dK, recip(dK))));
     F[0] = K1 + SK * (f - K0);
     F[1] = (K1 * uK + pK) + SK * (f * Ss - K1);
     F[2] = K1 * vK + SK * (f * vK - K2);
     F[3] = (K3 + pK) * uK + SK * (s3 - K3);
-    return ok && den_ok(sd) && den_ok(sq) && den_ok(dK) && num_ok(sn, K3, pK);
+    return ok && den_ok(sd) && den_ok(sq) && den_ok(dK) && fin_ok(sn) && pos_ok(K3);
 }
 
 // (a product with 2 or 4 is exact, so fused with the sum beside it it rounds
-// as the separate operations do)
-template <int ORDER>
+// as the separate operations do; SMALL: sums whose quotients underflow are
+// looked after)
+template <int ORDER, bool SMALL>
 __device__ __forceinline__ void d2_recon_near(const double *s, double &vL, double &vR)
 {
+    constexpr double D = ORDER == 3 ? 6.0 : ORDER == 5 ? 60.0 : ORDER == 9 ? 2520.0 : 420.0;
+    double a, b;
     if constexpr (ORDER == 3) {
-        vL = quot(fma(2.0, s[2], -s[0] + 5.0 * s[1]), 6.0, 1.0 / 6.0);
-        vR = quot(fma(2.0, s[1], 5.0 * s[2]) - s[3], 6.0, 1.0 / 6.0);
+        a = fma(2.0, s[2], -s[0] + 5.0 * s[1]);
+        b = fma(2.0, s[1], 5.0 * s[2]) - s[3];
     } else if constexpr (ORDER == 5) {
-        vL = quot(fma(2.0, s[0], -(13.0 * s[1])) + 47.0 * s[2] + 27.0 * s[3] - 3.0 * s[4], 60.0, 1.0 / 60.0);
-        vR = quot(fma(2.0, s[5], -3.0 * s[1] + 27.0 * s[2] + 47.0 * s[3] - 13.0 * s[4]), 60.0, 1.0 / 60.0);
+        a = fma(2.0, s[0], -(13.0 * s[1])) + 47.0 * s[2] + 27.0 * s[3] - 3.0 * s[4];
+        b = fma(2.0, s[5], -3.0 * s[1] + 27.0 * s[2] + 47.0 * s[3] - 13.0 * s[4]);
     } else if constexpr (ORDER == 9) {
-        vL = quot(3.0 * s[0] - 25.0 * s[1] + 101.0 * s[2] - 319.0 * s[3] + 2765.0 * s[4] + 2139.0 * s[5] -
-                      533.0 * s[6] + 97.0 * s[7] - 11.0 * s[8],
-                  2520.0, 1.0 / 2520.0);
-        vR = quot(-11.0 * s[1] + 97.0 * s[2] - 533.0 * s[3] + 2139.0 * s[4] + 2765.0 * s[5] - 319.0 * s[6] +
-                      101.0 * s[7] - 25.0 * s[8] + 3.0 * s[9],
-                  2520.0, 1.0 / 2520.0);
+        a = 3.0 * s[0] - 25.0 * s[1] + 101.0 * s[2] - 319.0 * s[3] + 2765.0 * s[4] + 2139.0 * s[5] - 533.0 * s[6] +
+            97.0 * s[7] - 11.0 * s[8];
+        b = -11.0 * s[1] + 97.0 * s[2] - 533.0 * s[3] + 2139.0 * s[4] + 2765.0 * s[5] - 319.0 * s[6] + 101.0 * s[7] -
+            25.0 * s[8] + 3.0 * s[9];
     } else {
-        vL = quot(fma(4.0, s[6], -3.0 * s[0] + 25.0 * s[1] - 101.0 * s[2] + 319.0 * s[3] + 214.0 * s[4] -
-                                     38.0 * s[5]),
-                  420.0, 1.0 / 420.0);
-        vR = quot(fma(4.0, s[1], -(38.0 * s[2])) + 214.0 * s[3] + 319.0 * s[4] - 101.0 * s[5] + 25.0 * s[6] -
-                      3.0 * s[7],
-                  420.0, 1.0 / 420.0);
+        a = fma(4.0, s[6], -3.0 * s[0] + 25.0 * s[1] - 101.0 * s[2] + 319.0 * s[3] + 214.0 * s[4] - 38.0 * s[5]);
+        b = fma(4.0, s[1], -(38.0 * s[2])) + 214.0 * s[3] + 319.0 * s[4] - 101.0 * s[5] + 25.0 * s[6] - 3.0 * s[7];
+    }
+    vL = quot(a, D, 1.0 / D);
+    vR = quot(b, D, 1.0 / D);
+    if (SMALL && is_small(a, b)) {
+        if (is_small(a)) vL = small_quot(a, D, 1.0 / D);
+        if (is_small(b)) vR = small_quot(b, D, 1.0 / D);
     }
 }
 
@@ -210,8 +228,8 @@ struct D2Shape {
 };
 
 // the flux of one face in its normal frame, b its right / top cell, st the
-// stride to the left / bottom one; NEAR: the shared-reciprocal form
-template <int ORDER, bool NEAR>
+// stride to the left / bottom one
+template <int ORDER, int FORM>
 __device__ __forceinline__ bool d2_face(const double *Q, int b, int st, bool xf, double gam, double Fn[4])
 {
     using S = D2Shape<ORDER>;
@@ -222,20 +240,51 @@ __device__ __forceinline__ bool d2_face(const double *Q, int b, int st, bool xf,
         double s[2 * HW];
 #pragma unroll
         for (int d = 0; d < 2 * HW; ++d) s[d] = Q[q * S::PL + b + (d - HW) * st];
-        if constexpr (NEAR) d2_recon_near<ORDER>(s, L[q], R[q]);
-        else d2_recon<ORDER>(s, L[q], R[q]);
+        if constexpr (FORM == D2_PLAIN) d2_recon<ORDER>(s, L[q], R[q]);
+        else if (q == 1 || q == 2) d2_recon_near<ORDER, FORM == D2_SMALL>(s, L[q], R[q]);
+        else d2_recon_near<ORDER, false>(s, L[q], R[q]);
     }
     const double UL[4] = {L[0], xf ? L[1] : L[2], xf ? L[2] : L[1], L[3]};
     const double UR[4] = {R[0], xf ? R[1] : R[2], xf ? R[2] : R[1], R[3]};
-    if constexpr (NEAR) return d2_hllc_near(gam, UL, UR, Fn);
+    if constexpr (FORM != D2_PLAIN) return d2_hllc_near<FORM>(gam, UL, UR, Fn);
     d2_hllc(gam, UL, UR, Fn);
     return true;
 }
 
+// a face that the forms above gave up
 template <int ORDER>
 __device__ __noinline__ void d2_face_any(const double *Q, int b, int st, bool xf, double gam, double Fn[4])
 {
-    d2_face<ORDER, false>(Q, b, st, xf, gam, Fn);
+    d2_face<ORDER, D2_PLAIN>(Q, b, st, xf, gam, Fn);
+}
+
+// the faces of a tile
+template <int ORDER, int FORM>
+__device__ __forceinline__ void d2_faces(const double *Q, double *FX, double *FY, double gam, int tid)
+{
+    using S = D2Shape<ORDER>;
+    constexpr int HB = S::HB, BW = S::BW;
+    for (int f = tid; f < S::NFX + S::NFY; f += DNT) {
+        const bool xf = f < S::NFX;
+        int r, c, st;
+        if (xf) { r = f / (DTX + 1); c = f - r * (DTX + 1); st = 1; }
+        else { const int f2 = f - S::NFX; r = f2 / DTX; c = f2 - r * DTX; st = BW; }
+        const int b = (r + HB) * BW + (c + HB);
+        double Fn[4];
+        if (!d2_face<ORDER, FORM>(Q, b, st, xf, gam, Fn)) {
+            double Fa[4];
+            d2_face_any<ORDER>(Q, b, st, xf, gam, Fa);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) Fn[q] = Fa[q];
+        }
+        const int qn = xf ? 1 : 2, qt = xf ? 2 : 1;
+        double *o = xf ? FX + r * (DTX + 1) + c : FY + r * DTX + c;
+        const int os = xf ? S::NFX : S::NFY;
+        o[0] = Fn[0];
+        o[qn * os] = Fn[1];
+        o[qt * os] = Fn[2];
+        o[3 * os] = Fn[3];
+    }
 }
 
 // per-cell quantities of the box in the operator form
@@ -265,14 +314,16 @@ struct D2Cell {
     double h, yh, h60, y60, c2h, cgh, sch, dt;  // y*: reciprocals of h and 60 h
     int stage;
     bool global;  // Cg is not 0
+    bool hok;     // h within 2^+-90: h and 60 h are denominators in range, and see d2_cell
 };
 
 // residual (flux divergence, Ducros weight, viscosity) and RK combination of
-// the cell at b of the box; ua: U0 of the cell.  NEAR: quotients by h and by
-// the sensor's denominator in the shared-reciprocal form
+// the cell at b of the box; ua: U0 of the cell; false: out of range.  (Only the
+// momenta can be as small as a flux difference whose quotient underflows, and a
+// velocity difference of that kind squares to 0.)
 //                                          fv_up7_ducros_2d.cu.bak:344-445
-template <int ORDER, bool NEAR>
-__device__ __forceinline__ void d2_cell(const double *Q, const double *FX, const double *FY, int b, int r, int c,
+template <int ORDER, int FORM>
+__device__ __forceinline__ bool d2_cell(const double *Q, const double *FX, const double *FY, int b, int r, int c,
                                         const D2Cell &k, const double ua[4], double v[4])
 {
     using S = D2Shape<ORDER>;
@@ -286,7 +337,7 @@ __device__ __forceinline__ void d2_cell(const double *Q, const double *FX, const
         du_dx += wc[m] * SU[b + wo[m]];
         dv_dy += wc[m] * SV[b + wo[m] * BW];
     }
-    if constexpr (NEAR) {
+    if constexpr (FORM != D2_PLAIN) {
         du_dx = quot(du_dx, k.h60, k.y60);
         dv_dy = quot(dv_dy, k.h60, k.y60);
     } else {
@@ -299,8 +350,13 @@ __device__ __forceinline__ void d2_cell(const double *Q, const double *FX, const
     const double sos2 = k.sch * c0 * c0;
     const double dd = div_u * div_u, den = dd + sos2 + 1e-40;
     double S_D;
-    if constexpr (NEAR) S_D = quot(dd, den, recip(den));
-    else S_D = dd / den;
+    if constexpr (FORM != D2_PLAIN) {
+        const double y = recip(den);
+        S_D = quot(dd, den, y);
+        if (FORM == D2_SMALL && is_small(dd)) S_D = small_quot(dd, den, y);
+    } else {
+        S_D = dd / den;
+    }
     // face-averaged directional wave speeds   :359-367
     const double lamx_c = LX[b], lamy_c = LY[b];
     const double lhxp = 0.5 * (lamx_c + LX[b + 1]);
@@ -315,26 +371,43 @@ __device__ __forceinline__ void d2_cell(const double *Q, const double *FX, const
         const double dyp = Qq[b + BW] - Uc, dym = Uc - Qq[b - BW];
         double D2 = k.c2h * (lhxp * S_D * dxp - lhxm * S_D * dxm + lhyp * S_D * dyp - lhym * S_D * dym);
         // (with Cg = 0 the term is +0 or -0 for finite states: nothing to add)
-        if (!NEAR || k.global)
+        if (FORM == D2_PLAIN || k.global)
             D2 = D2 + k.cgh * (lhxp * (1. - S_D) * dxp - lhxm * (1. - S_D) * dxm + lhyp * (1. - S_D) * dyp -
                                lhym * (1. - S_D) * dym);
         const double *fx = FX + q * S::NFX + r * (DTX + 1) + c;
         const double *fy = FY + q * S::NFY + r * DTX + c;
         double L;
-        if constexpr (NEAR) L = -quot(fx[1] - fx[0], k.h, k.yh) - quot(fy[DTX] - fy[0], k.h, k.yh) + D2;
-        else L = -(fx[1] - fx[0]) / k.h - (fy[DTX] - fy[0]) / k.h + D2;  // :386
+        if constexpr (FORM != D2_PLAIN) {
+            const double dx = fx[1] - fx[0], dy = fy[DTX] - fy[0];
+            double qx = quot(dx, k.h, k.yh), qy = quot(dy, k.h, k.yh);
+            if (FORM == D2_SMALL && (q == 1 || q == 2) && is_small(dx)) qx = small_quot(dx, k.h, k.yh);
+            if (FORM == D2_SMALL && (q == 1 || q == 2) && is_small(dy)) qy = small_quot(dy, k.h, k.yh);
+            L = -qx - qy + D2;
+        } else {
+            L = -(fx[1] - fx[0]) / k.h - (fy[DTX] - fy[0]) / k.h + D2;  // :386
+        }
         if (k.stage == 1) v[q] = ua[q] + k.dt * L;                                   // :433-435
         else if (k.stage == 2) v[q] = 0.75 * ua[q] + 0.25 * (Uc + k.dt * L);         // :437-440
         else v[q] = (1. / 3.) * ua[q] + (2. / 3.) * (Uc + k.dt * L);                 // :442-445
     }
+    return FORM == D2_PLAIN || (k.hok && pos_ok(den) && (FORM == D2_SMALL || !is_small(dd)) && fin_ok(v[0], v[1]) &&
+                                fin_ok(v[2], v[3]));
 }
 
 template <int ORDER>
 __device__ __noinline__ void d2_cell_any(const double *Q, const double *FX, const double *FY, int b, int r, int c,
                                          const D2Cell &k, const double ua[4], double v[4])
 {
-    d2_cell<ORDER, false>(Q, FX, FY, b, r, c, k, ua, v);
+    d2_cell<ORDER, D2_PLAIN>(Q, FX, FY, b, r, c, k, ua, v);
 }
+
+// A tile whose momenta are 0 or at least 2^-300 and whose densities lie within
+// 2^+-30, box and all, has no face and no flux difference with a small numerator
+// (fvb_ieee.cuh): a sum that is not 0 is at least an ulp of its smaller term, so
+// reconstructions are 0 or from 2^-364 on, velocities 2^-396, products of the
+// two 2^-760, fluxes 2^-812 and their differences 2^-864.  The others, in the
+// tails ahead of a front, take the form that looks after them.
+constexpr unsigned kMomMin = 0x2d300000u, kRhoMin = 0x3e100000u, kRhoMax = 0x41d00000u;
 
 // one SSP-RK3 stage                        fv_up7_ducros_2d.cu.bak:287-446
 template <int ORDER>
@@ -342,7 +415,7 @@ __global__ void __launch_bounds__(DNT, D2Shape<ORDER>::MINB)
     d2av_stage_kernel(const __grid_constant__ GridDev gd, int stage, int ntiles, D2Params av)
 {
     using S = D2Shape<ORDER>;
-    constexpr int HW = S::HW, HB = S::HB, BW = S::BW, PL = S::PL;
+    constexpr int HB = S::HB, BW = S::BW, PL = S::PL;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double *Q = reinterpret_cast<double *>(smem_raw);  // [4][BH][BW] stage input
     double *SU = Q + 4 * PL;                           // rho u / max(rho, 1e-14)
@@ -367,8 +440,7 @@ __global__ void __launch_bounds__(DNT, D2Shape<ORDER>::MINB)
     const TileCtl ctl = tile_control<P64>(gd.ctrl, stage, tid == 0 && blockIdx.x == 0);
     if (tid == 0)
         ck = D2Cell{h, recip(h), 60. * h, recip(60. * h), av.c2 / h, av.cg / h, av.sc / (h * h), ctl.dt, stage,
-                    av.cg != 0.0};
-    const bool hok = den_ok(h) && den_ok(60. * h);
+                    av.cg != 0.0, h > 0x1p-90 && h < 0x1p90};
 
     // From two whole waves up a CTA takes its next tile as it comes free: us a
     // stage, fixed share / taken, order 5: 600^2 34.4 / 32.7, 800^2 55.7 / 54.8, 1024^2
@@ -380,6 +452,7 @@ __global__ void __launch_bounds__(DNT, D2Shape<ORDER>::MINB)
         // ---- halo box of the stage input and its per-cell quantities: the
         //      sensor's velocities in the rows / columns it reaches, the wave
         //      speeds on the cells and their direct neighbours --------------
+        unsigned least = 0x7fffffffu;  // least momentum of this thread's cells; 0: a density out of range
         for (int k = tid; k < PL; k += DNT) {
             const int r = k / BW, c = k - r * BW, jp = ty0 + r, ip = tx0 + c;
             double U[4] = {1.0, 0.0, 0.0, 2.5};  // admissible filler beyond the padded grid
@@ -390,10 +463,13 @@ __global__ void __launch_bounds__(DNT, D2Shape<ORDER>::MINB)
             }
 #pragma unroll
             for (int q = 0; q < 4; ++q) Q[q * PL + k] = U[q];
+            least = min(least, min(hi_below(U[1]), hi_below(U[2])));
+            if ((unsigned)__double2hiint(U[0]) - kRhoMin >= kRhoMax - kRhoMin) least = 0u;
             const bool inr = (unsigned)(r - HB) < (unsigned)DTY, inc = (unsigned)(c - HB) < (unsigned)DTX;
             if (!inr && !inc) continue;
             D2State w;
-            // (the sensor's velocities divide by the density floored at 1e-14)
+            // (the sensor's velocities divide by the density floored at 1e-14; one that is
+            // off is below 2^-850 and changes no divergence whose square is not 0)
             if (d2_prim_near(gam, U, w) && U[0] > 1e-14) {
                 SU[k] = w.u;
                 SV[k] = w.v;
@@ -407,32 +483,13 @@ __global__ void __launch_bounds__(DNT, D2Shape<ORDER>::MINB)
                 for (int m = 0; m < 5; ++m) SU[m * PL + k] = o[m];
             }
         }
-        __syncthreads();
+        const bool small = __syncthreads_or(least < kMomMin);
         int taken = ntiles;  // the next tile, taken while the faces are computed
         if (queued && tid == 0) taken = (int)gridDim.x + atomicAdd(tile_queue(gd.ctrl, stage), 1);
         // ---- faces: x-face (r, c) between tile cells c-1 and c, y-face
         //      (r, c) between rows r-1 and r; b = the right / top cell -----
-        for (int f = tid; f < S::NFX + S::NFY; f += DNT) {
-            const bool xf = f < S::NFX;
-            int r, c, st;
-            if (xf) { r = f / (DTX + 1); c = f - r * (DTX + 1); st = 1; }
-            else { const int f2 = f - S::NFX; r = f2 / DTX; c = f2 - r * DTX; st = BW; }
-            const int b = (r + HB) * BW + (c + HB);
-            double Fn[4];
-            if (!d2_face<ORDER, true>(Q, b, st, xf, gam, Fn)) {
-                double Fa[4];
-                d2_face_any<ORDER>(Q, b, st, xf, gam, Fa);
-#pragma unroll
-                for (int q = 0; q < 4; ++q) Fn[q] = Fa[q];
-            }
-            const int qn = xf ? 1 : 2, qt = xf ? 2 : 1;
-            double *o = xf ? FX + r * (DTX + 1) + c : FY + r * DTX + c;
-            const int os = xf ? S::NFX : S::NFY;
-            o[0] = Fn[0];
-            o[qn * os] = Fn[1];
-            o[qt * os] = Fn[2];
-            o[3 * os] = Fn[3];
-        }
+        if (small) d2_faces<ORDER, D2_SMALL>(Q, FX, FY, gam, tid);
+        else d2_faces<ORDER, D2_NEAR>(Q, FX, FY, gam, tid);
         if (queued && tid == 0) s_next = taken;
         __syncthreads();
         next = queued ? s_next : t + (int)gridDim.x;
@@ -446,8 +503,9 @@ __global__ void __launch_bounds__(DNT, D2Shape<ORDER>::MINB)
             double ua[4], v[4];
 #pragma unroll
             for (int q = 0; q < 4; ++q) ua[q] = stage == 1 ? Q[q * PL + b] : u0[e + q * gd.plane];
-            d2_cell<ORDER, true>(Q, FX, FY, b, r, c, ck, ua, v);
-            if (!hok || max(max(hi_mag(v[0]), hi_mag(v[1])), max(hi_mag(v[2]), hi_mag(v[3]))) >= kHiMax) {
+            const bool ok = small ? d2_cell<ORDER, D2_SMALL>(Q, FX, FY, b, r, c, ck, ua, v)
+                                  : d2_cell<ORDER, D2_NEAR>(Q, FX, FY, b, r, c, ck, ua, v);
+            if (!ok) {
                 double ub[4], va[4];
 #pragma unroll
                 for (int q = 0; q < 4; ++q) ub[q] = ua[q];

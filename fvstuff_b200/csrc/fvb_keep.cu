@@ -74,7 +74,7 @@ __device__ __forceinline__ bool k_prim_near(const double U[4], double gam, doubl
     W[2] = v;
     W[3] = smax<double>((gam - 1.) * (E - 0.5 * rho * (u * u + v * v)), KG_MIN);
     Uf[0] = rho; Uf[1] = mx; Uf[2] = my; Uf[3] = E;
-    return den_ok(rho) && num_ok(mx, my) && num_ok(W[3]);
+    return pos_ok(rho) && num_ok(mx, my) && fin_ok(W[3]);
 }
 
 __device__ __forceinline__ bool k_evars_near(const double W[4], double s, double gam, double ygm1, double V[4])
@@ -87,7 +87,10 @@ __device__ __forceinline__ bool k_evars_near(const double W[4], double s, double
     V[1] = quot(ru, p, y);
     V[2] = quot(rv, p, y);
     V[3] = -quot(rho, p, y);
-    return den_ok(p) && num_ok(ke, ru, rv) && num_ok(s);
+    // (ru and rv are the momenta but for a rounding or two, which k_prim_near
+    // tests; beside the quotient of a gamma - s that is not 0 the last bits of a
+    // small ke's are nothing)
+    return pos_ok(p) && fin_ok(ke, s) && den_ok(gam - s);
 }
 
 // both in the operator form
@@ -249,7 +252,8 @@ __device__ __forceinline__ bool k_face_near(const double *U, const double *W, co
     const double rav = 0.5 * (rL + rR);
     double sx;
     const double aav = k_snd_near(rav, pb, gam, sx);
-    bool ok = num_ok(num) && den_ok(den) && den_ok(sx) && num_ok(EL, ER);
+    // (a small num's quotient changes the energy by nothing)
+    bool ok = fin_ok(num) && pos_ok(den) && pos_ok(sx) && fin_ok(EL, ER);
     // shock sensor                                 keep_fv:249-258, :347-349
     const double dU0 = rR - rL, dU1 = U[KPL + b] - U[KPL + a], dU2 = U[2 * KPL + b] - U[2 * KPL + a];
     const double dU3 = U[3 * KPL + b] - U[3 * KPL + a];
@@ -286,11 +290,11 @@ __device__ __forceinline__ bool k_face_near(const double *U, const double *W, co
     for (int q = 0; q < 4; ++q) {
         const double dU = dUq[q], dF = dFq[q];
         const bool small = fabs(dU) < 1e-12;
-        double sk = small ? lmin : fabs(quot(dF, dU, recip(small ? 1.0 : dU)));
+        double sk = small ? lmin : fabs(squot(dF, dU, recip(small ? 1.0 : dU)));
         if (sk >= lmax) sk = lmax;
         else if (sk <= lmin) sk = lmin;
         if (sk < aS) aS = sk;
-        ok = ok && num_ok(dF, dU);
+        ok = ok && fin_ok(dF) && hi_mag(dU) < kDenMax;  // (a smaller |dF| gives a speed that the fix replaces)
     }
     if (aS < 0.1) aS = (aS * aS + 0.1 * 0.1) / (2. * 0.1);
     const double dUc[4] = {dU0, dU1, dU2, dU3};
@@ -520,7 +524,7 @@ __global__ void __launch_bounds__(KNT, 2) keep_stage_kernel(const __grid_constan
                 double Wn[4], Fn[4], x;
                 bool ok = k_prim_near(v, gam, Wn, Fn);
                 double cs = k_snd_near(Wn[0], Wn[3], gam, x);
-                if (!(ok && den_ok(x))) {
+                if (!(ok && pos_ok(x))) {
                     k_prim_any(v, gam, Wn);
                     cs = k_snd_any(Wn[0], Wn[3], gam);
                 }

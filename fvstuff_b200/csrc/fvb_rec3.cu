@@ -142,15 +142,22 @@ __device__ __forceinline__ void r3_scale_w(const double Ub[4], double U[4], doub
 // (`ok` stays true); the caller evaluates the operator form otherwise.
 constexpr double R3_GM1 = R3_GAM - 1.0, R3_YGM1 = 1.0 / R3_GM1;
 
-// velocity and pressure of a conserved state; r: the floored density
-__device__ __forceinline__ double r3_p_near(const double U[4], double &r, double &u, double &v, bool &ok)
+// Velocity and pressure of a conserved state; r: the floored density.  (The
+// pressure takes nothing from a small momentum: its square is 0.  The velocities
+// do, so who uses them tests that.)
+__device__ __forceinline__ double r3_p_of(const double U[4], double &r, double &u, double &v)
 {
     r = smax<double>(U[0], R3_RHOFLOOR);
     const double y = recip(r);
     u = quot(U[1], r, y);
     v = quot(U[2], r, y);
-    ok = ok && den_ok(r) && num_ok(U[1], U[2], U[3]);
     return R3_GM1 * (U[3] - 0.5 * r * (u * u + v * v));
+}
+__device__ __forceinline__ double r3_p_near(const double U[4], double &r, double &u, double &v, bool &ok)
+{
+    const double p = r3_p_of(U, r, u, v);
+    ok = ok && pos_ok(r) && fin_ok(U[1], U[2]) && fin_ok(U[3]);
+    return p;
 }
 
 __device__ __noinline__ void r3_scale_any(const double Ub[4], double U[4], double W[4])
@@ -159,12 +166,12 @@ __device__ __noinline__ void r3_scale_any(const double Ub[4], double U[4], doubl
 }
 
 // r3_scale_w of a face state that clears its floors (nearly all): converted
-// at once; false: it needs the scaling
+// at once; false: it needs the scaling, or is out of range.  (Momenta out of
+// range above give no pressure that clears the floor.)
 __device__ __forceinline__ bool r3_clear_near(const double U[4], double W[4])
 {
-    bool ok = U[0] >= R3_RHOFLOOR;
-    W[3] = r3_p_near(U, W[0], W[1], W[2], ok);
-    return ok && W[3] >= R3_PFLOOR;
+    W[3] = r3_p_of(U, W[0], W[1], W[2]);
+    return U[0] >= R3_RHOFLOOR && pos_ok(U[0]) && fin_ok(U[3]) && !is_small(U[1], U[2]) && W[3] >= R3_PFLOOR;
 }
 
 // r3_scale_w with the bisection's pressures in the shared-reciprocal form
@@ -197,7 +204,7 @@ __device__ __forceinline__ void r3_scale_near(const double Ub[4], double U[4], d
         p = r3_p_near(S, W[0], W[1], W[2], ok);
     }
     W[3] = smax<double>(p, R3_PFLOOR);
-    if (!ok) {
+    if (!(ok && num_ok(S[1], S[2]))) {
         // (by copies, so that the arrays of the usual path stay in registers)
         double B[4], X[4];
 #pragma unroll
@@ -217,12 +224,12 @@ __device__ __forceinline__ bool r3_hllc_near(const double L[4], const double R[4
     const double yL = recip(rL), yR = recip(rR);
     const double xL = quot(R3_GAM * pL, rL, yL), xR = quot(R3_GAM * pR, rR, yR);
     const double cL = root(xL), cR = root(xR);
-    bool ok = den_ok(rL) && den_ok(rR) && den_ok(xL) && den_ok(xR) && num_ok(pL, pR);
+    bool ok = pos_ok(rL) && pos_ok(rR) && pos_ok(xL) && pos_ok(xR) && fin_ok(pL, pR);  // (p >= 1e-9)
     const double SL = smin<double>(uL - cL, uR - cR), SR = smax<double>(uL + cL, uR + cR);
     const bool supL = SL >= 0., sup = supL || SR <= 0.;
     const double dL = rL * (SL - uL), dR = rR * (SR - uR);
     const double sn = pR - pL + dL * uL - dR * uR, sd = dL - dR;
-    const double Ss = quot(sn, sd, recip(sd));
+    const double Ss = squot(sn, sd, recip(sd));
     // the side whose state the flux needs: the upwind one, or the contact's
     const bool left = sup ? supL : Ss >= 0.;
     const double rK = left ? rL : rR, uK = left ? uL : uR, tK = left ? tL : tR, pK = left ? pL : pR;
@@ -235,13 +242,13 @@ __device__ __forceinline__ bool r3_hllc_near(const double L[4], const double R[4
         return ok;
     }
     const double sq = SK - Ss;
-    const double f = quot(dK, sq, recip(sq));
-    const double Us3 = f * (quot(EK, rK, yK) + (Ss - uK) * (Ss + quot(pK, dK, recip(dK))));
+    const double f = squot(dK, sq, recip(sq));
+    const double Us3 = f * (quot(EK, rK, yK) + (Ss - uK) * (Ss + squot(pK, dK, recip(dK))));
     F[0] = F0 + SK * (f - rK);
     F[1] = F1 + SK * (f * Ss - mK);
     F[2] = F2 + SK * (f * tK - rK * tK);
     F[3] = F3 + SK * (Us3 - EK);
-    return ok && den_ok(sd) && den_ok(sq) && den_ok(dK) && num_ok(sn, EK);
+    return ok && den_ok(sd) && den_ok(sq) && den_ok(dK) && num_ok(sn) && fin_ok(EK);
 }
 
 __device__ __noinline__ void r3_hllc_any(const double L[4], const double R[4], double F[4]) { r3_hllc(L, R, F); }
@@ -582,7 +589,7 @@ __global__ void __launch_bounds__(RNT, 2) rec3_stage_kernel(const __grid_constan
                     const double p = smax<double>(r3_p_near(U, rr, u, v, ok), R3_PFLOOR);
                     const double x = quot(R3_GAM * p, rr, recip(rr));
                     const double lam = fabs(u) + fabs(v) + root(x);
-                    lacc = smax<double>(ok && den_ok(x) ? lam : r3_lam_any(U[0], U[1], U[2], U[3]), lacc);
+                    lacc = smax<double>(ok && pos_ok(x) ? lam : r3_lam_any(U[0], U[1], U[2], U[3]), lacc);
                 }
             }
         }

@@ -1,0 +1,140 @@
+"""The shared-reciprocal quotients of the kernels (fvb_ieee.cuh) compiled for
+the host: wherever a caller's range tests hold, the value has the bits of the
+operator's, the sign of a zero included, and the tests hold for every zero
+numerator.  No GPU needed; the device's reciprocal seed is the host's exact one
+here (test_gpu_quotients.py has the device's)."""
+from __future__ import annotations
+
+import ctypes as C
+import os
+import subprocess
+from pathlib import Path
+
+import numpy as np
+import pytest
+
+ROOT = Path(__file__).resolve().parent.parent
+CUDA = Path(os.environ.get("CUDA_HOME", "/usr/local/cuda")) / "include"
+
+HOST = r"""
+#include <cmath>
+#include <cstring>
+#include <stdint.h>
+#include <cuda_runtime.h>
+using std::fma; using std::fabs; using std::sqrt;
+static inline unsigned max(unsigned a, unsigned b) { return a > b ? a : b; }
+static inline unsigned min(unsigned a, unsigned b) { return a < b ? a : b; }
+static inline long long __double_as_longlong(double x) { long long v; std::memcpy(&v, &x, 8); return v; }
+static inline int __double2hiint(double x) { return (int)(__double_as_longlong(x) >> 32); }
+static inline int __double2loint(double x) { return (int)__double_as_longlong(x); }
+static inline double __hiloint2double(int h, int l)
+{
+    const long long v = ((long long)h << 32) | (unsigned)l;
+    double x;
+    std::memcpy(&x, &v, 8);
+    return x;
+}
+static inline unsigned __float_as_uint(float x) { unsigned v; std::memcpy(&v, &x, 4); return v; }
+using std::rint; using std::copysign;
+static inline double __drcp_rn(double x) { return 1.0 / x; }
+static inline float __frcp_rn(float x) { return 1.0f / x; }
+static inline float __fmaf_rn(float a, float b, float c) { return std::fma(a, b, c); }
+static inline float __fmul_rn(float a, float b) { return a * b; }
+static inline float __fdividef(float a, float b) { return a / b; }
+static inline float rsqrtf(float x) { return 1.0f / std::sqrt(x); }
+#define FVB_EXACT_RCP_SQRT 1
+#include "fvb_ieee.cuh"
+#include "fvb_face32.cuh"
+extern "C" {
+// 1: the range tests hold, and q is the kernels' quotient
+void quot64(int n, const double *a, const double *b, double *q, int *ok)
+{
+    for (int i = 0; i < n; ++i) {
+        q[i] = fvb::quot(a[i], b[i], fvb::recip(b[i]));
+        ok[i] = fvb::num_ok(a[i]) && fvb::den_ok(b[i]) && b[i] > 0;
+    }
+}
+void small64(int n, const double *a, const double *b, double *q, int *ok)
+{
+    for (int i = 0; i < n; ++i) {
+        q[i] = fvb::small_quot(a[i], b[i], fvb::recip(b[i]));
+        ok[i] = (fvb::is_small(a[i]) || a[i] == 0) && fvb::den_ok(b[i]);
+    }
+}
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def host(tmp_path_factory):
+    d = tmp_path_factory.mktemp("quot")
+    src, so = d / "host.cpp", d / "host.so"
+    src.write_text(HOST)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-mfma", "-ffp-contract=off", "-fPIC", "-shared", "-I", str(CUDA),
+                    "-I", str(ROOT / "include"), "-I", str(ROOT / "fvstuff_b200" / "csrc"), "-o", str(so), str(src)],
+                   check=True)
+    return C.CDLL(str(so))
+
+
+RNG = np.random.default_rng(20)
+N = 200000
+
+
+def _mag(lo, hi, dtype=np.float64):
+    with np.errstate(over="ignore", under="ignore"):
+        return np.ldexp(RNG.uniform(1, 2, N), RNG.integers(lo, hi, N)).astype(dtype)
+
+
+def _signed(x):
+    return np.where(RNG.random(N) < 0.5, -x, x).astype(x.dtype)
+
+
+def _ints(k):
+    return RNG.integers(1, k, N).astype(np.float64) * 2.0 ** RNG.integers(-1074, 960, N).astype(np.float64)
+
+
+OPERANDS64 = {
+    "ordinary": lambda: (_signed(_mag(-60, 60)), _mag(-60, 60)),
+    "tiny numerators": lambda: (_signed(_mag(-1074, -700)), _mag(-40, 40)),
+    "subnormal numerators": lambda: (_signed(RNG.integers(1, 1000, N) * 5e-324), _mag(-3, 3)),
+    "zeros": lambda: (_signed(np.zeros(N)), _mag(-500, 99)),
+    "whole range": lambda: (_signed(_mag(-1074, 1023)), _mag(-1000, 1000)),
+    "beside powers of two": lambda: (_signed(_ints(9)), np.ldexp(1.0 + RNG.integers(-4, 5, N) * 2.0 ** -53,
+                                                                 RNG.integers(-20, 20, N))),
+}
+
+
+@pytest.mark.parametrize("name", list(OPERANDS64))
+def test_fp64_quotient_where_its_range_tests_hold(host, name):
+    a, b = (np.ascontiguousarray(x, np.float64) for x in OPERANDS64[name]())
+    q, ok = np.empty(N), np.empty(N, np.int32)
+    p = lambda x: x.ctypes.data_as(C.c_void_p)
+    host.quot64(N, p(a), p(b), p(q), p(ok))
+    with np.errstate(all="ignore"):
+        want = a / b
+    ok = ok.astype(bool)
+    assert np.array_equal(q[ok].view(np.int64), want[ok].view(np.int64))
+    if name in ("ordinary", "zeros"):
+        assert ok.all()  # the usual path
+
+
+@pytest.mark.parametrize("name", list(OPERANDS64) + ["ties"])
+def test_fp64_quotient_of_small_numerators(host, name):
+    """Below num_ok's range, subnormal quotients and their ties included, for
+    denominators of either sign."""
+    if name == "ties":  # (k + 1/2) 2^-1074, exactly, just above and just below
+        b = 2.0 * RNG.integers(1, 1 << 20, N)
+        a = ((2 * RNG.integers(0, 1 << 20, N) + 1) * (b / 2) + RNG.integers(-1, 2, N)) * 5e-324
+        a = _signed(a)
+    else:
+        a, b = OPERANDS64[name]()
+    a, b = np.ascontiguousarray(a, np.float64), np.ascontiguousarray(_signed(np.asarray(b, np.float64)))
+    q, ok = np.empty(N), np.empty(N, np.int32)
+    p = lambda x: x.ctypes.data_as(C.c_void_p)
+    host.small64(N, p(a), p(b), p(q), p(ok))
+    with np.errstate(all="ignore"):
+        want = a / b
+    ok = ok.astype(bool) & ~((a == 0) & np.signbit(a) & (b > 0))  # (squot: a zero numerator is +0)
+    assert np.array_equal(q[ok].view(np.int64), want[ok].view(np.int64))
+    if name in ("ties", "subnormal numerators"):
+        assert ok.all()
