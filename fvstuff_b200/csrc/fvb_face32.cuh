@@ -4,20 +4,23 @@
 //
 // A quotient whose denominator is a constant or shared comes from the rounded
 // reciprocal and the remainder correction of fvb_ieee.cuh, which gives the
-// operator's bits; where an operand is not finite (the corrected quotient is
-// then NaN) the operator itself is evaluated.
+// operator's bits where neither the quotient nor the remainder underflows or
+// overflows (numerators from 2^-101 on, quotients from 2^-126); elsewhere the
+// operator itself is evaluated.
 #pragma once
 #include "fvb_ieee.cuh"
 
 namespace fvb {
 namespace f32 {
 
-// a / b from y = 1 / b rounded to nearest
+// a / b from y = 1 / b rounded to nearest, b > 0
 __device__ __forceinline__ float quot(float a, float b, float y)
 {
-    const float q = a * y;
-    return __fmaf_rn(__fmaf_rn(-q, b, a), y, q);
+    const float q = a * y, r = __fmaf_rn(q, b, -a);
+    return __fmaf_rn(r, -y, q);
 }
+// twice the bits of the number below |a|, in order of magnitude; a zero: the most
+__device__ __forceinline__ unsigned below(float a) { return (__float_as_uint(a) << 1) - 1u; }
 
 struct Gas {
     float gam, gm1, ygm1;  // ygm1: 1 / gm1, rounded to nearest
@@ -30,12 +33,25 @@ __device__ __forceinline__ float sound(float p, float rho, const Gas &gs)
     return sqrtf(cs2 > 1e-14f ? cs2 : 1e-14f);
 }
 
-// total energy of a normal-frame state; the rounding of a fused multiply-add
-// on the normal velocity is written out, so that it is the same wherever the
-// energy is formed                              fv_up7_ducros_2d.cu:77, :251
-__device__ __forceinline__ float energy(float r, float un, float ut, float p, const Gas &gs)
+// p / (gamma - 1): of a cell's pressure, whatever it is (gamma - 1 is at least
+// 2^-23), and of a floored one, where only the overflow needs a look
+__device__ __forceinline__ float over_gm1(float p, const Gas &gs)
 {
-    return __fmaf_rn(0.5f * r, __fmaf_rn(un, un, __fmul_rn(ut, ut)), quot(p, gs.gm1, gs.ygm1));
+    const bool in = __float_as_uint(p) - 0x0f800000u < 0x6f800000u - 0x0f800000u;  // 2^-96 ... 2^96
+    return in ? quot(p, gs.gm1, gs.ygm1) : p / gs.gm1;
+}
+__device__ __forceinline__ float over_gm1_floored(float p, const Gas &gs)
+{
+    const float q = p * gs.ygm1, r = __fmaf_rn(q, gs.gm1, -p);
+    return fabsf(r) <= 3.402823466e38f ? __fmaf_rn(r, -gs.ygm1, q) : q;  // (q is infinite, or a NaN)
+}
+
+// total energy of a normal-frame state from pe = p / (gamma - 1); the rounding
+// of a fused multiply-add on the normal velocity is written out, so that it is
+// the same wherever the energy is formed       fv_up7_ducros_2d.cu:77, :251
+__device__ __forceinline__ float energy(float r, float un, float ut, float pe)
+{
+    return __fmaf_rn(0.5f * r, __fmaf_rn(un, un, __fmul_rn(ut, ut)), pe);
 }
 
 // UP7 face values from the 8-point stencil s (the face lies between s[3] and
@@ -64,7 +80,7 @@ __device__ __forceinline__ void hllc(const float L[4], const float Rr[4], float 
     const float rL = L[0], uL = L[1], tL = L[2], pL = L[3];
     const float rR = Rr[0], uR = Rr[1], tR = Rr[2], pR = Rr[3];
     const float cL = sound(pL, rL, gs), cR = sound(pR, rR, gs);
-    const float EL = energy(rL, uL, tL, pL, gs), ER = energy(rR, uR, tR, pR, gs);
+    const float EL = energy(rL, uL, tL, over_gm1_floored(pL, gs)), ER = energy(rR, uR, tR, over_gm1_floored(pR, gs));
     const float SL = fminf(uL - cL, uR - cR);
     const float SR = fmaxf(uL + cL, uR + cR);
     if (SL >= 0.f) {
@@ -113,11 +129,22 @@ __device__ __forceinline__ void hlle(const float L[4], const float Rr[4], float 
     F[1] = quot(a1, dS, y);
     F[2] = quot(a2, dS, y);
     F[3] = quot(a3, dS, y);
+    // the least numerator against 2^-100 and, for the quotient, 2^-124 dS
+    const unsigned least = min(min(below(a0), below(a1)), min(below(a2), below(a3)));
+    const unsigned bound = max(0x1b000000u, __float_as_uint(dS * 0x1p-124f) << 1);
     if (!(fabsf(F[0]) + fabsf(F[1]) + fabsf(F[2]) + fabsf(F[3]) < 1e37f)) {
         F[0] = a0 / dS;
         F[1] = a1 / dS;
         F[2] = a2 / dS;
         F[3] = a3 / dS;
+    } else if (least < bound) {
+        // in FP64, where nothing underflows and whose quotient's 53 bits round to
+        // FP32 as the quotient itself does (53 >= 2 * 24 + 2)
+        const double D = dS, Y = recip(D);
+        F[0] = (float)fvb::quot(a0, D, Y);
+        F[1] = (float)fvb::quot(a1, D, Y);
+        F[2] = (float)fvb::quot(a2, D, Y);
+        F[3] = (float)fvb::quot(a3, D, Y);
     }
 }
 

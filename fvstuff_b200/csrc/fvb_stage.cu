@@ -203,8 +203,9 @@ __global__ void __launch_bounds__(NT, MINB) stage32_kernel(const __grid_constant
                 const int r = k / SW - (G - 1), c = k % SW - (G - 1);
                 if ((unsigned)r < (unsigned)(TY + 2) && (unsigned)c < (unsigned)CW) {
                     CE[r * CW + c] = f32::sound(w3, w0, g32);
-                    CE[CP + r * CW + c] = f32::energy(w0, w1, w2, w3, g32);
-                    CE[2 * CP + r * CW + c] = f32::energy(w0, w2, w1, w3, g32);
+                    const R pe = f32::over_gm1(w3, g32);
+                    CE[CP + r * CW + c] = f32::energy(w0, w1, w2, pe);
+                    CE[2 * CP + r * CW + c] = f32::energy(w0, w2, w1, pe);
                 }
             }
         }

@@ -54,6 +54,31 @@ void quot64(int n, const double *a, const double *b, double *q, int *ok)
         ok[i] = fvb::num_ok(a[i]) && fvb::den_ok(b[i]) && b[i] > 0;
     }
 }
+// the FP32 face's p / (gamma - 1), and HLLE with its quotients as operators
+void over_gm1_32(int n, const float *p, float gm1, float *e, float *floored, float *plain)
+{
+    const fvb::f32::Gas gs{gm1 + 1.0f, gm1, __frcp_rn(gm1)};
+    for (int i = 0; i < n; ++i) {
+        e[i] = fvb::f32::over_gm1(p[i], gs);
+        floored[i] = fvb::f32::over_gm1_floored(p[i], gs);
+        plain[i] = p[i] / gm1;
+    }
+}
+void hlle32(int n, const float *L, const float *R, const float *c, const float *E, float *F, float *P)
+{
+    for (int i = 0; i < n; ++i) {
+        const float *l = L + 4 * i, *r = R + 4 * i, cL = c[2 * i], cR = c[2 * i + 1], EL = E[2 * i], ER = E[2 * i + 1];
+        fvb::f32::hlle(l, r, cL, cR, EL, ER, F + 4 * i);
+        float *o = P + 4 * i;
+        const float FL[4] = {l[0] * l[1], l[0] * l[1] * l[1] + l[3], l[0] * l[1] * l[2], (EL + l[3]) * l[1]};
+        const float FR[4] = {r[0] * r[1], r[0] * r[1] * r[1] + r[3], r[0] * r[1] * r[2], (ER + r[3]) * r[1]};
+        const float U[4] = {l[0], l[0] * l[1], l[0] * l[2], EL}, V[4] = {r[0], r[0] * r[1], r[0] * r[2], ER};
+        const float SL = std::fmin(l[1] - cL, r[1] - cR), SR = std::fmax(l[1] + cL, r[1] + cR);
+        const float dS = std::fmax(SR - SL, 1e-10f), SRL = SR * SL;
+        for (int q = 0; q < 4; ++q)
+            o[q] = SL >= 0.f ? FL[q] : SR <= 0.f ? FR[q] : (SR * FL[q] - SL * FR[q] + SRL * (V[q] - U[q])) / dS;
+    }
+}
 void small64(int n, const double *a, const double *b, double *q, int *ok)
 {
     for (int i = 0; i < n; ++i) {
@@ -138,3 +163,46 @@ def test_fp64_quotient_of_small_numerators(host, name):
     assert np.array_equal(q[ok].view(np.int64), want[ok].view(np.int64))
     if name in ("ties", "subnormal numerators"):
         assert ok.all()
+
+
+def _f32(*x):
+    return [np.ascontiguousarray(a, np.float32) for a in x]
+
+
+def _same32(got, want):
+    nan = np.isnan(got) & np.isnan(want)
+    return np.array_equal(got.view(np.int32)[~nan], want.view(np.int32)[~nan]) and not np.isnan(got[~nan]).any()
+
+
+@pytest.mark.parametrize("gm1", [0.4, 2.0 / 3.0, 0.0625, 1e-5])
+def test_fp32_pressure_over_gamma_minus_one(host, gm1):
+    """Pressures over all of FP32, infinities among them; floored ones (1e-14 and
+    up) by the form without a range test."""
+    p, = _f32(_mag(-149, 128))
+    p[:100], p[100:200], p[200:300] = np.inf, 0.0, np.nan
+    e, f, plain = (np.empty(N, np.float32) for _ in range(3))
+    ptr = lambda x: x.ctypes.data_as(C.c_void_p)
+    host.over_gm1_32(N, ptr(p), C.c_float(gm1), ptr(e), ptr(f), ptr(plain))
+    assert _same32(e, plain)
+    up = p >= np.float32(1e-14)
+    assert _same32(f[up], plain[up])
+
+
+@pytest.mark.parametrize("vel", [(-20, 4), (-120, -90), (-149, -120), None])
+@pytest.mark.parametrize("unit", [0, 12, 26])
+def test_fp32_hlle(host, vel, unit):
+    """Cell velocities down to subnormal and zero, sound speeds near 1, 2^12 and
+    2^26: numerators and quotients that underflow."""
+    z = np.zeros(N)
+    w = [[_mag(-2, 2), _signed(_mag(*vel) * 2.0 ** unit if vel else z), _signed(_mag(*vel) * 2.0 ** unit if vel else z),
+          _mag(-2, 2) * 4.0 ** unit] for _ in range(2)]
+    same = RNG.random(N) < 0.5  # equal densities and pressures: nothing but the small terms
+    for q in (0, 3):
+        w[1][q] = np.where(same, w[0][q], w[1][q])
+    L, R = (np.ascontiguousarray(np.stack(x, 1), np.float32) for x in w)
+    c = np.ascontiguousarray(np.stack([np.sqrt(1.4 * x[3] / x[0]) for x in w], 1), np.float32)
+    E = np.ascontiguousarray(np.stack([2.5 * x[3] for x in w], 1), np.float32)
+    F, P = np.empty((N, 4), np.float32), np.empty((N, 4), np.float32)
+    ptr = lambda x: x.ctypes.data_as(C.c_void_p)
+    host.hlle32(N, ptr(L), ptr(R), ptr(c), ptr(E), ptr(F), ptr(P))
+    assert _same32(F, P)
