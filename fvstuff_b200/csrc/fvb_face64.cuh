@@ -27,15 +27,16 @@ struct Gas {
     double gam, igm1, gm1;  // gamma, 1/(gamma-1), gamma-1
 };
 
-// floor used on reconstructed and updated rho and p (NaN -> the floor)
-// (compared by the high words, on the ALU instead of the FP64 pipe: what is
-// within 2^-20 of the floor counts as at it)
-template <unsigned HI>  // high word of the floor
+// floor used on reconstructed and updated rho and p (NaN -> the floor): x > C by
+// the bits, C < x <= inf as one unsigned range, on the ALU instead of the FP64
+// pipe
+template <unsigned long long C>  // the bits of the floor
 __device__ __forceinline__ bool above(double x)
 {
-    return (unsigned)__double2hiint(x) - (HI + 1) <= 0x7ff00000u - (HI + 1);
+    constexpr unsigned long long lo = C + 1, span = 0x7ff0000000000000ull - lo;
+    return (unsigned)(((unsigned long long)__double_as_longlong(x) - lo) >> 32) <= (unsigned)(span >> 32);
 }
-__device__ __forceinline__ double fl14(double x) { return above<0x3d06849bu>(x) ? x : 1e-14; }
+__device__ __forceinline__ double fl14(double x) { return above<0x3d06849b86a12b9bull>(x) ? x : 1e-14; }
 
 // gp / sqrt(gp r) = sqrt(gp / r): reciprocal root from the hardware seed
 // (2^-20) and one third-order step
@@ -55,7 +56,7 @@ __device__ __forceinline__ double snd_raw(double gp, double r)
 __device__ __forceinline__ double snd(double gp, double r)
 {
     const double c = snd_raw(gp, r);
-    return above<0x3e7ad7f2u>(c) ? c : 1e-7;
+    return above<0x3e7ad7f29abcaf48ull>(c) ? c : 1e-7;
 }
 
 __device__ __forceinline__ double energy(double r, double a, double b, double p, const Gas &gs)

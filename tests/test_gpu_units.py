@@ -58,3 +58,20 @@ def test_f32c_against_f64(V, mean):
     a, b = (_run(w, precision=p).get_state(layout="cons", interior=True) for p in ("f32c", "f64"))
     for q in range(4):
         assert np.sum(np.abs(a[q] - b[q])) <= 1e-6 * np.sum(np.abs(b[q]))
+
+
+@pytest.mark.parametrize("tile", [0, 3])
+def test_f64_just_above_the_floors(tile):
+    """A resting gas whose pressure, or whose squared sound speed, is 5e-7 of
+    itself above the floor of 1e-14 stays what it is, and is not taken for the
+    floor.  (Each step rounds p / (gamma - 1) and back: a few ulp.)"""
+    over = 1e-14 * (1 + 5e-7)
+    for rho, p in ((1.0, over), (1.4, over)):  # the second: c^2 = 1.4 p / rho = over
+        w = np.stack([np.full((N, N), x) for x in (rho, 0.0, 0.0, p)])
+        s = F.Solver(N, bc="periodic", tile=tile)
+        s.set_state(w, interior=True)
+        s.step(3)
+        got, st = s.get_state(interior=True), s.sync()
+        assert st.steps == 3
+        assert np.max(np.abs(got[3] - p)) <= 1e-14 * p
+        assert abs(st.lam_max - np.sqrt(1.4 * p / rho)) <= 1e-14 * st.lam_max

@@ -2,7 +2,8 @@
 the host: wherever a caller's range tests hold, the value has the bits of the
 operator's, the sign of a zero included, and the tests hold for every zero
 numerator.  No GPU needed; the device's reciprocal seed is the host's exact one
-here (test_gpu_quotients.py has the device's)."""
+here (test_gpu_quotients.py has the device's).  Also the FP64 face's floors.
+"""
 from __future__ import annotations
 
 import ctypes as C
@@ -45,6 +46,7 @@ static inline float rsqrtf(float x) { return 1.0f / std::sqrt(x); }
 #define FVB_EXACT_RCP_SQRT 1
 #include "fvb_ieee.cuh"
 #include "fvb_face32.cuh"
+#include "fvb_face64.cuh"
 extern "C" {
 // 1: the range tests hold, and q is the kernels' quotient
 void quot64(int n, const double *a, const double *b, double *q, int *ok)
@@ -77,6 +79,14 @@ void hlle32(int n, const float *L, const float *R, const float *c, const float *
         const float dS = std::fmax(SR - SL, 1e-10f), SRL = SR * SL;
         for (int q = 0; q < 4; ++q)
             o[q] = SL >= 0.f ? FL[q] : SR <= 0.f ? FR[q] : (SR * FL[q] - SL * FR[q] + SRL * (V[q] - U[q])) / dS;
+    }
+}
+// the FP64 face's floors: of rho and p, and of a sound speed whose square is p / r
+void floors64(int n, const double *x, double *f, double *c)
+{
+    for (int i = 0; i < n; ++i) {
+        f[i] = fvb::f64::fl14(x[i]);
+        c[i] = fvb::f64::snd(x[i], 1.0);
     }
 }
 void small64(int n, const double *a, const double *b, double *q, int *ok)
@@ -206,3 +216,19 @@ def test_fp32_hlle(host, vel, unit):
     ptr = lambda x: x.ctypes.data_as(C.c_void_p)
     host.hlle32(N, ptr(L), ptr(R), ptr(c), ptr(E), ptr(F), ptr(P))
     assert _same32(F, P)
+
+
+def test_fp64_floors(host):
+    """x > 1e-14 ? x : 1e-14 to the last bit, for numbers beside the floor, of
+    either sign, infinite and NaN; the sound speed's at 1e-7 likewise."""
+    near = 1e-14 * (1 + RNG.uniform(-4e-6, 4e-6, N // 4))
+    ulps = 1e-14 + RNG.integers(-4, 5, N // 4) * np.spacing(1e-14)
+    x = np.concatenate([near, ulps, -near, _mag(-1074, 1023)[: N // 4]])
+    x[:5] = [0.0, -0.0, np.inf, -np.inf, np.nan]
+    f, c = np.empty_like(x), np.empty_like(x)
+    p = lambda a: a.ctypes.data_as(C.c_void_p)
+    host.floors64(len(x), p(x), p(f), p(c))
+    assert np.array_equal(f, np.where(x > 1e-14, x, 1e-14))
+    with np.errstate(invalid="ignore"):
+        r = np.sqrt(x)
+    assert np.array_equal(c, np.where(r > 1e-7, r, 1e-7))
