@@ -124,14 +124,15 @@ float time_shape(int prec, int order, int n, int shape, cudaStream_t s)
 
 }  // namespace
 
-// FVB_TILE's variant, or -1
+// FVB_TILE's variant, FVB_AUTOTUNE=0's, or -1
 static int forced_shape()
 {
     if (const char *f = std::getenv("FVB_TILE")) {
         const int k = std::atoi(f);
         if (k >= 0 && k < kNumTileShapes) return k;
     }
-    return -1;
+    const char *a = std::getenv("FVB_AUTOTUNE");
+    return a && a[0] == '0' ? 0 : -1;
 }
 
 // Tile variant of a batch, fixed before its grids are known.  FP32c: 32 x 16
@@ -150,8 +151,6 @@ int autotune_shape(int prec, int order, int n)
 {
     const int forced = forced_shape();
     if (forced >= 0) return forced;
-    if (const char *a = std::getenv("FVB_AUTOTUNE"))
-        if (a[0] == '0') return 0;
     int dev = 0;
     cudaGetDevice(&dev);
     const auto key = std::make_tuple(dev, prec, order, size_class(n));

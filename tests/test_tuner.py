@@ -113,3 +113,15 @@ def test_timed_launches_find_a_cleared_step_control(tuner, prec):
     _, launches, dirty = tuner(prec, 640)
     assert launches == 7 * (2 + 3 * 4) * 3  # variants x (warm-up + timed steps) x stages
     assert dirty == 0
+
+
+@pytest.mark.parametrize("n", [0, 640])
+@pytest.mark.parametrize("prec", [0, 1, 2])
+def test_knobs_hold_for_grids_and_batches(tuner, prec, n):
+    assert tuner(prec, n, FVB_AUTOTUNE="0") == [0, 0, 0]
+    assert tuner(prec, n, FVB_AUTOTUNE="0", FVB_TILE="3") == [3, 0, 0]
+    assert tuner(prec, n, FVB_TILE="4") == [4, 0, 0]
+
+
+def test_an_fp32c_batch_is_not_timed(tuner):
+    assert tuner(2, 0) == [5, 0, 0]
