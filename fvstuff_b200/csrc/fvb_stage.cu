@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(NT, MINB) stage32_kernel(const __grid_constant
             if (tid == 0 && gd.ctrl) gd.ctrl->status = FVB_ERR_TIMEOUT;
             break;
         }
-        if (ctl.run && a.stage >= 0) {
+        if (ctl.run) {
             for (int k = tid; k < PL; k += NT) {
                 const R w0 = IN[k], w1 = IN[PL + k], w2 = IN[2 * PL + k], w3 = IN[3 * PL + k];
                 W[k] = w0;
@@ -530,8 +530,8 @@ cudaError_t launch_stage(int prec, int order, int shape, const StageArgs &a, int
     const bool queued = e.fn_queued && !a.grids && a.grid.tmap && a.stage > 0 && a.ntiles_static > 2 * grid_ctas;
     void *fn = a.grids ? e.fn_batched : queued ? e.fn_queued : e.fn;
     if (!fn) return cudaErrorInvalidValue;
-    int max_ctas = 0;
-    cudaError_t err = prepare(e, max_ctas);
+    LaunchFacts f{};
+    const cudaError_t err = launch_facts(fn, e.nt, e.smem, f);
     if (err != cudaSuccess) return err;
     if (grid_ctas <= 0) return cudaSuccess;
     void *args[] = {(void *)&a};

@@ -701,7 +701,7 @@ __global__ void __launch_bounds__((RowPair<TX, TY>::NT), (RowPair<TX, TY>::MINB)
         const float dt = (float)ctl.dt;
         const float dt_h = dt * (float)gd.inv_h;
 
-        if (ctl.run && a.stage == 3) {
+        if (a.stage == 3) {
             // the lo words come from DRAM: into L2 while the faces are computed
             for (int m = tid; m < 4 * TY; m += NT) {
                 const int q = m / TY, j = ty0 + (m - q * TY);
