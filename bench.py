@@ -386,7 +386,8 @@ def run_gpu(args):
                          "traffic": traffic_from_profiles(args.precision, n),
                          "peak_kind": peak_kind,
                          "bytes_per_cell_stage": BYTES_PER_CELL_STAGE[args.precision],
-                         "kernel": "fvb::stage_kernel (one launch per RK stage)",
+                         "kernel": "fvb::%s (one launch per RK stage)" % {
+                             "f64": "stage64_kernel", "f32c": "stage32p_kernel / stage32c_kernel", "f32": "stage32_kernel"}[args.precision],
                          # what bounds it instead (ncu summary of the same kernel): the FP64
                          # pipe, busy this share of the time; at 100 % the stage would
                          # still move only ~45 % of the HBM peak

@@ -507,10 +507,10 @@ __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, 
 
 // What bounds it is memory: 16 values a cell move (12 in stage 1), all loads in
 // flight before the arithmetic, and one reciprocal serves the three quotients
-// of the new density and both energies share gamma - 1's.  2048^2, from cold
-// caches: 72 us in FP64 (86 with an operator a quotient and Uk loaded behind
-// the branch), 50 in FP32 (56); bit-identical, the roundings of the shared
-// products written out.
+// of the new density and both energies share gamma - 1's.  Stage 2 at 2048^2,
+// from cold caches: 88 us in FP64 (107 with an operator a quotient and Uk loaded
+// behind the branch), 53 in FP32 (68), 537 and 268 MB; bit-identical, the
+// roundings of the shared products written out.
 template <class R>
 __global__ void rk3_kernel(int stage, R *Uo, const R *U0, const R *Uk, const R *L, R dt, int n, int np, int g,
                            Gas<R> gs)

@@ -481,7 +481,7 @@ fvb_status fvb_batch_remove(fvb_batch *b, int id)
         if (st) return st;
     }
     cudaFreeAsync(I.block, b->stream);
-    // a zero step control is inactive: the stage-control kernel leaves it be
+    // (no tile names the slot any more; the next grid in it resets the control)
     cudaError_t e = cudaMemsetAsync(b->ctrl_dev + id, 0, sizeof(Ctrl), b->stream);
     b->in_use -= I.bytes;
     I = Instance();

@@ -122,8 +122,8 @@ constexpr const TileShape &tile_shape(int prec, int shape)
     return prec == P64 ? kTileShapes64[shape] : prec == P32C ? kTileShapes32c[shape] : kTileShapes[shape];
 }
 
-// TMA descriptors (fvb_stage.cu): encode the four maps of a grid for a
-// tile shape into host memory; false if this grid cannot use TMA
+// TMA descriptors (fvb_stage.cu): encode the TM_COUNT maps of a grid for
+// a tile shape into host memory; false if this grid cannot use TMA
 bool encode_tile_maps(const GridDev &gd, int prec, int order, int shape, CUtensorMap out[TM_COUNT]);
 // the same for the kernels of BoxPipe (fvb_tma.cuh) with tx x ty tiles
 bool encode_family_maps(const GridDev &gd, int tx, int ty, CUtensorMap out[TM_COUNT]);

@@ -160,7 +160,7 @@ __device__ __forceinline__ void issue_tile_load64(const GridDev &gd, int stage, 
 
 // The loads of a single-grid FP64 kernel that walks tiles with two alternating
 // halo boxes (barriers 0, 1) and, in stages 2 and 3, the tile's U0 (barrier
-// 2): the KEEP, rec3 and D2-viscosity kernels.  Without descriptors the boxes
+// 2): the rec3 kernel.  Without descriptors the boxes
 // are loaded cooperatively and U0 is read where it is used.
 template <int G, int TX, int TY, int NT>
 struct BoxPipe {
