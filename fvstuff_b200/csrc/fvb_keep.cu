@@ -25,7 +25,7 @@
 // reciprocals (fvb_ieee.cuh), a face evaluates the one dissipation its sensor
 // selects, and exp is evaluated only next to the sensor's threshold: 1890
 // instructions a cell, 202 -> 131 us a stage, bit-identical.  With registers
-// in place of local arrays, step control once a CTA and chained launches: 110.
+// in place of local arrays, step control once a CTA and chained launches: 108.
 #include "fvb_aux.h"
 #include "fvb_physics.cuh"
 #include "fvb_device.cuh"

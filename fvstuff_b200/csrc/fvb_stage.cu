@@ -107,8 +107,8 @@ struct L32 {
 // is converted once and not by each of its 64 stencil uses (an eighth-rate
 // instruction), the divisions by 420 and by the HLLE's span come from
 // reciprocals with the same bits (fvb_face32.cuh), and each cell's HLLE sound
-// speed and energy are formed once: 2107 -> 1568 instructions a cell, 34 -> 21 us a stage
-// at 400^2 (351 tiles), bit-identical.
+// speed and energy are formed once: 3396 -> 2133 instructions a cell on the Sod,
+// 34 -> 22 us a stage at 400^2 (351 tiles), bit-identical.
 template <int TX, int TY, int NT, int MINB>
 __global__ void __launch_bounds__(NT, MINB) stage32_kernel(const __grid_constant__ StageArgs a)
 {

@@ -23,7 +23,8 @@
 // stage is 55 us of memory at the copy bandwidth).  Against one face a
 // thread, a copied working tile and U0 through registers, a cell takes 826
 // instructions instead of 1097 and 405 FP64 ones instead of 480, and a 2048^2
-// stage 179 us instead of 231; 801 and 164 with queued tiles (below).
+// stage 179 us instead of 231; 801 and 164 with queued tiles (below), 833 and 165
+// with floors that compare all bits (fvb_face64.cuh).
 #pragma once
 #include <stdint.h>
 
